@@ -155,8 +155,11 @@ struct sgdlm_engine {
   DevBuf<uint32_t> dev_epoch;
   LuPlan plan{};
   LuOptions lu_opt{};
-  JacobiPlan jac{};        // iterative forecast solves of FP32 draws
+  JacobiPlan jac32{}, jac64{};  // iterative forecast solves of FP32 and FP64 draws
   int forecast_iterative = 1;
+  // FP64: the current draws' log|det| were not needed by the forecast that drew them
+  // (sgdlm_get_draws computes them)
+  bool logdet_pending = false;
   DevBuf<int> jac_list;    // nsim + 1: count, then the forecast draws left to factor
   ProposalState prop;
   int chunks = 0;          // VB draw chunks and draws per chunk (vb_chunking)
@@ -292,8 +295,9 @@ int upload_gamma_rows(sgdlm_engine *h) {
   });
   CK(h->g_jac_order.alloc(m));
   CK(cudaMemcpy(h->g_jac_order.ptr, order.data(), m * sizeof(int), cudaMemcpyHostToDevice));
-  h->jac = plan_jacobi((int)m, max_row, h->num_sms);
-  h->jac.order = h->g_jac_order.ptr;
+  h->jac32 = plan_jacobi<float>((int)m, max_row, h->num_sms);
+  h->jac64 = plan_jacobi<double>((int)m, max_row, h->num_sms);
+  h->jac32.order = h->jac64.order = h->g_jac_order.ptr;
   return SGDLM_OK;
 }
 
@@ -506,6 +510,7 @@ int alloc_sim(sgdlm_engine *h, size_t nsim) {
   CK(h->jac_list.reserve(nsim + 1));
   CK(h->part_a.reserve((size_t)h->chunks * m * (P + 2) + m * P));
   CK(h->part_b.reserve((size_t)h->chunks * m * P * P));
+  if (h->nsim != nsim) h->logdet_pending = false;
   h->nsim = nsim;
   return SGDLM_OK;
 }
@@ -582,15 +587,20 @@ void sample_draws(sgdlm_engine *h, const double *m_t, const double *C_t, const d
 // Small systems: one warp per draw, partial pivoting, no redo.
 bool warp_lu(const sgdlm_engine *h) { return h->m <= (size_t)kWarpLuMaxM && h->lu_opt.allow_warp; }
 
-// Forecasts of FP32 draws are solved iteratively first (block LU path only).
+// Forecasts are solved iteratively first (block LU path only).
+template <typename T> const JacobiPlan &jacobi_plan(const sgdlm_engine *h) {
+  return std::is_same<T, float>::value ? h->jac32 : h->jac64;
+}
 template <typename T> bool iterative_forecast(const sgdlm_engine *h) {
-  return std::is_same<T, float>::value && h->forecast_iterative && h->jac.ok && !warp_lu(h);
+  return h->forecast_iterative && jacobi_plan<T>(h).ok && !warp_lu(h);
 }
 
 template <typename T>
 int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
   const long n = (long)h->nsim;
   const bool refine = (h->precision != SGDLM_PRECISION_FP64);
+  // FP64: the log|det| of iteratively solved draws are left to sgdlm_get_draws
+  h->logdet_pending = std::is_same<T, double>::value && x && iterative_forecast<T>(h);
   const GammaRows rows{h->g_rowptr.ptr, h->g_ent.ptr, h->g_extptr.ptr, h->g_extk.ptr};
   if (x) {
     const size_t nx = h->m * h->P;
@@ -606,14 +616,13 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
     h->launches += 1;
     return SGDLM_OK;
   }
-  // forecasts of FP32 draws: the iterative solve first; the LU kernels then
-  // factor only the draws it leaves in jac_list
+  // forecasts: the iterative solve first; the LU kernels then factor only the draws
+  // it leaves in jac_list
   const bool iterative = iterative_forecast<T>(h) && x;
   if (iterative) {
     CK(cudaMemsetAsync(h->jac_list.ptr, 0, sizeof(int), h->stream));
-    launch_forecast_jacobi(h->stream, h->jac, (int)h->m, (int)h->P, n, rows,
-                           reinterpret_cast<const float *>(h->theta_g.ptr), h->g_nnz, h->nu_fc.ptr, y,
-                           h->logdet.ptr, h->jac_list.ptr);
+    launch_forecast_jacobi<T>(h->stream, jacobi_plan<T>(h), (int)h->m, n, rows, as<T>(h->theta_g),
+                              h->g_nnz, h->nu_fc.ptr, y, h->logdet.ptr, h->jac_list.ptr);
     h->launches += 1;
   }
   // the fast pass appends the draws it flags to pivot_list; the redo visits those
@@ -1070,6 +1079,9 @@ int export_draws(sgdlm_engine *h, double *o_lambda, double *o_theta, double *o_l
     th.resize(m * n * P);
     if ((st = d2h(h, th.data(), h->theta.ptr, m * n * P * sizeof(T)))) return st;
   }
+  if (o_logdet && h->logdet_pending &&
+      (st = lu_draws<T>(h, nullptr, h->key((uint32_t)h->epoch), nullptr)))
+    return st;
   if (o_logdet && (st = d2h(h, o_logdet, h->logdet.ptr, n * sizeof(double)))) return st;
   if ((st = sync(h))) return st;
   if (o_lambda)
@@ -1471,6 +1483,7 @@ int sgdlm_set_precision(sgdlm_handle h, int precision) {
   if (precision == h->precision) return SGDLM_OK;
   const int old = h->precision;
   h->precision = precision;
+  h->logdet_pending = false;
   if (h->sim_init) {
     const size_t nsim = h->nsim, batch = h->nsim_batch;
     cudaStreamSynchronize(h->stream);
@@ -1813,6 +1826,7 @@ struct sgdlm_batch {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   std::vector<uint64_t> launches_per_step;
+  std::vector<char> logdet_pending;  // the engines' logdet_pending after a step
   // the recording's arguments (re-recorded by the autotuner)
   std::vector<const double *> y, F, x;
   std::vector<double *> fc, w, st;
@@ -1849,6 +1863,7 @@ int batch_capture(sgdlm_batch *b) {
                  : filter_step<float>(h, b->y[i], b->F[i], b->x[i], b->ess, b->fc[i], b->w[i],
                                       b->st[i]);
     b->launches_per_step[i] = h->launches - l0;
+    b->logdet_pending[i] = h->logdet_pending ? 1 : 0;
     h->launches = l0;   // counted when the graph runs
     h->epoch = ep0;     // advanced when the graph runs
     if (status == SGDLM_OK) e = cudaEventRecord(b->join[i], h->stream);
@@ -1884,6 +1899,7 @@ int batch_launch(sgdlm_batch *b) {
     h->epoch += 2;
     h->launches += b->launches_per_step[i];
     h->is_prior = true;
+    h->logdet_pending = b->logdet_pending[i] != 0;
   }
   return SGDLM_OK;
 }
@@ -1949,6 +1965,7 @@ int sgdlm_batch_create(const sgdlm_handle *handles, size_t count, sgdlm_batch_ha
   for (auto &e : b->join)
     if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return SGDLM_ERR_DEVICE;
   b->launches_per_step.assign(count, 0);
+  b->logdet_pending.assign(count, 0);
   *out = b.release();
   return SGDLM_OK;
 }

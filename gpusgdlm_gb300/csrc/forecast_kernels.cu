@@ -1,21 +1,33 @@
-// Forecast solves y_i = (I - Gamma_i)^-1 nu_i of FP32 draws by fixed-point
-// (Jacobi) iteration, y <- nu + Gamma_i y, on the sparse Gamma_i itself.
+// Forecast solves y_i = (I - Gamma_i)^-1 nu_i by fixed-point (Jacobi) iteration,
+// y <- nu + Gamma_i y, on the sparse Gamma_i itself.
 //
 // The reference factors every forecast draw's dense (I - Gamma_i) and forms its
 // inverse (getrf + getri, rSGDLM/src/SGDLM/SGDLM.cu:594-617): (2/3 + 4/3) m^3
 // flop per draw.  (I - Gamma_i) has at most max_p entries per row, and in the
 // filtering regime the spectral radius of Gamma_i is well below one, so the
 // iteration converges geometrically at O(nnz) per sweep -- a few ten thousand
-// flop per draw at m = 400 instead of 10^8.  A draw is solved here when
-//   (1) the sweeps from y = nu reach max|dy| <= 2^-20 max|y| within kMaxSweeps
-//       (FP32; one thread per row holds the row's Gamma entries in registers in
-//       ELL form, the iterate is in shared memory),
-//   (2) the FP64 residual r = nu - (I - Gamma_i) y, solved by the same
-//       iteration, gives a correction d with max|d| <= 1e-3 max|y| (the rule
-//       the factorising path applies to its refinement step); y + d is written.
+// flop per draw at m = 400 instead of 10^8.  The sweeps run in FP32 (one thread
+// per row holds the row's Gamma entries in registers in ELL form, the iterates are
+// in shared memory); FP64 residuals r = nu - (I - Gamma_i) y, solved by the same
+// iteration, correct their result:
+//   FP32 draws: the sweeps from y = nu reach max|dy| <= 2^-20 max|y| within
+//     kMaxSweeps, then one correction d; max|d| <= 1e-3 max|y| (the rule the
+//     factorising path applies to its refinement step); y + d is written.
+//   FP64 draws: y, nu and the residual's Gamma entries are FP64, and corrections
+//     are added until one is at most 2^-36 max|y| (usually the second).  A
+//     correction is right to about 2^-19 of its size, so what is left is below the
+//     rounding of y itself: the result is as good as a solve with FP64 factors.
 // Any other draw (slow or no convergence: spectral radius near or above one,
 // non-finite values) is appended to `list` and solved by the LU kernels
-// (partial pivoting where needed), as every draw was before.
+// (partial pivoting where needed).
+//
+// A block solves NB = 2 draws at a time, their iterates side by side in shared
+// memory: one gather of two floats, one column index and one barrier per sweep serve
+// both.  The sweeps are bound by the gathers' shared-memory wavefronts (bank
+// conflicts: 32 scattered 4-byte loads take about 3.5, two 16-lane phases of 8-byte
+// loads about 6 for two draws) and by issue slots.  10 000 FP32 draws at m = 400: one
+// draw per block 908 us, two 833 us, four 949 us (the registers leave one block per
+// SM); FP64 draws: two 1.52 ms, four 1.87 ms, and 94.5 ms with FP64 factors.
 #include <algorithm>
 
 #include "kernels.hpp"
@@ -24,188 +36,350 @@ namespace sgdlm {
 namespace {
 
 constexpr int kJacMaxThreads = 1024;  // one row per thread: m <= 1024
+constexpr int kJacGroupThreads = 512;  // two draws per block: m <= 512 (registers)
 constexpr int kMaxSweeps = 128;
-// The first solve stops at max|dy| <= 2^-20 max|y|; the correction, whose size
-// is that of y's error, needs only 2^-10 of its own size: y + d is then within
-// about 2^-30 of the solution (FP32 sweeps reach a few ulps, not further).
+// The first solve stops at max|dy| <= 2^-20 max|y|; the FP32 draws' correction,
+// whose size is that of y's error, needs only 2^-10 of its own size: y + d is then
+// within about 2^-30 of the solution (FP32 sweeps reach a few ulps, not further).
 constexpr float kSweepTol = 9.5367431640625e-07f;   // 2^-20
 constexpr float kCorrSweepTol = 9.765625e-04f;      // 2^-10
 constexpr double kCorrTol = 1e-3;
+constexpr int kCorrBits = 20;                         // bits a correction adds
+constexpr double kDoneTol = 1.4551915228366852e-11;  // 2^-36: FP64 draws' last correction
+constexpr int kMaxCorrections = 4;                    // FP64 draws
 
 struct JacSmem {
-  size_t nud, nuf, ya, yb, res, red, total;
-  __host__ __device__ JacSmem(int m) {
+  size_t yd, xa, xb, yv, red, total;
+  __host__ __device__ JacSmem(int m, int nb) {
     size_t o = 0;
     auto take = [&](size_t bytes) {
       const size_t at = o;
       o = (o + bytes + 15) & ~(size_t)15;
       return at;
     };
-    nud = take((size_t)m * sizeof(double));
-    nuf = take((size_t)m * sizeof(float));
-    ya = take((size_t)m * sizeof(float));
-    yb = take((size_t)m * sizeof(float));
-    res = take((size_t)m * sizeof(float));
-    red = take(2 * (kJacMaxThreads / 32) * sizeof(float));
+    yd = take((size_t)m * nb * sizeof(double));
+    xa = take((size_t)m * nb * sizeof(float));
+    xb = take((size_t)m * nb * sizeof(float));
+    yv = take((size_t)m * nb * sizeof(float));
+    red = take(4 * (size_t)nb * sizeof(unsigned));
     total = o;
   }
 };
 
-// Block-wide maxima of two non-negative values; a NaN counts as infinity.
-__device__ __forceinline__ void block_max2f(float &a, float &b, float *red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  a = (a == a) ? a : INFINITY;
-  b = (b == b) ? b : INFINITY;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a = fmaxf(a, __shfl_xor_sync(0xffffffffu, a, o));
-    b = fmaxf(b, __shfl_xor_sync(0xffffffffu, b, o));
-  }
-  __syncthreads();
-  if (lane == 0) {
-    red[2 * warp] = a;
-    red[2 * warp + 1] = b;
-  }
-  __syncthreads();
-  a = b = 0.f;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-    a = fmaxf(a, red[2 * w]);
-    b = fmaxf(b, red[2 * w + 1]);
+// The NB (1 or 2) values of row r.
+template <int NB> __device__ __forceinline__ void ld_row(const float *x, int r, float (&v)[NB]) {
+  if constexpr (NB == 2) {
+    const float2 q = reinterpret_cast<const float2 *>(x)[r];
+    v[0] = q.x, v[1] = q.y;
+  } else {
+    v[0] = x[r];
   }
 }
+template <int NB> __device__ __forceinline__ void st_row(float *x, int r, const float (&v)[NB]) {
+  if constexpr (NB == 2)
+    reinterpret_cast<float2 *>(x)[r] = make_float2(v[0], v[1]);
+  else
+    x[r] = v[0];
+}
+template <int NB> __device__ __forceinline__ void ld_row(const double *x, int r, double (&v)[NB]) {
+  if constexpr (NB == 2) {
+    const double2 q = reinterpret_cast<const double2 *>(x)[r];
+    v[0] = q.x, v[1] = q.y;
+  } else {
+    v[0] = x[r];
+  }
+}
+template <int NB> __device__ __forceinline__ void st_row(double *x, int r, const double (&v)[NB]) {
+  if constexpr (NB == 2)
+    reinterpret_cast<double2 *>(x)[r] = make_double2(v[0], v[1]);
+  else
+    x[r] = v[0];
+}
 
-// The thread's row r = threadIdx.x in ELL form held in registers: K slots
-// (entries beyond the row's length have value 0 and point at the row itself),
-// the column indices packed two to a register.
-template <int K> struct Row {
+// A non-negative float as an ordered integer key; a NaN counts as infinity.
+__device__ __forceinline__ unsigned key_of(float v) {
+  return __float_as_uint(v == v ? fabsf(v) : INFINITY);
+}
+// Block-wide maxima of 2 NB keys (all zero-based): in place.  red: two sets of 2 NB
+// words used in turn (par); the set not in use is cleared for the next call.  Ends
+// on a barrier.
+template <int NB>
+__device__ __forceinline__ void block_max(unsigned (&a)[NB], unsigned (&b)[NB], unsigned *red,
+                                          int &par) {
+  unsigned *cur = red + par * 2 * NB;
+#pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    const unsigned u = __reduce_max_sync(0xffffffffu, a[q]);
+    const unsigned v = __reduce_max_sync(0xffffffffu, b[q]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(cur + 2 * q, u);
+      atomicMax(cur + 2 * q + 1, v);
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NB; ++q) {
+    a[q] = cur[2 * q];
+    b[q] = cur[2 * q + 1];
+  }
+  par ^= 1;
+  // every thread has passed the barrier, so has read the other set's last maxima
+  if (threadIdx.x < 2 * NB) red[par * 2 * NB + threadIdx.x] = 0u;
+}
+
+// The thread's row in ELL form held in registers: K slots (entries beyond the row's
+// length have value 0 and point at the row itself), the column indices packed two
+// to a register, NB draws' values.
+template <int K, int NB> struct Row {
   uint32_t col[K / 2];
-  float val[K];
+  float val[NB][K];
   __device__ __forceinline__ int c(int q) const {
     return (int)((col[q >> 1] >> (16 * (q & 1))) & 0xFFFFu);
   }
 };
 
-// Sweeps x <- c + Gamma x from x = c over this thread's row r.  Returns whether
-// they converged (max|dx| <= tol max|x|, everything finite); *out is the last
-// iterate.  wlen: the longest row of this warp, rounded up to even (warp-uniform):
-// slots beyond it are padding in every row of the warp (value 0, so skipping them
-// leaves every sum unchanged).
-template <int K>
-__device__ bool jacobi(int m, int r, int wlen, const Row<K> &R, const float *c, float *xa,
-                       float *xb, float *red, float tol, float **out) {
-  if (r < m) xa[r] = c[r];
+// Sweeps x <- c + Gamma x from x = c over this thread's row r, for the draws in
+// `todo` (a mask).  Returns the mask of the draws that converged (max|dx| <= tol
+// max|x|, everything finite); x receives the row's last iterate of each draw, which
+// stops there while the others go on.  wlen: the longest row of this warp, rounded
+// up to even (warp-uniform): slots beyond it are padding in every row of the warp
+// (value 0, so skipping them leaves every sum unchanged).  Ends on a barrier; xa and
+// xb are free on entry and after it.
+template <int K, int NB>
+__device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row<K, NB> &R,
+                                           const float (&c)[NB], float *xa, float *xb,
+                                           unsigned *red, int &par, float tol, unsigned todo,
+                                           float (&x)[NB]) {
+  unsigned conv = 0;
+#pragma unroll
+  for (int b = 0; b < NB; ++b) x[b] = c[b];
+  if (mine) st_row<NB>(xa, r, x);
   __syncthreads();
   float *cur = xa, *nxt = xb;
-  for (int it = 1; it <= kMaxSweeps; ++it) {
-    float dmax = 0.f, xmax = 0.f;
-    if (r < m) {
-      float a0 = c[r], a1 = 0.f;
+  for (int it = 1; it <= kMaxSweeps && todo; ++it) {
+    float a0[NB], a1[NB];
 #pragma unroll
-      for (int q = 0; q < K; q += 2) {
-        if (q >= wlen) break;
-        a0 = fmaf(R.val[q], cur[R.c(q)], a0);
-        a1 = fmaf(R.val[q + 1], cur[R.c(q + 1)], a1);
+    for (int b = 0; b < NB; ++b) a0[b] = c[b], a1[b] = 0.f;
+#pragma unroll
+    for (int q = 0; q < K; q += 2) {
+      if (q >= wlen) break;
+      float u[NB], v[NB];
+      ld_row<NB>(cur, R.c(q), u);
+      ld_row<NB>(cur, R.c(q + 1), v);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        a0[b] = fmaf(R.val[b][q], u[b], a0[b]);
+        a1[b] = fmaf(R.val[b][q + 1], v[b], a1[b]);
       }
-      const float v = a0 + a1;
-      nxt[r] = v;
-      // fmaxf drops NaN operands: a NaN (an overflowed iterate times a padded
-      // zero slot, or inf - inf) must count as divergence, so it becomes infinity
-      // here
-      const float av = fabsf(v), dv = fabsf(v - cur[r]);
-      xmax = (av == av) ? av : INFINITY;
-      dmax = (dv == dv) ? dv : INFINITY;
     }
+#pragma unroll
+    for (int b = 0; b < NB; ++b) a0[b] = a0[b] + a1[b];
+    if (mine) st_row<NB>(nxt, r, a0);
     float *t = cur;
     cur = nxt;
     nxt = t;
-    if ((it & 3) == 0 || it == kMaxSweeps) {
-      block_max2f(dmax, xmax, red);  // also the barrier between sweeps
-      if (!(xmax < INFINITY)) break;
-      if (dmax <= tol * xmax) {
-        *out = cur;
-        return true;
+    const bool check = (it & 3) == 0;
+    unsigned dk[NB], xk[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const bool live = mine && (todo >> b & 1);
+      if (check) {
+        dk[b] = live ? key_of(a0[b] - x[b]) : 0u;
+        xk[b] = live ? key_of(a0[b]) : 0u;
+      }
+      if (live) x[b] = a0[b];
+    }
+    if (check) {
+      block_max<NB>(dk, xk, red, par);  // also the barrier between sweeps
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const float xmax = __uint_as_float(xk[b]);
+        if (!(todo >> b & 1)) continue;
+        if (!(xmax < INFINITY)) {
+          todo &= ~(1u << b);
+        } else if (__uint_as_float(dk[b]) <= tol * xmax) {
+          todo &= ~(1u << b);
+          conv |= 1u << b;
+        }
       }
     } else {
       __syncthreads();
     }
   }
-  *out = cur;
-  return false;
+  return conv;
 }
 
-template <int K>
-__global__ void __launch_bounds__(kJacMaxThreads)
-    k_forecast_jacobi(int m, int P, long n, GammaRows rows, const float *__restrict__ theta_g,
-                      int nnz,
+template <typename T, int K, int NB>
+__global__ void __launch_bounds__(NB > 1 ? kJacGroupThreads : kJacMaxThreads)
+    k_forecast_jacobi(int m, long n, GammaRows rows, const T *__restrict__ theta_g, int nnz,
                       const double *__restrict__ nu, double *__restrict__ y,
                       double *__restrict__ logdet, int *__restrict__ list,
                       const int *__restrict__ order) {
+  static_assert(NB == 1 || NB == 2, "");
+  static_assert(kMaxSweeps % 4 == 0, "the last sweep is a checked one");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const JacSmem L(m);
-  double *nud = reinterpret_cast<double *>(smem_raw + L.nud);
-  float *nuf = reinterpret_cast<float *>(smem_raw + L.nuf);
-  float *ya = reinterpret_cast<float *>(smem_raw + L.ya);
-  float *yb = reinterpret_cast<float *>(smem_raw + L.yb);
-  float *res = reinterpret_cast<float *>(smem_raw + L.res);
-  float *red = reinterpret_cast<float *>(smem_raw + L.red);
+  const JacSmem L(m, NB);
+  double *yds = reinterpret_cast<double *>(smem_raw + L.yd);
+  float *xa = reinterpret_cast<float *>(smem_raw + L.xa);
+  float *xb = reinterpret_cast<float *>(smem_raw + L.xb);
+  float *yv = reinterpret_cast<float *>(smem_raw + L.yv);
+  unsigned *red = reinterpret_cast<unsigned *>(smem_raw + L.red);
   const int tid = threadIdx.x;
-  const int r = (tid < m && order) ? order[tid] : tid;  // this thread's row (r >= m: none)
-  Row<K> R;
-  const int e0 = r < m ? rows.rowptr[r] : 0;
-  const int len = r < m ? rows.rowptr[r + 1] - e0 : 0;
+  const bool mine = tid < m;
+  const int r = mine ? (order ? order[tid] : tid) : 0;  // this thread's row
+  Row<K, NB> R;
+  const int e0 = mine ? rows.rowptr[r] : 0;
+  const int len = mine ? rows.rowptr[r + 1] - e0 : 0;
   const int wlen = (__reduce_max_sync(0xffffffffu, (unsigned)len) + 1) & ~1;
 #pragma unroll
   for (int q = 0; q < K; q += 2) {
-    const uint32_t self = (uint32_t)(r < m ? r : 0);
-    const uint32_t c0 = q < len ? (uint32_t)rows.ent[e0 + q].y : self;
-    const uint32_t c1 = q + 1 < len ? (uint32_t)rows.ent[e0 + q + 1].y : self;
+    const uint32_t c0 = q < len ? (uint32_t)rows.ent[e0 + q].y : (uint32_t)r;
+    const uint32_t c1 = q + 1 < len ? (uint32_t)rows.ent[e0 + q + 1].y : (uint32_t)r;
     R.col[q >> 1] = c0 | (c1 << 16);
   }
-  for (long i = blockIdx.x; i < n; i += gridDim.x) {
-    // this draw's Gamma entries (row r's run of its Gamma copy) and nu
-    const float *th = theta_g + (size_t)i * nnz + e0;
+  if (tid < 4 * NB) red[tid] = 0u;
+  int par = 0;
+  __syncthreads();
+  for (long i0 = (long)blockIdx.x * NB; i0 < n; i0 += (long)gridDim.x * NB) {
+    const int nd = (int)min((long)NB, n - i0);
+    unsigned ok = (1u << nd) - 1u;  // the draws that are solved here (uniform)
+    // the draws' Gamma entries (row r's runs of their Gamma copies) and nu
+    double nud[NB], out[NB];
 #pragma unroll
-    for (int q = 0; q < K; ++q) R.val[q] = q < len ? th[q] : 0.f;
-    if (r < m) {
-      const double v = nu[(size_t)r * n + i];
-      nud[r] = v;
-      nuf[r] = (float)v;
-    }
-    __syncthreads();
-    float *yv = nullptr;
-    bool ok = jacobi<K>(m, r, wlen, R, nuf, ya, yb, red, kSweepTol, &yv);
-    if (ok) {
-      // residual in FP64 and its correction by the same iteration
-      float *other = (yv == ya) ? yb : ya;
-      if (r < m) {
-        double v = nud[r] - (double)yv[r];
+    for (int b = 0; b < NB; ++b) {
+      const T *th = theta_g + (size_t)(i0 + b) * nnz + e0;
 #pragma unroll
-        for (int q = 0; q < K; ++q) v += (double)R.val[q] * (double)yv[R.c(q)];
-        res[r] = (float)v;
-      }
-      __syncthreads();
-      // the correction's iterates go to `other` and nuf (nu's FP32 copy is no
-      // longer needed); yv keeps y
-      float *dv = nullptr;
-      ok = jacobi<K>(m, r, wlen, R, res, other, nuf, red, kCorrSweepTol, &dv);
-      float dmax = 0.f, ymax = 0.f;
-      if (r < m) {
-        const float ad = fabsf(dv[r]), ay = fabsf(yv[r]);
-        dmax = (ad == ad) ? ad : INFINITY;
-        ymax = (ay == ay) ? ay : INFINITY;
-      }
-      block_max2f(dmax, ymax, red);
-      ok = ok && ymax < INFINITY && dmax < INFINITY && (double)dmax <= kCorrTol * (double)ymax;
-      // thread t writes row t (block_max2f ended on a barrier): a warp's stores are
-      // one contiguous run, also when y is page-locked host memory
-      if (ok && tid < m) y[(size_t)i * m + tid] = (double)yv[tid] + (double)dv[tid];
+      for (int q = 0; q < K; ++q) R.val[b][q] = (b < nd && q < len) ? (float)th[q] : 0.f;
+      nud[b] = (mine && b < nd) ? nu[(size_t)r * n + i0 + b] : 0.0;
     }
-    if (tid == 0) {
+    float c[NB], x[NB], yo[NB];
+    unsigned ka[NB], kb[NB];
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int b = 0; b < NB; ++b) c[b] = (float)nud[b];
+      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kSweepTol, ok, yo);
       if (ok) {
-        logdet[i] = NAN;  // no factorisation: no log|det| for this forecast draw
+        // residual in FP64 and its correction by the same iteration
+        if (mine) st_row<NB>(yv, r, yo);
+        __syncthreads();
+        double v[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[b] = nud[b] - (double)yo[b];
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+          if (q >= wlen) break;
+          float u[NB];
+          ld_row<NB>(yv, R.c(q), u);
+#pragma unroll
+          for (int b = 0; b < NB; ++b) v[b] += (double)R.val[b][q] * (double)u[b];
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) c[b] = (float)v[b];
+        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kCorrSweepTol, ok, x);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          ka[b] = mine ? key_of(x[b]) : 0u;
+          kb[b] = mine ? key_of(yo[b]) : 0u;
+          out[b] = (double)yo[b] + (double)x[b];
+        }
+        block_max<NB>(ka, kb, red, par);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const float dmax = __uint_as_float(ka[b]), ymax = __uint_as_float(kb[b]);
+          if (!((conv >> b & 1) && ymax < INFINITY && dmax < INFINITY &&
+                (double)dmax <= kCorrTol * (double)ymax))
+            ok &= ~(1u << b);
+        }
+      }
+    } else {
+      // FP64 draws.  The system is scaled by a power of two to max|nu| in [1, 2), and
+      // a correction's right-hand side by the bits gained so far, so that the FP32
+      // sweeps meet values of normal range whatever the data's (powers of two: exact)
+      double inv[NB];
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        ka[b] = (unsigned)__double2hiint(nud[b]) & 0x7FFFFFFFu;
+        kb[b] = 0u;
+      }
+      block_max<NB>(ka, kb, red, par);
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const int ex = (int)(ka[b] >> 20);  // biased exponent of the largest |nu|
+        if (ex == 0x7FF) ok &= ~(1u << b);
+        const int e = max(-1000, min(1000, ex - 1023));
+        const bool sc = ex > 0 && ex < 0x7FF;
+        inv[b] = sc ? __hiloint2double((1023 + e) << 20, 0) : 1.0;
+        if (sc) nud[b] *= __hiloint2double((1023 - e) << 20, 0);
+        c[b] = (float)nud[b];
+      }
+      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kSweepTol, ok, yo);
+      unsigned todo = ok;
+#pragma unroll
+      for (int b = 0; b < NB; ++b) out[b] = (double)yo[b];
+      double up = 1.0, down = 1.0;
+#pragma unroll 1
+      for (int it = 1; it <= kMaxCorrections && todo; ++it) {
+        up *= (double)(1 << kCorrBits);
+        down *= 1.0 / (double)(1 << kCorrBits);
+        if (mine) st_row<NB>(yds, r, out);
+        __syncthreads();
+        double v[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) v[b] = nud[b] - out[b];
+#pragma unroll 2
+        for (int q = 0; q < len; ++q) {
+          double u[NB];
+          ld_row<NB>(yds, rows.ent[e0 + q].y, u);
+#pragma unroll
+          for (int b = 0; b < NB; ++b)
+            if (b < nd) v[b] = fma((double)theta_g[(size_t)(i0 + b) * nnz + e0 + q], u[b], v[b]);
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) c[b] = (float)(v[b] * up);
+        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kSweepTol, todo, x);
+        ok &= ~(todo & ~conv);
+        todo &= conv;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          if (todo >> b & 1) out[b] += (double)x[b] * down;
+          ka[b] = mine ? key_of(x[b]) : 0u;
+          kb[b] = mine ? key_of((float)out[b]) : 0u;
+        }
+        block_max<NB>(ka, kb, red, par);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const double dmax = (double)__uint_as_float(ka[b]) * down, ymax = (double)__uint_as_float(kb[b]);
+          if (!(todo >> b & 1)) continue;
+          if (!(ymax < INFINITY && dmax <= kCorrTol * ymax)) {
+            ok &= ~(1u << b);
+            todo &= ~(1u << b);
+          } else if (dmax <= kDoneTol * ymax) {
+            todo &= ~(1u << b);
+          }
+        }
+      }
+      ok &= ~todo;  // corrections that do not shrink
+#pragma unroll
+      for (int b = 0; b < NB; ++b) out[b] *= inv[b];
+    }
+    if (ok) {
+      // thread t writes row t: a warp's stores are one contiguous run, also when y is
+      // page-locked host memory
+      if (mine) st_row<NB>(yds, r, out);
+      __syncthreads();
+      if (mine) {
+        ld_row<NB>(yds, tid, out);
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+          if (ok >> b & 1) y[(size_t)(i0 + b) * m + tid] = out[b];
+      }
+    }
+    if (tid < nd) {
+      if (ok >> tid & 1) {
+        logdet[i0 + tid] = NAN;  // no factorisation: no log|det| for this forecast draw
       } else {
         const int q = atomicAdd(list, 1);
-        if (q < n) list[1 + q] = (int)i;
+        if (q < n) list[1 + q] = (int)(i0 + tid);
       }
     }
     __syncthreads();
@@ -215,22 +389,30 @@ __global__ void __launch_bounds__(kJacMaxThreads)
 // ELL widths: the smallest of these that holds the longest row
 constexpr int kJacWidths[] = {8, 12, 16, 18, 20, 24, 32};
 
-template <int K> void *jacobi_kernel() { return reinterpret_cast<void *>(k_forecast_jacobi<K>); }
-void *jacobi_kernel_for(int K) {
+// Calls f with the kernel of type T, width K and draws per block (group: two).
+template <typename T, typename F> void with_jacobi_kernel(int K, bool group, F f) {
+#define SGDLM_JACOBI(KK)                  \
+  case KK:                                \
+    if (group)                            \
+      f(k_forecast_jacobi<T, KK, 2>, 2);  \
+    else                                  \
+      f(k_forecast_jacobi<T, KK, 1>, 1);  \
+    break
   switch (K) {
-    case 8: return jacobi_kernel<8>();
-    case 12: return jacobi_kernel<12>();
-    case 16: return jacobi_kernel<16>();
-    case 18: return jacobi_kernel<18>();
-    case 20: return jacobi_kernel<20>();
-    case 24: return jacobi_kernel<24>();
-    default: return jacobi_kernel<32>();
+    SGDLM_JACOBI(8);
+    SGDLM_JACOBI(12);
+    SGDLM_JACOBI(16);
+    SGDLM_JACOBI(18);
+    SGDLM_JACOBI(20);
+    SGDLM_JACOBI(24);
+    SGDLM_JACOBI(32);
   }
+#undef SGDLM_JACOBI
 }
 
 }  // namespace
 
-JacobiPlan plan_jacobi(int m, int max_row, int num_sms) {
+template <typename T> JacobiPlan plan_jacobi(int m, int max_row, int num_sms) {
   JacobiPlan jp{};
   if (m < 1 || m > kJacMaxThreads || max_row > 32) return jp;
   jp.nnz = 32;
@@ -240,37 +422,53 @@ JacobiPlan plan_jacobi(int m, int max_row, int num_sms) {
       break;
     }
   jp.threads = (m + 31) / 32 * 32;
-  jp.smem = JacSmem(m).total;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, jacobi_kernel_for(jp.nnz), jp.threads,
-                                                    jp.smem) != cudaSuccess ||
-      per_sm < 1) {
-    (void)cudaGetLastError();
-    return jp;
+  // [0] one draw per block, [1] two
+  for (int g = 0; g < 2; ++g) {
+    if (g == 1 && jp.threads > kJacGroupThreads) break;
+    int per_sm = 0;
+    cudaError_t e = cudaSuccess;
+    with_jacobi_kernel<T>(jp.nnz, g == 1, [&](auto kernel, int nb) {
+      jp.draws[g] = nb;
+      jp.smem[g] = JacSmem(m, nb).total;
+      if (jp.smem[g] > 48 * 1024)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jp.smem[g]);
+      if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, jp.threads, jp.smem[g]);
+    });
+    if (e != cudaSuccess || per_sm < 1) {
+      (void)cudaGetLastError();
+      jp.draws[g] = 0;
+      continue;
+    }
+    jp.grid[g] = num_sms * per_sm;
   }
-  jp.grid = num_sms * per_sm;
-  jp.ok = 1;
+  jp.ok = jp.draws[0] > 0;
   return jp;
 }
+template JacobiPlan plan_jacobi<float>(int, int, int);
+template JacobiPlan plan_jacobi<double>(int, int, int);
 
-void launch_forecast_jacobi(cudaStream_t s, const JacobiPlan &jp, int m, int P, long n,
-                            GammaRows rows, const float *theta_g, int nnz, const double *nu,
-                            double *y, double *logdet, int *list) {
-  const unsigned grid = (unsigned)std::max<long>(std::min<long>(jp.grid, n), 1);
-  const unsigned th = (unsigned)jp.threads;
-#define SGDLM_JACOBI(K)                                                                    \
-  k_forecast_jacobi<K><<<grid, th, jp.smem, s>>>(m, P, n, rows, theta_g, nnz, nu, y, logdet, list, \
-                                                 jp.order)
-  switch (jp.nnz) {
-    case 8: SGDLM_JACOBI(8); break;
-    case 12: SGDLM_JACOBI(12); break;
-    case 16: SGDLM_JACOBI(16); break;
-    case 18: SGDLM_JACOBI(18); break;
-    case 20: SGDLM_JACOBI(20); break;
-    case 24: SGDLM_JACOBI(24); break;
-    default: SGDLM_JACOBI(32); break;
-  }
-#undef SGDLM_JACOBI
+template <typename T>
+void launch_forecast_jacobi(cudaStream_t s, const JacobiPlan &jp, int m, long n, GammaRows rows,
+                            const T *theta_g, int nnz, const double *nu, double *y,
+                            double *logdet, int *list) {
+  // two draws per block once they fill half of the SMs' resident blocks; below that
+  // one draw per block spreads them over more SMs
+  const int g = jp.draws[1] > 0 && n >= (long)jp.grid[1] * jp.draws[1] / 2 ? 1 : 0;
+  const long blocks = (n + jp.draws[g] - 1) / jp.draws[g];
+  const unsigned grid = (unsigned)std::max<long>(std::min<long>(jp.grid[g], blocks), 1);
+  with_jacobi_kernel<T>(jp.nnz, g == 1, [&](auto kernel, int) {
+    if (jp.smem[g] > 48 * 1024)
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jp.smem[g]);
+    kernel<<<grid, (unsigned)jp.threads, jp.smem[g], s>>>(m, n, rows, theta_g, nnz, nu, y, logdet, list,
+                                                          jp.order);
+  });
 }
+template void launch_forecast_jacobi<float>(cudaStream_t, const JacobiPlan &, int, long, GammaRows,
+                                            const float *, int, const double *, double *, double *,
+                                            int *);
+template void launch_forecast_jacobi<double>(cudaStream_t, const JacobiPlan &, int, long, GammaRows,
+                                             const double *, int, const double *, double *, double *,
+                                             int *);
 
 }  // namespace sgdlm

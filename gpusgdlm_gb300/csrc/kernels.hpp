@@ -157,26 +157,27 @@ void launch_lu(cudaStream_t s, const LuPlan &plan, long n, const EliminationPlan
                int *pivot_list = nullptr,
                // the same form: only the listed draws are factored, or nullptr: all
                const int *draw_list = nullptr);
-// Forecast solves of FP32 draws by fixed-point iteration on the sparse Gamma_i
-// (forecast_kernels.cu).  ok = 0: the shared-memory working set of a draw does
-// not fit, every draw keeps the factorising path.
+// Forecast solves by fixed-point iteration on the sparse Gamma_i
+// (forecast_kernels.cu).  ok = 0: every draw keeps the factorising path.
 struct JacobiPlan {
-  int ok, grid, threads, nnz;  // threads: m rounded up to 32; nnz: ELL slots per row (8..32)
-  size_t smem;
+  int ok, threads, nnz;  // threads: m rounded up to 32; nnz: ELL slots per row (8..32)
+  // [0]: one draw per block, [1]: two (draws[1] = 0: not available at this m)
+  int draws[2], grid[2];
+  size_t smem[2];
   // thread t takes row order[t] (the rows by decreasing length, so that a warp's
   // rows are of similar length and its sweeps stop at its own longest row), or
   // nullptr: thread t takes row t
   const int *order;
 };
 // m <= 1024 and at most 32 simultaneous parents per series, else ok = 0.
-JacobiPlan plan_jacobi(int m, int max_row, int num_sms);
+template <typename T> JacobiPlan plan_jacobi(int m, int max_row, int num_sms);
 // y (draw-major) of every draw whose iteration converges (logdet[i] set to NaN:
 // not factored); the others are appended to list (n + 1 ints, [0] zero on entry).
 // theta_g: the draws' Gamma entries (GammaDraws layout, nnz per draw); nu:
 // series-major right-hand sides.
-void launch_forecast_jacobi(cudaStream_t s, const JacobiPlan &jp, int m, int P, long n,
-                            GammaRows rows, const float *theta_g, int nnz, const double *nu,
-                            double *y,
+template <typename T>
+void launch_forecast_jacobi(cudaStream_t s, const JacobiPlan &jp, int m, long n, GammaRows rows,
+                            const T *theta_g, int nnz, const double *nu, double *y,
                             double *logdet, int *list);
 // The forecast right-hand sides nu_ij = z_ij / sqrt(lambda_ij) + x_j' phi_ij of all
 // draws (series-major, nu[j*n + i]); theta series-major; x32: an FP32 copy of x

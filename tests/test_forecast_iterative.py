@@ -1,0 +1,78 @@
+"""The iterative forecast solves against the factorising path (which the other tests
+compare with the oracle), at the edges of their launch rule: one draw per block, two
+draws per block, a last block with a single draw, m at and beside multiples of 32,
+more rows than the two-draw form takes, and values far outside FP32's range.
+
+Tolerance of the FP64 form: both solve the same FP64 system with a backward error of
+a few 2^-53 (growth below 8, condition numbers below 100 for these draws), so they
+agree to 100 * 2^-53 * a few = 1e-13 of the draw's largest value; 1e-12 leaves a
+factor of ten.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from gpusgdlm_gb300 import SGDLM
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(m, kmax, precision, seed=3, levels=4):
+    import bench
+
+    wl = bench.make_workload(m=m, kmax=kmax, T=4, seed=seed)
+    P = wl["P"]
+    s = SGDLM(1, strict=True, precision=precision)
+    s.setSimultaneousParents(wl["p"], np.where(wl["sp"] >= m * m, np.nan, wl["sp"]).astype(float))
+    s.setWarpLu(False)  # m <= 32 takes the warp path by default
+    s.setDiscountFactors(np.full(m, 0.97), np.full((P, P, m), 0.98))
+    rng = np.random.default_rng(seed)
+    s.setPriorParameters(rng.uniform(-0.05, 0.05, size=(P, m)),
+                         np.repeat((1e-4 * np.eye(P))[:, :, None], m, axis=2),
+                         np.full(m, 20.0), np.full(m, 1.0))
+    return s, wl
+
+
+def _forecast(s, wl, n, x, iterative):
+    s.setForecastSolver(iterative)
+    s.setRngState(11, 0)
+    return s.computeForecast(n, n, x)
+
+
+@pytest.mark.parametrize("m,kmax,n,scale", [
+    (3, 2, 5, 1.0), (32, 4, 1, 1.0), (33, 4, 4001, 1.0), (100, 10, 3000, 1e-250), (100, 10, 3000, 1e250),
+    (129, 17, 2501, 1.0), (400, 17, 601, 1.0), (540, 5, 700, 1.0)])
+def test_fp64_matches_factored(built_lib, m, kmax, n, scale):
+    s, wl = _engine(m, kmax, "fp64")
+    x = scale * wl["F_of"](2, False)
+    y = _forecast(s, wl, n, x, True)
+    assert s.getStats()["forecast_draws_factored"] == 0
+    ref = _forecast(s, wl, n, x, False)
+    assert s.getStats()["forecast_draws_factored"] == n
+    err = np.abs(y - ref).max(axis=0) / np.abs(ref).max(axis=0)
+    assert err.max() <= 1e-12
+    s.close()
+
+
+def test_fp64_log_dets_after_forecast(built_lib):
+    """The draws' log|det| are not needed by the solve; getDraws still has them."""
+    s, wl = _engine(70, 6, "fp64")
+    n = 500
+    _forecast(s, wl, n, wl["F_of"](2, False), True)
+    d = s.getDraws()
+    ld = oracle.logdet(wl["sp"], np.asfortranarray(d["thetas"].transpose(0, 2, 1)))
+    np.testing.assert_allclose(d["log_dets"], ld, rtol=0, atol=1e-12)
+    s.close()
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("m", [33, 250, 520])
+def test_draws_do_not_depend_on_their_block(built_lib, precision, m):
+    """The same draw solved in a block of its own (few draws) and beside another one
+    (many draws) gives the same bits."""
+    s, wl = _engine(m, 6, precision)
+    x = wl["F_of"](2, False)
+    many = _forecast(s, wl, 4000, x, True)
+    few = _forecast(s, wl, 3, x, True)
+    np.testing.assert_array_equal(few, many[:, :3])
+    s.close()
