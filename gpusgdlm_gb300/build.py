@@ -33,6 +33,7 @@ SOURCES = [
     "proposal_kernels.cu",
     "forecast_kernels.cu",
     "warp_lu.cu",
+    "logdet64.cu",
 ]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3"]

@@ -138,6 +138,12 @@ struct sgdlm_engine {
   EliminationPlanHost eplan;
   DevBuf<int> elim_buf;
   EliminationPlan elim_dev{};
+  // FP64 draws: the deep elimination for log|det| (planned when FP64 simulation
+  // memory is first needed for the current parental sets)
+  bool deep_planned = false;
+  DevBuf<int> deep_buf;
+  LogdetPlan deep_dev{};
+  Logdet64Launch deep_launch{};
   DevBuf<double> y_t, F_t, x_t;
   DevBuf<double> fm_t, fC_t, fn_t, fs_t, fW_t;
   DevBuf<double> U64;
@@ -306,6 +312,7 @@ int upload_gamma_rows(sgdlm_engine *h) {
 int upload_elimination(sgdlm_engine *h) {
   const int m = (int)h->m, P = (int)h->P;
   h->eplan = plan_elimination(m, P, h->h_sp, h->elim_levels);
+  h->deep_planned = false;
   const EliminationPlanHost &pl = h->eplan;
   std::vector<int> buf;
   std::vector<size_t> offs;
@@ -377,6 +384,48 @@ int upload_elimination(sgdlm_engine *h) {
   d.core_node = b + offs[k++];
   // without levels the whole matrix is the dense core, built from the parental sets
   d.core_map = pl.nlev > 0 ? reinterpret_cast<const uint16_t *>(b + offs[k]) : nullptr;
+  return SGDLM_OK;
+}
+
+// Plans the deep elimination of FP64 draws for the current parental sets and uploads
+// it as one int array; deep_dev.core_n = 0: none (no levels wanted, or too large).
+int upload_logdet_plan(sgdlm_engine *h) {
+  if (h->deep_planned) return SGDLM_OK;
+  h->deep_dev = LogdetPlan{};
+  h->deep_planned = true;
+  if (h->eplan.nlev == 0) return SGDLM_OK;
+  const LogdetPlanHost pl = plan_logdet((int)h->m, (int)h->P, h->h_sp, logdet64_max_slots());
+  if (pl.core_n == 0) return SGDLM_OK;
+  std::vector<int> buf;
+  std::vector<size_t> offs;
+  auto put = [&](const void *data, size_t n_ints) {
+    while (buf.size() % 4) buf.push_back(0);
+    offs.push_back(buf.size());
+    const int *p = static_cast<const int *>(data);
+    buf.insert(buf.end(), p, p + n_ints);
+  };
+  put(pl.diag_slot.data(), pl.diag_slot.size());
+  put(pl.l0_slot.data(), pl.l0_slot.size());
+  put(pl.lev_piv.data(), pl.lev_piv.size());
+  put(pl.piv.data(), pl.piv.size());
+  put(pl.lev_scale.data(), pl.lev_scale.size());
+  put(pl.scale.data(), pl.scale.size());
+  put(pl.lev_chunk.data(), pl.lev_chunk.size());
+  put(pl.chunk_tofs.data(), pl.chunk_tofs.size());
+  put(pl.ent.data(), pl.ent.size());
+  put(pl.terms.data(), pl.terms.size());
+  std::vector<uint16_t> map(pl.core_map);
+  if (map.size() % 2) map.push_back(0);
+  put(map.data(), map.size() / 2);
+  CK(h->deep_buf.alloc(buf.size()));
+  CK(cudaMemcpy(h->deep_buf.ptr, buf.data(), buf.size() * sizeof(int), cudaMemcpyHostToDevice));
+  const int *b = h->deep_buf.ptr;
+  auto u = [&](size_t k) { return reinterpret_cast<const unsigned *>(b + offs[k]); };
+  h->deep_dev = LogdetPlan{pl.m,          (int)pl.l0_slot.size(), pl.nlev,     pl.nv,
+                           pl.core_n,     pl.ld,                  b + offs[0], b + offs[1],
+                           b + offs[2],   b + offs[3],            b + offs[4], u(5),
+                           b + offs[6],   b + offs[7],            u(8),        u(9),
+                           reinterpret_cast<const uint16_t *>(b + offs[10])};
   return SGDLM_OK;
 }
 
@@ -461,6 +510,9 @@ void release_all(sgdlm_engine *h) {
   h->x32.release();
   h->elim_buf.release();
   h->elim_dev = EliminationPlan{};
+  h->deep_buf.release();
+  h->deep_dev = LogdetPlan{};
+  h->deep_planned = false;
   h->series_flags.release();
   h->dev_epoch.release();
   h->mem_init = false;
@@ -481,6 +533,16 @@ int plan_sim(sgdlm_engine *h, long n, LuPlan *out) {
              "(limit 232448); use the mixed precision or a smaller m",
              h->m, std::max(pl.smem, pl.smem_fallback));
     return h->fail(SGDLM_ERR_UNSUPPORTED, buf);
+  }
+  h->deep_launch = Logdet64Launch{};
+  if (h->precision == SGDLM_PRECISION_FP64) {
+    int st = upload_logdet_plan(h);
+    if (st) return st;
+    if (h->deep_dev.core_n > 0)
+      h->deep_launch = plan_logdet64_launch(h->deep_dev, n, h->num_sms, h->lu_opt.max_grid);
+    if (h->deep_launch.ok)
+      pl.scratch_elems_total = std::max(pl.scratch_elems_total,
+                                        (size_t)h->deep_launch.grid * h->deep_launch.slab_elems);
   }
   *out = pl;
   return SGDLM_OK;
@@ -627,7 +689,16 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
   }
   // the fast pass appends the draws it flags to pivot_list; the redo visits those
   CK(cudaMemsetAsync(h->pivot_list.ptr, 0, sizeof(int), h->stream));
-  launch_lu<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
+  bool deep = false;
+  if constexpr (std::is_same<T, double>::value) {
+    // log|det| of FP64 draws: the deep elimination where there is one (2 to 30 times
+    // fewer FP64 operations than the levels and dense core below)
+    deep = !x && h->deep_launch.ok;
+    if (deep)
+      launch_logdet64(h->stream, h->deep_launch, n, h->deep_dev, as<T>(h->theta_g),
+                      as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, h->pivot_list.ptr);
+  }
+  if (!deep) launch_lu<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
                as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x, as<T>(h->lambda), key,
                refine, y, rows, x ? h->nu_fc.ptr : nullptr, h->pivot_list.ptr,
                iterative ? h->jac_list.ptr : nullptr);
