@@ -69,6 +69,7 @@ template <typename T> struct DevBuf {
 };
 
 constexpr size_t kMaxP = 64;
+constexpr size_t kGivenKept = 256u << 20;  // bytes of loss_and_gradient's workspace kept between calls
 
 // The learned importance proposal's configuration, network, replay buffer and
 // per-call buffers (proposal.hpp).
@@ -84,6 +85,8 @@ struct ProposalState {
   DevBuf<float> bX, bY, bM;              // replay ring, cap rows
   DevBuf<float> Xb, Yb, Mb;              // training batch
   DevBuf<float> Z1, A1, Z2, A2, Out, dOut, dA, dA2;  // activations, max(batch, m) rows
+  DevBuf<float> work;                    // the backward's partial sums
+  DevBuf<float> given;                   // loss_and_gradient: the caller's batch and its activations
   DevBuf<double> fsum, loss;
   DevBuf<double> mq, nq, sq, Uq64, cst, lr, logw;
   DevBuf<float> Uq32;
@@ -92,7 +95,7 @@ struct ProposalState {
   }
   void release() {
     for (auto *b : {&w, &grad, &m1, &m2, &X, &Y, &M, &bX, &bY, &bM, &Xb, &Yb, &Mb, &Z1, &A1, &Z2,
-                    &A2, &Out, &dOut, &dA, &dA2, &Uq32})
+                    &A2, &Out, &dOut, &dA, &dA2, &work, &given, &Uq32})
       b->release();
     for (auto *b : {&fsum, &loss, &mq, &nq, &sq, &Uq64, &cst, &lr, &logw}) b->release();
     w16.release();
@@ -769,6 +772,7 @@ int proposal_ensure(sgdlm_engine *h) {
   for (auto *b : {&q.Z1, &q.A1, &q.Z2, &q.A2, &q.dA, &q.dA2}) CK(b->alloc((size_t)rows * H));
   CK(q.Out.alloc((size_t)rows * O));
   CK(q.dOut.alloc((size_t)rows * O));
+  CK(q.work.alloc(mlp_workspace(q.L, cfg.batch)));
   CK(q.fsum.alloc(2 * (size_t)F + 1));
   CK(q.loss.alloc(1));
   CK(q.mq.alloc((size_t)m * P));
@@ -814,11 +818,11 @@ int proposal_train(sgdlm_engine *h) {
     launch_replay_gather(s, B, F, O, q.count, q.cfg.seed, step, q.bX.ptr, q.bY.ptr, q.bM.ptr,
                          q.fsum.ptr, q.Xb.ptr, q.Yb.ptr, q.Mb.ptr);
     mlp_forward(s, q.L, B, q.Xb.ptr, q.w.ptr, q.w16.ptr, q.acts());
-    mlp_loss_backward(s, q.L, B, q.Xb.ptr, q.Yb.ptr, q.Mb.ptr, q.w16.ptr, q.acts(), q.grad.ptr,
-                      q.loss.ptr);
+    mlp_loss_backward(s, q.L, B, q.Xb.ptr, q.Yb.ptr, q.Mb.ptr, q.w16.ptr, q.acts(), q.work.ptr,
+                      q.grad.ptr, q.loss.ptr);
     mlp_adam(s, q.L, q.w.ptr, q.w16.ptr, q.grad.ptr, q.m1.ptr, q.m2.ptr, (float)q.cfg.lr,
              (long)step);
-    h->launches += 16;
+    h->launches += 11;
   }
   q.info.training_calls += 1;
   q.info.samples = (uint64_t)q.count;
@@ -1724,25 +1728,42 @@ int sgdlm_proposal_loss_and_gradient(sgdlm_handle h, size_t batch, const float *
   ProposalState &q = h->prop;
   const MlpLayout &L = q.L;
   const size_t B = batch;
-  DevBuf<float> x, y, mk, g, z1, a1, z2, a2, out, dout, da, da2;
-  DevBuf<double> l;
-  CK(x.alloc(B * L.F));
-  CK(y.alloc(B * L.O));
-  CK(mk.alloc(B * L.O));
-  CK(g.alloc(L.total));
-  for (auto *b : {&z1, &a1, &z2, &a2, &da, &da2}) CK(b->alloc(B * L.H));
-  CK(out.alloc(B * L.O));
-  CK(dout.alloc(B * L.O));
-  CK(l.alloc(1));
-  if ((st = h2d(h, x.ptr, X, B * L.F * sizeof(float)))) return st;
-  if ((st = h2d(h, y.ptr, Y, B * L.O * sizeof(float)))) return st;
-  if ((st = h2d(h, mk.ptr, mask, B * L.O * sizeof(float)))) return st;
-  const MlpActs a{z1.ptr, a1.ptr, z2.ptr, a2.ptr, out.ptr, dout.ptr, da.ptr, da2.ptr};
-  mlp_forward(h->stream, L, (int)B, x.ptr, q.w.ptr, q.w16.ptr, a);
-  mlp_loss_backward(h->stream, L, (int)B, x.ptr, y.ptr, mk.ptr, q.w16.ptr, a, g.ptr, l.ptr);
-  h->launches += 13;
-  if (loss && (st = d2h(h, loss, l.ptr, sizeof(double)))) return st;
-  if (grad && (st = d2h(h, grad, g.ptr, L.total * sizeof(float)))) return st;
+  // one workspace for the batch, its activations and the gradient, kept between
+  // calls up to kGivenKept
+  size_t need = 0;
+  auto take = [&](size_t n) {
+    const size_t at = need;
+    need += (n + 3) / 4 * 4;
+    return at;
+  };
+  const size_t o_l = take(2), o_x = take(B * L.F), o_y = take(B * L.O), o_mk = take(B * L.O),
+               o_g = take(L.total), o_w = take(mlp_workspace(L, (int)B));
+  size_t o_h[6];
+  for (size_t &o : o_h) o = take(B * L.H);
+  const size_t o_out = take(B * L.O), o_dout = take(B * L.O);
+  if (q.given.count < need) {
+    q.given.release();
+    CK(cudaMalloc(&q.given.ptr, need * sizeof(float)));
+    q.given.count = need;
+  }
+  float *w = q.given.ptr;
+  double *l = reinterpret_cast<double *>(w + o_l);
+  struct Drop {  // a large workspace is given back at the end of the call
+    DevBuf<float> &b;
+    ~Drop() {
+      if (b.count * sizeof(float) > kGivenKept) b.release();
+    }
+  } drop{q.given};
+  if ((st = h2d(h, w + o_x, X, B * L.F * sizeof(float)))) return st;
+  if ((st = h2d(h, w + o_y, Y, B * L.O * sizeof(float)))) return st;
+  if ((st = h2d(h, w + o_mk, mask, B * L.O * sizeof(float)))) return st;
+  const MlpActs a{w + o_h[0], w + o_h[1], w + o_h[2],  w + o_h[3],
+                  w + o_out,  w + o_dout, w + o_h[4], w + o_h[5]};
+  mlp_forward(h->stream, L, (int)B, w + o_x, q.w.ptr, q.w16.ptr, a);
+  mlp_loss_backward(h->stream, L, (int)B, w + o_x, w + o_y, w + o_mk, q.w16.ptr, a, w + o_w, w + o_g, l);
+  h->launches += 9;
+  if (loss && (st = d2h(h, loss, l, sizeof(double)))) return st;
+  if (grad && (st = d2h(h, grad, w + o_g, L.total * sizeof(float)))) return st;
   return sync(h);
 }
 

@@ -64,10 +64,12 @@ struct MlpActs {
 void mlp_forward(cudaStream_t s, const MlpLayout &L, int B, const float *X, const float *w,
                  const __nv_bfloat16 *w16, MlpActs a);
 // Masked MSE of a.Out against Y and the gradient of every parameter into grad
-// (flat layout); the forward must have run on the same X.
+// (flat layout); the forward must have run on the same X.  work: mlp_workspace
+// floats, 8-byte aligned.
+size_t mlp_workspace(const MlpLayout &L, int B);
 void mlp_loss_backward(cudaStream_t s, const MlpLayout &L, int B, const float *X, const float *Y,
-                       const float *mask, const __nv_bfloat16 *w16, MlpActs a, float *grad,
-                       double *loss);
+                       const float *mask, const __nv_bfloat16 *w16, MlpActs a, float *work,
+                       float *grad, double *loss);
 void mlp_adam(cudaStream_t s, const MlpLayout &L, float *w, __nv_bfloat16 *w16, const float *grad,
               float *m1, float *m2, float lr, long step);
 void mlp_refresh_bf16(cudaStream_t s, const MlpLayout &L, const float *w, __nv_bfloat16 *w16);

@@ -296,3 +296,31 @@ def test_low_ess_falls_back_to_plain_proposal(built_lib):
     assert info["ess_learned"] < 0.5 * n and info["ess_plain"] > 0.5 * n
     assert abs(1.0 / np.sum(vb["IS_weights"] ** 2) - info["ess_plain"]) < 1e-6 * n
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("max_p,batch", [(1, 1), (4, 63), (5, 65), (15, 4096), (16, 4160), (24, 300), (24, 9001)])
+def test_gradient_chunks_and_tiles(built_lib, max_p, batch):
+    """The gradient's sums over chunks of the batch and 64 x 64 tiles of each layer, at
+    their edges (a chunk of one row, more than 64 chunks' rows, tiles of one column),
+    against the FP64 restatement with the same BF16 weights.  FP32 sums of `batch`
+    products: relative error at most sqrt(batch) 2^-24 of the gradient's norm with
+    some room for the forward's rounding, 2e-5 in all."""
+    from gpusgdlm_gb300 import SGDLM
+    from oracle import mlp
+
+    F, O = 2 * max_p + 5, 2 * max_p + 2
+    rng = np.random.default_rng(batch)
+    s = SGDLM(1, strict=True)
+    s.setSimultaneousParents(np.full(3, max_p), np.full((max_p, 3), np.nan))
+    n, _, _ = s.proposalSizes()
+    w = (0.1 * rng.normal(size=n)).astype(np.float32)
+    s.setProposalParams(w)
+    X = rng.normal(size=(batch, F)).astype(np.float32)
+    Y = rng.normal(size=(batch, O)).astype(np.float32)
+    M = (rng.random((batch, O)) < 0.7).astype(np.float32)
+    loss, grad = s.proposalLossAndGradient(X, Y, M)
+    ref_loss, ref = mlp.loss_and_gradient(w, X, Y, M, F, O)
+    assert abs(loss - ref_loss) <= 1e-5 * ref_loss
+    assert np.linalg.norm(grad - ref) <= 2e-5 * np.linalg.norm(ref)
+    s.close()
