@@ -330,9 +330,10 @@ class SGDLM:
             return None
         n = self.nsim
         F3 = np.asfortranarray(F.reshape(P, m, K, order="F"))
-        y = np.zeros((m, n, K), order="F")
-        lam = np.zeros((m, n, K), order="F") if debug else None
-        th = np.zeros((P, m, n, K), order="F") if debug else None
+        # every horizon's draws are written into their own (contiguous) slice
+        y = np.empty((m, n, K), order="F")
+        lam = np.empty((m, n, K), order="F") if debug else None
+        th = np.empty((P, m, n, K), order="F") if debug else None
         if G4 is not None and not self._check(self._lib.sgdlm_manage_evo_memory(self._h, 1)):
             return None  # RcppWrapper.cpp:649
         if not self._check(self._lib.sgdlm_init_forecast_priors(self._h)):
@@ -345,16 +346,10 @@ class SGDLM:
             elif k > 0 and not self._check(self._lib.sgdlm_evolve_forecast_samples(self._h)):
                 return None
             xk = np.asfortranarray(F3[:, :, k])
-            yk = np.zeros((m, n), order="F")
-            lk = np.zeros((m, n), order="F") if debug else None
-            tk = np.zeros((P, m, n), order="F") if debug else None
             if not self._check(self._lib.sgdlm_compute_forecast(
-                    self._h, _pd(yk), _pd(xk), _pd(lk), _pd(tk), 1 if k > 0 else 0)):
+                    self._h, _pd(y[:, :, k]), _pd(xk), _pd(lam[:, :, k]) if debug else None,
+                    _pd(th[:, :, :, k]) if debug else None, 1 if k > 0 else 0)):
                 return None
-            y[:, :, k] = yk
-            if debug:
-                lam[:, :, k] = lk
-                th[:, :, :, k] = tk
         if F.ndim == 2:
             y = y[:, :, 0]
             if debug:
