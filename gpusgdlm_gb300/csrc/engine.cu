@@ -203,7 +203,9 @@ struct sgdlm_engine {
   int g_nnz = 0;  // Gamma entries (rows' CSR length)
   DevBuf<double> logdet, w, y_fc, nu_fc, stats6, wpart, part_a, part_b;
   DevBuf<int> draw_flags, series_flags;
-  DevBuf<int> pivot_list;  // nsim + 1: count, then the draws flagged for the redo
+  // nsim + 2: the work counter of k_logdet64, then the count of the draws flagged for
+  // the redo and their list
+  DevBuf<int> pivot_list;
   DevBuf<double> mean_m, mean_C, mean_n, mean_s, mean_lambda, mean_log_lambda, mean_Q;
   DevBuf<uint32_t> dev_epoch;
   LuPlan plan{};
@@ -633,7 +635,7 @@ int alloc_sim(sgdlm_engine *h, size_t nsim) {
   CK(h->y_fc.reserve(nsim * m));
   CK(h->nu_fc.reserve(nsim * m));
   CK(h->draw_flags.reserve(nsim));
-  CK(h->pivot_list.reserve(nsim + 1));
+  CK(h->pivot_list.reserve(nsim + 2));
   CK(h->jac_list.reserve(nsim + 1));
   CK(h->part_a.reserve((size_t)h->chunks * m * (P + 2) + m * P));
   CK(h->part_b.reserve((size_t)h->chunks * m * P * P));
@@ -753,7 +755,8 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
     h->launches += 1;
   }
   // the fast pass appends the draws it flags to pivot_list; the redo visits those
-  CK(cudaMemsetAsync(h->pivot_list.ptr, 0, sizeof(int), h->stream));
+  CK(cudaMemsetAsync(h->pivot_list.ptr, 0, 2 * sizeof(int), h->stream));
+  int *next = h->pivot_list.ptr, *pivot_list = next + 1;
   bool deep = false;
   if constexpr (std::is_same<T, double>::value) {
     // log|det| of FP64 draws: the deep elimination where there is one (2 to 30 times
@@ -761,15 +764,15 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
     deep = !x && h->deep_launch.ok;
     if (deep)
       launch_logdet64(h->stream, h->deep_launch, n, h->deep_dev, as<T>(h->theta_g),
-                      as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, h->pivot_list.ptr);
+                      as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, pivot_list, next);
   }
   if (!deep) launch_lu<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
                as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x, as<T>(h->lambda), key,
-               refine, y, rows, x ? h->nu_fc.ptr : nullptr, h->pivot_list.ptr,
+               refine, y, rows, x ? h->nu_fc.ptr : nullptr, pivot_list,
                iterative ? h->jac_list.ptr : nullptr);
   launch_lu_fallback<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
                         as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x,
-                        as<T>(h->lambda), key, y, rows, h->pivot_list.ptr);
+                        as<T>(h->lambda), key, y, rows, pivot_list);
   h->launches += 2;
   return SGDLM_OK;
 }

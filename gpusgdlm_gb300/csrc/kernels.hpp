@@ -158,7 +158,8 @@ void launch_lu(cudaStream_t s, const LuPlan &plan, long n, const EliminationPlan
                // the same form: only the listed draws are factored, or nullptr: all
                const int *draw_list = nullptr);
 // log|det| of FP64 draws by the deep elimination of elimination.hpp (logdet64.cu).
-// Draws whose elimination needs pivoting are appended to pivot_list.
+// Draws whose elimination needs pivoting are appended to pivot_list; next: the
+// blocks' work counter, zero on entry.
 struct LogdetPlan;
 struct Logdet64Launch {
   int ok, threads, grid;
@@ -169,7 +170,7 @@ int logdet64_max_slots();  // live values (doubles) that a block's shared memory
 Logdet64Launch plan_logdet64_launch(const LogdetPlan &pl, long n, int num_sms, int max_grid);
 void launch_logdet64(cudaStream_t s, const Logdet64Launch &L, long n, const LogdetPlan &pl,
                      const double *theta_g, double *slabs, double *logdet, int *draw_flags,
-                     int *pivot_list);
+                     int *pivot_list, int *next);
 // Forecast solves by fixed-point iteration on the sparse Gamma_i
 // (forecast_kernels.cu).  ok = 0: every draw keeps the factorising path.
 struct JacobiPlan {

@@ -11,7 +11,10 @@
 // multiplied up (their product kept as a mantissa and an exponent) and one logarithm
 // (30 FMAs) is taken per draw, reciprocals (5 FMAs) are taken once per pivot, and
 // blocks are as small as the dense part allows (32 .. 512 threads): the levels' and
-// columns' latencies of one draw are covered by the others on the SM.  10 000 draws:
+// columns' latencies of one draw are covered by the others on the SM.  A block takes
+// its next draw from a counter: where several engines share the GPU, a block whose SM
+// was held by another engine's kernel starts late and takes fewer (three engines' steps
+// at m = 400 in turn: 62.3 ms a step with a fixed share per block, 56.0 ms).  10 000 draws:
 // m = 400 40.7 ms (76 % of the FP64 pipe; one block per SM, so the panels' columns are
 // not covered), 94.5 ms with four levels and the 224 x 224 core; m = 100 0.46 ms
 // (13.0 ms); m = 200 3.3 ms.  Panels of 16 columns: 45.2 ms at m = 400.
@@ -95,19 +98,23 @@ template <int NT>
 __global__ void __launch_bounds__(NT, NT == 512 ? 1 : kWarpsPerSm * 32 / NT)
     k_logdet64(long n, LogdetPlan pl, int m_at, const double *__restrict__ theta_g,
                double *__restrict__ slabs, size_t slab_elems, double *__restrict__ logdet,
-               int *__restrict__ draw_flags, int *__restrict__ pivot_list) {
+               int *__restrict__ draw_flags, int *__restrict__ pivot_list, int *__restrict__ next) {
   constexpr int NW = NT / 32;
   extern __shared__ __align__(16) double vals[];  // the slots, and the dense part M at m_at
   __shared__ double prow[2][kW + 1];               // a panel's pivot row (16: its reciprocal)
   __shared__ double red_m[NW];
   __shared__ int red_e[NW], red_b[NW];
+  __shared__ unsigned s_next;                      // the block's next draw
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nc = pl.core_n, ld = pl.ld, cells = ld * nc;
-  for (long i = blockIdx.x; i < n; i += gridDim.x) {
+  for (long i = blockIdx.x; i < n;) {
     bool bad = false;
     Product prod;
     // ---- the draw's values
-    if (tid == 0) vals[kSlotZero] = 0.0;
+    if (tid == 0) {
+      vals[kSlotZero] = 0.0;
+      s_next = gridDim.x + (unsigned)atomicAdd(next, 1);
+    }
     for (int r = tid; r < pl.m; r += NT) vals[pl.diag_slot[r]] = 1.0;
     const double *th = theta_g + (size_t)i * pl.nnz0;
     for (int q = tid; q < pl.nnz0; q += NT) vals[pl.l0_slot[q]] = -th[q];
@@ -277,6 +284,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : kWarpsPerSm * 32 / NT)
         if (q < n) pivot_list[1 + q] = (int)i;
       }
     }
+    i = (long)s_next;
     group_sync<NT>();
   }
 }
@@ -331,11 +339,11 @@ Logdet64Launch plan_logdet64_launch(const LogdetPlan &pl, long n, int num_sms, i
 
 void launch_logdet64(cudaStream_t s, const Logdet64Launch &L, long n, const LogdetPlan &pl,
                      const double *theta_g, double *slabs, double *logdet, int *draw_flags,
-                     int *pivot_list) {
+                     int *pivot_list, int *next) {
   with_kernel(L.threads, [&](auto kernel) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
     kernel<<<L.grid, L.threads, L.smem, s>>>(n, pl, L.m_at, theta_g, slabs, L.slab_elems, logdet,
-                                             draw_flags, pivot_list);
+                                             draw_flags, pivot_list, next);
   });
 }
 
