@@ -34,6 +34,7 @@
 #include "elimination.hpp"
 #include "kernels.hpp"
 #include "proposal.hpp"
+#include "rng.cuh"
 
 using namespace sgdlm;
 
@@ -208,6 +209,7 @@ struct sgdlm_engine {
   DevBuf<int> pivot_list;
   DevBuf<double> mean_m, mean_C, mean_n, mean_s, mean_lambda, mean_log_lambda, mean_Q;
   DevBuf<uint32_t> dev_epoch;
+  DevBuf<double> tab64;  // RngKey::tab, made with the first FP64 simulation memory
   LuPlan plan{};
   LuOptions lu_opt{};
   JacobiPlan jac32{}, jac64{};  // iterative forecast solves of FP32 and FP64 draws
@@ -290,7 +292,7 @@ struct sgdlm_engine {
   }
   size_t tsize() const { return precision == SGDLM_PRECISION_FP64 ? sizeof(double) : sizeof(float); }
   RngKey key(uint32_t ep) const {
-    return RngKey{(uint32_t)(seed & 0xffffffffu), (uint32_t)(seed >> 32), ep, nullptr};
+    return RngKey{(uint32_t)(seed & 0xffffffffu), (uint32_t)(seed >> 32), ep, nullptr, tab64.ptr};
   }
 };
 
@@ -615,11 +617,44 @@ int plan_sim(sgdlm_engine *h, long n, LuPlan *out) {
   return SGDLM_OK;
 }
 
+// The table of rng.cuh's FP64 logarithm, sine and cosine.
+std::vector<double> trig_log_table() {
+  std::vector<double> t(kTabSize, 0.0);
+  const long double pi = acosl(-1.0L), grid = ldexpl(1.0L, 42);
+  const long double ln2 = logl(2.0L), ln2_hi = kLn2Hi;
+  for (int i = 0; i < 1024; ++i) {
+    const long double a = 2.0L * pi * i / 1024.0L;
+    t[2 * i] = i % 512 == 256 ? 0.0 : (double)cosl(a);
+    t[2 * i + 1] = i % 512 == 0 ? 0.0 : (double)sinl(a);
+  }
+  for (int j = 0; j < kLogIntervals; ++j) {
+    long double c = 1.0L + (j + 0.5L) / kLogIntervals;
+    if (j >= kLogIntervals / 2) c *= 0.5L;
+    if (j == 0 || j == kLogIntervals - 1) c = 1.0L;
+    const double inv = (double)(1.0L / c);
+    const long double l = -logl((long double)inv), hi = roundl(l * grid) / grid;
+    double *e = &t[kTabLog + 4 * j];
+    e[0] = inv;
+    e[1] = (double)hi;
+    e[2] = (double)(l - hi);
+  }
+  for (int k = 0; k < 34; ++k) {
+    t[kTabLn2 + 2 * k] = (double)(-k * ln2_hi);
+    t[kTabLn2 + 2 * k + 1] = (double)(-k * (ln2 - ln2_hi));
+  }
+  return t;
+}
+
 int alloc_sim(sgdlm_engine *h, size_t nsim) {
   const size_t m = h->m, P = h->P, ts = h->tsize();
   LuPlan pl;
   int st = plan_sim(h, (long)nsim, &pl);
   if (st) return st;
+  if (h->precision == SGDLM_PRECISION_FP64 && !h->tab64.ptr) {
+    static const std::vector<double> table = trig_log_table();
+    CK(h->tab64.alloc(table.size()));
+    CK(cudaMemcpy(h->tab64.ptr, table.data(), table.size() * sizeof(double), cudaMemcpyHostToDevice));
+  }
   // grow-only: a smaller draw count (e.g. forecasts of fewer draws between VB
   // calls with more) keeps the allocations, so that alternating counts do not
   // free and allocate gigabytes every call; every buffer is written before it
@@ -784,7 +819,7 @@ template <typename T> void vb_moments(sgdlm_engine *h, double *w) {
   launch_vb<T>(h->stream, m, P, n, h->p.ptr, h->n_t.ptr, h->s_t.ptr, w, as<T>(h->lambda),
                as<T>(h->theta), scr, h->mean_m.ptr, h->mean_C.ptr, h->mean_n.ptr,
                h->mean_s.ptr, h->mean_lambda.ptr, h->mean_log_lambda.ptr, h->mean_Q.ptr,
-               h->series_flags.ptr);
+               h->series_flags.ptr, h->tab64.ptr);
   h->launches += 4;
 }
 

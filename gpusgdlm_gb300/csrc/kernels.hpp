@@ -35,6 +35,7 @@ enum : int {
 struct RngKey {
   uint32_t k0, k1, epoch;
   const uint32_t *dev_epoch;
+  const double *tab;  // table of the FP64 logarithm, sine and cosine (rng.cuh); FP64 draws
 };
 
 // Advances the device-side epoch counter by `delta` (fused step).
@@ -232,7 +233,9 @@ void launch_vb(cudaStream_t s, int m, int P, long n, const unsigned *p,
                const double *n_t, const double *s_t, const double *w, const T *lambda,
                const T *theta, VbScratch scr, double *mean_m, double *mean_C,
                double *mean_n, double *mean_s, double *mean_lambda,
-               double *mean_log_lambda, double *mean_Q, int *series_flags);
+               double *mean_log_lambda, double *mean_Q, int *series_flags,
+               // RngKey::tab (FP64 draws)
+               const double *tab);
 
 // Device-side ESS gate of the fused filter step: copy (mean_m, mean_C, mean_n,
 // mean_s) into the state when stats[1] (ESS) > threshold.

@@ -263,7 +263,7 @@ __device__ void forecast_rhs(int m, int P, long n, long i, GammaRows rows, Theta
   for (int j = threadIdx.x; j < m; j += blockDim.x) {
     const U4 g = philox((uint32_t)i, (uint32_t)j, tag_sub(TAG_NU, 0), ep, key.k0, key.k1);
     T z0, z1;
-    box_muller<T>(g.x, g.y, z0, z1);
+    box_muller<T>(g.x, g.y, z0, z1, key.tab);
     const T lam = lambda[(size_t)j * n + i];
     double v = (double)(z0 / dev_sqrt(lam));
     const T *th = theta.row(i, j);
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(128)
   const uint32_t ep = key_epoch(key);
   const U4 g = philox((uint32_t)i, (uint32_t)j, tag_sub(TAG_NU, 0), ep, key.k0, key.k1);
   T z0, z1;
-  box_muller<T>(g.x, g.y, z0, z1);
+  box_muller<T>(g.x, g.y, z0, z1, key.tab);
   const T lam = lambda[(size_t)j * n + i];
   const T *th = theta + ((size_t)j * n + i) * P;
   if constexpr (sizeof(T) == 4) {

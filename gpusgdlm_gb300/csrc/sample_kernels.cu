@@ -67,7 +67,8 @@ __global__ void __launch_bounds__(kSampleThreads)
   T *Us = reinterpret_cast<T *>(smem_raw);  // P*P, U[row + P*col]
   T *ms = Us + P * P;                       // P
   T *stage = ms + P;                        // blockDim.x * P
-  __shared__ T ser[3];                      // the series' gamma shape and rate, s_j
+  __shared__ GammaShape<T> shape;           // the series' gamma shape
+  __shared__ T ser[2];                      // its rate, s_j
   __shared__ int gks[64], gcnt, gq0;        // its Gamma coefficients (gamma_row_of)
   const int j = blockIdx.y;
   // the series' active coefficients: U_j is zero outside its leading pj x pj
@@ -82,33 +83,33 @@ __global__ void __launch_bounds__(kSampleThreads)
   if (threadIdx.x == 0) {
     // FP64 once per series (FP64 is a narrow pipe on this GPU)
     const double nj = n_t[j], sj = s_t[j];
-    ser[0] = (T)(0.5 * nj);
-    ser[1] = (T)(0.5 * nj * sj);
-    ser[2] = (T)sj;
+    shape = gamma_shape<T>((T)(0.5 * nj), false);
+    ser[0] = (T)(0.5 * nj * sj);
+    ser[1] = (T)sj;
   }
   __syncthreads();
   const long i0 = (long)blockIdx.x * blockDim.x;
   const long i = i0 + threadIdx.x;
   if (i < n) {
     const uint32_t ep = key_epoch(key);
-    const T alpha = ser[0], rate = ser[1];
+    const T rate = ser[0];
     bool fail = false;
-    const T lam = gamma_mt<T>(alpha, (uint32_t)i, (uint32_t)j, TAG_GAMMA, ep, key.k0,
-                              key.k1, false, &fail) / rate;
+    const T lam = gamma_mt<T>(shape, (uint32_t)i, (uint32_t)j, TAG_GAMMA, ep, key.k0,
+                              key.k1, key.tab, &fail) / rate;
     T z[PMAX];
 #pragma unroll
     for (int q = 0; q < PMAX / 4; ++q) {
       if (4 * q < pj) {
         const U4 r = philox((uint32_t)i, (uint32_t)j, tag_sub(TAG_THETA, q), ep, key.k0, key.k1);
-        box_muller<T>(r.x, r.y, z[4 * q], z[4 * q + 1]);
-        box_muller<T>(r.z, r.w, z[4 * q + 2], z[4 * q + 3]);
+        box_muller<T>(r.x, r.y, z[4 * q], z[4 * q + 1], key.tab);
+        box_muller<T>(r.z, r.w, z[4 * q + 2], z[4 * q + 3], key.tab);
       } else {
         z[4 * q] = z[4 * q + 1] = z[4 * q + 2] = z[4 * q + 3] = T(0);
       }
     }
     // theta = m + (U' z) / sqrt(s lambda)   (makeVB_MVN, kernel_functions.cuh:72-83);
     // one reciprocal instead of P divisions (within 1-2 ulp of the quotients)
-    const T rden = T(1) / dev_sqrt(ser[2] * lam);
+    const T rden = T(1) / dev_sqrt(ser[1] * lam);
     T *row = stage + (size_t)threadIdx.x * P;
 #pragma unroll
     for (int k = 0; k < PMAX; ++k) {
@@ -156,8 +157,14 @@ __global__ void __launch_bounds__(kSampleThreads)
   T *Gs = Us + P * P;  // G_j when an evolution matrix is given
   T *stage = Gs + (G ? P * P : 0);
   __shared__ int gks[64], gcnt, gq0;  // the series' Gamma coefficients (gamma_row_of)
+  __shared__ GammaShape<T> shapes[2];  // of the Beta draw's two gammas
   const int j = blockIdx.y;
-  if (gd.v && (threadIdx.x >> 5) == 0)
+  if (threadIdx.x < 64 && threadIdx.x % 32 == 0) {  // one thread of warps 0 and 1 each
+    const double bj = beta[j], rj = r_t[j];
+    const bool second = threadIdx.x == 32;
+    shapes[second] = gamma_shape<T>((T)(second ? 0.5 * (1.0 - bj) * rj : 0.5 * bj * rj), compat_no_boost);
+  }
+  if (gd.v && (threadIdx.x >> 5) == 2)
     gamma_row_of(gd.sp, gd.rowptr, j, P, (unsigned)m * (unsigned)m, gks, &gcnt, &gq0);
   const long i0 = (long)blockIdx.x * blockDim.x;
   const long cnt = (long)min((long)blockDim.x, n - i0) * P;
@@ -170,15 +177,14 @@ __global__ void __launch_bounds__(kSampleThreads)
   const long i = i0 + threadIdx.x;
   if (i < n) {
     const uint32_t ep = key_epoch(key);
-    const double bj = beta[j], rj = r_t[j];
+    const double bj = beta[j];
     bool fail = false;
     T eta = T(1);
     if (bj != 1.0) {
-      const T ga = gamma_mt<T>((T)(0.5 * bj * rj), (uint32_t)i, (uint32_t)j, TAG_BETA_A,
-                               ep, key.k0, key.k1, compat_no_boost, &fail);
-      const T gb = gamma_mt<T>((T)(0.5 * (1.0 - bj) * rj), (uint32_t)i, (uint32_t)j,
-                               TAG_BETA_B, ep, key.k0, key.k1, compat_no_boost,
-                               &fail);
+      const T ga = gamma_mt<T>(shapes[0], (uint32_t)i, (uint32_t)j, TAG_BETA_A, ep, key.k0, key.k1,
+                               key.tab, &fail);
+      const T gb = gamma_mt<T>(shapes[1], (uint32_t)i, (uint32_t)j, TAG_BETA_B, ep, key.k0, key.k1,
+                               key.tab, &fail);
       eta = (ga / (ga + gb)) / (T)bj;
     }
     const T lam = lambda[(size_t)j * n + i] * eta;
@@ -188,8 +194,8 @@ __global__ void __launch_bounds__(kSampleThreads)
     for (int q = 0; q < PMAX / 4; ++q) {
       if (4 * q < P) {
         const U4 r = philox((uint32_t)i, (uint32_t)j, tag_sub(TAG_OMEGA, q), ep, key.k0, key.k1);
-        box_muller<T>(r.x, r.y, w[4 * q], w[4 * q + 1]);
-        box_muller<T>(r.z, r.w, w[4 * q + 2], w[4 * q + 3]);
+        box_muller<T>(r.x, r.y, w[4 * q], w[4 * q + 1], key.tab);
+        box_muller<T>(r.z, r.w, w[4 * q + 2], w[4 * q + 3], key.tab);
       } else {
         w[4 * q] = w[4 * q + 1] = w[4 * q + 2] = w[4 * q + 3] = T(0);
       }

@@ -22,6 +22,7 @@
 //  * the Newton solve for the gamma shape uses the reference's own asymptotic
 //    digamma/trigamma series and stopping rule, in FP64.
 #include "kernels.hpp"
+#include "rng.cuh"
 
 namespace sgdlm {
 namespace {
@@ -162,9 +163,6 @@ __global__ void __launch_bounds__(kWThreads)
   }
 }
 
-template <typename T> __device__ __forceinline__ T tlog(T v);
-template <> __device__ __forceinline__ float tlog<float>(float v) { return logf(v); }
-template <> __device__ __forceinline__ double tlog<double>(double v) { return log(v); }
 template <typename T> __device__ __forceinline__ T tsqrt(T v);
 template <> __device__ __forceinline__ float tsqrt<float>(float v) { return sqrtf(v); }
 template <> __device__ __forceinline__ double tsqrt<double>(double v) { return sqrt(v); }
@@ -174,7 +172,7 @@ template <typename T, int PMAX>
 __global__ void __launch_bounds__(kVbThreads)
     k_vb_a(int m, int P, long n, long chunk, const double *__restrict__ w,
            const T *__restrict__ lambda, const T *__restrict__ theta,
-           double *__restrict__ part_a) {
+           double *__restrict__ part_a, const double *__restrict__ tab) {
   __shared__ double red[32];
   const int j = blockIdx.y, c = blockIdx.x;
   const long i0 = (long)c * chunk;
@@ -189,7 +187,7 @@ __global__ void __launch_bounds__(kVbThreads)
     const T lam = lambda[(size_t)j * n + i];
     const T wl = wi * lam;
     sl += wl;
-    sll += wi * tlog(lam);
+    sll += wi * dev_log(lam, tab);
     const T *th = theta + ((size_t)j * n + i) * P;
     if (vec_rows) {
       // 16-byte loads of the row (P * sizeof(T) a multiple of 16)
@@ -709,18 +707,18 @@ void launch_vb(cudaStream_t s, int m, int P, long n, const unsigned *p, const do
                const double *s_t, const double *w, const T *lambda, const T *theta,
                VbScratch scr, double *mean_m, double *mean_C, double *mean_n,
                double *mean_s, double *mean_lambda, double *mean_log_lambda,
-               double *mean_Q, int *series_flags) {
+               double *mean_Q, int *series_flags, const double *tab) {
   const int chunks = scr.chunks;
   const long chunk = scr.chunk_draws;
   dim3 grid((unsigned)chunks, (unsigned)m);
   if (P <= 8)
-    k_vb_a<T, 8><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a);
+    k_vb_a<T, 8><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a, tab);
   else if (P <= 16)
-    k_vb_a<T, 16><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a);
+    k_vb_a<T, 16><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a, tab);
   else if (P <= 32)
-    k_vb_a<T, 32><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a);
+    k_vb_a<T, 32><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a, tab);
   else
-    k_vb_a<T, 64><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a);
+    k_vb_a<T, 64><<<grid, kVbThreads, 0, s>>>(m, P, n, chunk, w, lambda, theta, scr.part_a, tab);
   // mbar_full lives in mean_m's slot until the refit overwrites it with the cut mean;
   // a separate buffer keeps the kernels independent.
   double *mbar_full = scr.part_a + (size_t)chunks * m * (P + 2);
@@ -774,11 +772,12 @@ void launch_vb(cudaStream_t s, int m, int P, long n, const unsigned *p, const do
 template void launch_vb<float>(cudaStream_t, int, int, long, const unsigned *,
                                const double *, const double *, const double *,
                                const float *, const float *, VbScratch, double *, double *,
-                               double *, double *, double *, double *, double *, int *);
+                               double *, double *, double *, double *, double *, int *,
+                               const double *);
 template void launch_vb<double>(cudaStream_t, int, int, long, const unsigned *,
                                 const double *, const double *, const double *,
                                 const double *, const double *, VbScratch, double *,
                                 double *, double *, double *, double *, double *, double *,
-                                int *);
+                                int *, const double *);
 
 }  // namespace sgdlm
