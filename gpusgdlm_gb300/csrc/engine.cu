@@ -748,7 +748,7 @@ void sample_draws(sgdlm_engine *h, const double *m_t, const double *C_t, const d
   h->launches += 2;
 }
 
-// Small systems: one warp per draw, partial pivoting, no redo.
+// Small systems: a warp or part of one per draw, partial pivoting, no redo.
 bool warp_lu(const sgdlm_engine *h) { return h->m <= (size_t)kWarpLuMaxM && h->lu_opt.allow_warp; }
 
 // Forecasts are solved iteratively first (block LU path only).
@@ -774,9 +774,9 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
     h->launches += 2;
   }
   if (warp_lu(h)) {
-    launch_lu_warp<T>(h->stream, (int)h->m, (int)h->P, n, h->num_sms, h->sp.ptr, as<T>(h->theta),
-                      h->logdet.ptr, h->draw_flags.ptr,
-                      x ? h->nu_fc.ptr : nullptr, x ? y : nullptr);
+    launch_lu_warp<T>(h->stream, (int)h->m, n, h->num_sms, rows, as<T>(h->theta_g), h->g_nnz,
+                      h->logdet.ptr, h->draw_flags.ptr, x ? h->nu_fc.ptr : nullptr, x ? y : nullptr,
+                      h->tab64.ptr);
     h->launches += 1;
     return SGDLM_OK;
   }

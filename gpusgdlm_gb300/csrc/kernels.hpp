@@ -117,13 +117,6 @@ struct LuOptions {
   int allow_warp = 1;  // m <= kWarpLuMaxM: one warp per draw (launch_lu_warp)
 };
 constexpr int kWarpLuMaxM = 32;
-// Warp-per-draw LU with partial pivoting for m <= kWarpLuMaxM: log|det| of every
-// draw and, when y != nullptr, the forecast solve y_i = (I - Gamma_i)^-1 nu_i
-// (nu series-major, nu[r*n + i]; y draw-major, y[i*m + r]).
-template <typename T>
-void launch_lu_warp(cudaStream_t s, int m, int P, long n, int num_sms, const unsigned *sp,
-                    const T *theta, double *logdet, int *draw_flags,
-                    const double *nu, double *y);
 // core_n / nv / n_solve / prog_len come from the elimination plan (core_n = m and
 // the others 0 without one).
 template <typename T>
@@ -140,6 +133,14 @@ struct GammaRows {
   const int *ext_ptr;  // m + 1
   const int *ext_k;
 };
+// LU with partial pivoting for m <= kWarpLuMaxM, 4 to 32 lanes per draw: log|det| of
+// every draw and, when y != nullptr, the forecast solve y_i = (I - Gamma_i)^-1 nu_i
+// (nu series-major, nu[r*n + i]; y draw-major, y[i*m + r]).  theta_g: the draws' Gamma
+// entries (GammaDraws layout, nnz per draw); tab: RngKey::tab (FP64 draws).
+template <typename T>
+void launch_lu_warp(cudaStream_t s, int m, long n, int num_sms, GammaRows rows, const T *theta_g,
+                    int nnz, double *logdet, int *draw_flags, const double *nu, double *y,
+                    const double *tab);
 struct EliminationPlan;
 template <typename T>
 // theta: the draws series-major; theta_g: their Gamma entries (GammaDraws layout,

@@ -123,3 +123,26 @@ def test_warp_lu_not_used_above_32(built_lib):
     s.computeVBPosterior(64, 64)
     assert s.getWarpLu() == {"enabled": True, "in_use": False}
     s.close()
+
+
+@pytest.mark.parametrize("m,n", [(1, 5), (2, 33), (4, 31), (5, 9), (8, 1001), (9, 3), (16, 63), (17, 2)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_lanes_per_draw(built_lib, precision, m, n):
+    """4, 8, 16 and 32 lanes per draw at the edges of their ranges, with draw counts that
+    leave part of the last warp without a draw."""
+    s, wl, mt, C = _model(m, min(5, m - 1), precision, 300 + m)
+    s.setPosteriorParameters(mt, C, np.full(m, 20.0), np.full(m, 1.0))
+    s.setRngState(7, 0)
+    s.computeVBPosterior(n, n)
+    d = s.getDraws()
+    ld = oracle.logdet(_spu(wl), np.asfortranarray(d["thetas"].transpose(0, 2, 1)))
+    assert np.abs(d["log_dets"] - ld).max() <= (1e-5 if precision == "mixed" else 1e-12)
+    x = np.asfortranarray(np.random.default_rng(m).normal(size=(wl["P"], m)))
+    s.setPriorParameters(mt, C, np.full(m, 20.0), np.full(m, 1.0))
+    s.setRngState(11, 0)
+    out = s.computeForecastDebug(n, n, x)
+    y, _ = oracle.forecast(_spu(wl), np.asfortranarray(out["lambdas"].T),
+                           np.asfortranarray(out["thetas"].transpose(0, 2, 1)), x, 11, 0)
+    e = (np.abs(out["y"] - y).max(axis=0) / np.abs(y).max(axis=0)).max()
+    assert e <= (1e-5 if precision == "mixed" else 1e-10), e
+    s.close()
