@@ -207,7 +207,7 @@ struct sgdlm_engine {
   // nsim + 2: the work counter of k_logdet64, then the count of the draws flagged for
   // the redo and their list
   DevBuf<int> pivot_list;
-  DevBuf<double> mean_m, mean_C, mean_n, mean_s, mean_lambda, mean_log_lambda, mean_Q;
+  DevBuf<double> mean_m, mean_C, mean_n, mean_s, mean_lambda, mean_log_lambda;
   DevBuf<uint32_t> dev_epoch;
   DevBuf<double> tab64;  // RngKey::tab, made with the first FP64 simulation memory
   LuPlan plan{};
@@ -525,7 +525,6 @@ int alloc_state(sgdlm_engine *h) {
   CK(h->mean_s.alloc(m));
   CK(h->mean_lambda.alloc(m));
   CK(h->mean_log_lambda.alloc(m));
-  CK(h->mean_Q.alloc(m));
   CK(h->series_flags.alloc(m));
   CK(h->stats6.alloc(8));
   CK(h->wpart.alloc(4 * (size_t)kWeightBlocks));
@@ -564,7 +563,7 @@ void release_all(sgdlm_engine *h) {
   for (auto *b : {&h->m_t, &h->C_t, &h->n_t, &h->s_t, &h->W_t, &h->beta, &h->delta, &h->y_t,
                   &h->F_t, &h->x_t, &h->fm_t, &h->fC_t, &h->fn_t, &h->fs_t, &h->fW_t,
                   &h->U64, &h->mean_m, &h->mean_C, &h->mean_n, &h->mean_s, &h->mean_lambda,
-                  &h->mean_log_lambda, &h->mean_Q, &h->stats6, &h->wpart})
+                  &h->mean_log_lambda, &h->stats6, &h->wpart})
     b->release();
   h->U32.release();
   h->p.release();
@@ -818,8 +817,8 @@ template <typename T> void vb_moments(sgdlm_engine *h, double *w) {
   VbScratch scr{h->part_a.ptr, h->part_b.ptr, h->chunks, h->chunk_draws};
   launch_vb<T>(h->stream, m, P, n, h->p.ptr, h->n_t.ptr, h->s_t.ptr, w, as<T>(h->lambda),
                as<T>(h->theta), scr, h->mean_m.ptr, h->mean_C.ptr, h->mean_n.ptr,
-               h->mean_s.ptr, h->mean_lambda.ptr, h->mean_log_lambda.ptr, h->mean_Q.ptr,
-               h->series_flags.ptr, h->tab64.ptr);
+               h->mean_s.ptr, h->mean_lambda.ptr, h->mean_log_lambda.ptr, h->series_flags.ptr,
+               h->tab64.ptr);
   h->launches += 4;
 }
 

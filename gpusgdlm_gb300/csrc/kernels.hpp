@@ -234,7 +234,7 @@ void launch_vb(cudaStream_t s, int m, int P, long n, const unsigned *p,
                const double *n_t, const double *s_t, const double *w, const T *lambda,
                const T *theta, VbScratch scr, double *mean_m, double *mean_C,
                double *mean_n, double *mean_s, double *mean_lambda,
-               double *mean_log_lambda, double *mean_Q, int *series_flags,
+               double *mean_log_lambda, int *series_flags,
                // RngKey::tab (FP64 draws)
                const double *tab);
 

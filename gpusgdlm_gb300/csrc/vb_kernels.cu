@@ -15,10 +15,9 @@
 //    draws; the chunks are sized for the SM count), coalesced over the
 //    series-major draw buffers, FP64 chunk partials; pass B for FP32 draws keeps
 //    the next 128-draw sub-chunk in flight by cp.async;
-//  * Q_bar_j is evaluated as trace(V^-1 V): since V = sum_i w_i theta~_i theta~_i'
-//    with the same weights, sum_i w_i theta~_i' V^-1 theta~_i = tr(V^-1 V)
-//    exactly, so the m*n quadratic forms of the reference collapse to a p x p
-//    trace per series (equal to p_j up to the rounding of V^-1);
+//  * Q_bar_j is p_j: since V = sum_i w_i theta~_i theta~_i' with the same weights,
+//    sum_i w_i theta~_i' V^-1 theta~_i = tr(V^-1 V) = p_j exactly, so neither the m*n
+//    quadratic forms of the reference nor V^-1 are formed;
 //  * the Newton solve for the gamma shape uses the reference's own asymptotic
 //    digamma/trigamma series and stopping rule, in FP64.
 #include "kernels.hpp"
@@ -238,6 +237,22 @@ __global__ void __launch_bounds__(kVbThreads)
   (void)red;
 }
 
+// Sum of `chunks` values, stride apart, in order, eight loads in flight (few series make
+// many chunks: 79 at m = 6, 10 000 draws).
+__device__ __forceinline__ double sum_chunks(const double *__restrict__ src, size_t stride, int chunks) {
+  double v = 0.0;
+  int c = 0;
+  for (; c + 8 <= chunks; c += 8) {
+    double t[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t[q] = src[(size_t)(c + q) * stride];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v += t[q];
+  }
+  for (; c < chunks; ++c) v += src[(size_t)c * stride];
+  return v;
+}
+
 // Combines the chunk partials of pass A: E_w lambda, E_w log lambda, and the
 // uncut weighted mean m_bar = sum w lambda theta / sum w lambda over all P
 // (compute_mean_m_t, kernel_functions.cuh:949-967).
@@ -253,8 +268,7 @@ __global__ void k_vb_a_fin(int m, int P, int chunks, const double *__restrict__ 
   for (int k0 = 0; k0 < P + 2; k0 += 32) {
     const int k = k0 + lane;
     double v = 0.0;
-    if (k < P + 2)
-      for (int c = 0; c < chunks; ++c) v += part_a[((size_t)c * m + j) * (P + 2) + k];
+    if (k < P + 2) v = sum_chunks(part_a + (size_t)j * (P + 2) + k, (size_t)m * (P + 2), chunks);
     if (k0 == 0) {
       sl = __shfl_sync(0xffffffffu, v, 0);
       if (lane == 0) mean_lambda[j] = v;
@@ -528,18 +542,12 @@ __device__ __forceinline__ double psi1_series_r(double r) {
   return r + 0.5 * t + t * r * (1.0 / 6.0 + t * (-1.0 / 30.0 + t * (1.0 / 42.0 + t * (-1.0 / 30.0))));
 }
 
-// Orders |v| like the serial pivot scan's "v > best": the magnitude's bits as an
-// integer (monotone for non-negative doubles), NaN below every number.
-__device__ __forceinline__ long long pivot_key(double v) {
-  const long long b = __double_as_longlong(v) & 0x7fffffffffffffffLL;
-  return b > 0x7ff0000000000000LL ? -1LL : b;
-}
-
-// Per-series refit, one warp per series (FP64):
-//   V (p x p) from the chunk partials; V^-1 by Gauss-Jordan with partial
-//   pivoting; Q_bar = tr(V^-1 V); Newton for n_bar (compute_mean_n_t,
-//   kernel_functions.cuh:1025-1068); s_bar (compute_mean_s_t :1071-1085);
-//   C_bar = V s_bar inside p x p, zero outside; m_bar cut at p.
+// Per-series refit, one warp per series (FP64): V (p x p) from the chunk partials,
+// added in order; Newton for n_bar (compute_mean_n_t, kernel_functions.cuh:1025-1068);
+// s_bar (compute_mean_s_t :1071-1085); C_bar = V s_bar inside p x p, zero outside;
+// m_bar cut at p.  Q_bar = tr(V^-1 V) is p_j whatever V, so V is not inverted (the
+// Gauss-Jordan inversion that formed the trace to within rounding, and replaced it by
+// p_j for a singular V, was 80 of the kernel's 93 us at m = 400).
 __global__ void k_vb_fin(int m, int P, int chunks, const unsigned *__restrict__ p,
                          const double *__restrict__ n_t, const double *__restrict__ s_t,
                          const double *__restrict__ part_b,
@@ -547,124 +555,41 @@ __global__ void k_vb_fin(int m, int P, int chunks, const unsigned *__restrict__ 
                          const double *__restrict__ mean_log_lambda,
                          const double *__restrict__ mbar_full, double *__restrict__ mean_m,
                          double *__restrict__ mean_C, double *__restrict__ mean_n,
-                         double *__restrict__ mean_s, double *__restrict__ mean_Q,
-                         int *__restrict__ series_flags) {
-  extern __shared__ double sh[];
+                         double *__restrict__ mean_s, int *__restrict__ series_flags) {
   const int j = blockIdx.x;
   const int lane = threadIdx.x;
   const int pj = (int)min((unsigned)P, p[j]);
-  double *V = sh;                      // P x P, V[x + P*y]
-  double *G = V + (size_t)P * P;       // p x 2p augmented [V | I], G[r + pj*c]
-  double *f = G + (size_t)2 * P * P;   // multipliers of the current column
-  __shared__ int s_bad;
   __shared__ double s_sb;
-  if (lane == 0) s_bad = 0;
-  for (int e = lane; e < P * P; e += 32) {
-    const int x = e % P, y = e / P;
-    double v = 0.0;
-    if (x < pj && y < pj) {
-      const int a = min(x, y), b = max(x, y);
-      for (int c = 0; c < chunks; ++c) v += part_b[((size_t)c * m + j) * P * P + a + P * b];
-    }
-    V[e] = v;
-  }
-  __syncwarp();
-  for (int e = lane; e < pj * 2 * pj; e += 32) {
-    const int r = e % pj, cidx = e / pj;
-    G[e] = (cidx < pj) ? V[r + P * cidx] : ((cidx - pj) == r ? 1.0 : 0.0);
-  }
-  __syncwarp();
-  // Gauss-Jordan with partial pivoting on [V | I] -> [I | V^-1].  The pivot row is
-  // the first row of the largest |entry| at or below the diagonal, as a serial scan
-  // with "v > best" finds it (a NaN diagonal entry stays the pivot; NaN below it is
-  // never chosen): a warp reduction over integer keys, ties to the lower row.
-  double *grow = f + P;  // the normalised pivot row (2p values)
-  for (int k = 0; k < pj; ++k) {
-    const double dk = G[k + pj * k];
-    long long key = -2;
-    int idx = k;
-    if (lane >= k && lane < pj) {
-      key = lane == k ? pivot_key(dk) : pivot_key(G[lane + pj * k]);
-      idx = lane;
-    }
-    if (pj > 32)
-      for (int r = lane + 32; r < pj; r += 32) {
-        if (r < k) continue;
-        const long long kr = pivot_key(G[r + pj * k]);
-        if (kr > key) key = kr, idx = r;
-      }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long ko = __shfl_xor_sync(0xffffffffu, key, o);
-      const int io = __shfl_xor_sync(0xffffffffu, idx, o);
-      if (ko > key || (ko == key && io < idx)) key = ko, idx = io;
-    }
-    const bool nan_diag = isnan(dk);
-    const int pr = nan_diag ? k : idx;
-    if (lane == 0 && !((nan_diag ? -1LL : key) > 0)) s_bad = 1;  // |pivot| > 0 fails
-    if (pr != k)
-      for (int cidx = lane; cidx < 2 * pj; cidx += 32) {
-        const double t = G[k + pj * cidx];
-        G[k + pj * cidx] = G[pr + pj * cidx];
-        G[pr + pj * cidx] = t;
-      }
-    __syncwarp();
-    const double rpiv = 1.0 / G[k + pj * k];
-    for (int r = lane; r < pj; r += 32) f[r] = G[r + pj * k];
-    __syncwarp();
-    for (int cidx = lane; cidx < 2 * pj; cidx += 32) {
-      const double gk = G[k + pj * cidx] * rpiv;
-      G[k + pj * cidx] = gk;
-      grow[cidx] = gk;
-    }
-    __syncwarp();
-    for (int e = lane; e < 2 * pj * pj; e += 32) {
-      const int r = e % pj, cidx = e / pj;
-      if (r != k) G[e] -= f[r] * grow[cidx];
-    }
-    __syncwarp();
-  }
-  // Q_bar = sum_{x,y} Vinv[x][y] V[y][x]
-  double q = 0.0;
-  for (int e = lane; e < pj * pj; e += 32) {
-    const int x = e % pj, y = e / pj;
-    q += G[x + pj * (pj + y)] * V[y + P * x];
-  }
-  q = warp_sum(q);
   if (lane == 0) {
     const double El = mean_lambda[j], Ell = mean_log_lambda[j];
-    const double pd = (double)p[j];
-    // When the weights collapse onto fewer draws than p_j, V is singular to
-    // working precision and V^-1 is noise; tr(V^-1 V) = p_j is then used as is.
-    bool singular_v = s_bad != 0 || !(fabs(q - (double)pj) <= 1e-8 * (double)(pj > 0 ? pj : 1));
-    if (singular_v) q = (double)pj;
     double mn = n_t[j];
     double fun, dfun, step = 0.0;
     size_t iter = 0;
-    const double log2El = log(2 * El), dq = pd - q;
+    // (the reference's terms in p_j - Q_bar vanish)
+    const double log2El = log(2 * El);
     do {
       mn -= step;
       const double rmn = 1.0 / mn, r = 2.0 * rmn;  // r = 1 / (mn / 2)
-      fun = log(mn + dq) - psi_series_r(log(0.5 * mn), r) - dq * rmn - log2El + Ell;
-      dfun = 1.0 / (mn + dq) - .5 * psi1_series_r(r) + dq * rmn * rmn;
+      const double lmn = log(mn);
+      fun = lmn - psi_series_r(lmn - 0.69314718055994530942, r) - log2El + Ell;
+      dfun = rmn - .5 * psi1_series_r(r);
       step = fun / dfun;
       if (step > mn) step = .5 * mn;
     } while (fabs(fun) > 1e-6 && iter++ < 50);
-    int fl = singular_v ? 1 : 0;
+    int fl = 0;
     // A non-finite iterate ends the reference's loop through the NaN comparison and
     // would be returned as is; it is treated as non-convergence instead.
     if (iter >= 50 || !(fabs(mn) < INFINITY)) {
       mn = n_t[j];
       fl |= 2;
     }
-    double sb = (mn + pd - q) / (mn * El);
+    double sb = 1.0 / El;  // (n_bar + p_j - Q_bar) / (n_bar E lambda)
     if (sb < 0) {
       sb = s_t[j];
       fl |= 4;
     }
     mean_n[j] = mn;
     mean_s[j] = sb;
-    mean_Q[j] = q;
     if (series_flags) series_flags[j] = fl;
     s_sb = sb;
   }
@@ -672,7 +597,12 @@ __global__ void k_vb_fin(int m, int P, int chunks, const unsigned *__restrict__ 
   const double sb = s_sb;
   for (int e = lane; e < P * P; e += 32) {
     const int x = e % P, y = e / P;
-    mean_C[(size_t)j * P * P + e] = (x < pj && y < pj) ? V[e] * sb : 0.0;
+    double v = 0.0;
+    if (x < pj && y < pj) {
+      const double *src = part_b + (size_t)j * P * P + min(x, y) + P * max(x, y);
+      v = sum_chunks(src, (size_t)m * P * P, chunks);
+    }
+    mean_C[(size_t)j * P * P + e] = (x < pj && y < pj) ? v * sb : 0.0;
   }
   for (int k = lane; k < P; k += 32)
     mean_m[(size_t)j * P + k] = (k < pj) ? mbar_full[(size_t)j * P + k] : 0.0;
@@ -707,7 +637,7 @@ void launch_vb(cudaStream_t s, int m, int P, long n, const unsigned *p, const do
                const double *s_t, const double *w, const T *lambda, const T *theta,
                VbScratch scr, double *mean_m, double *mean_C, double *mean_n,
                double *mean_s, double *mean_lambda, double *mean_log_lambda,
-               double *mean_Q, int *series_flags, const double *tab) {
+               int *series_flags, const double *tab) {
   const int chunks = scr.chunks;
   const long chunk = scr.chunk_draws;
   dim3 grid((unsigned)chunks, (unsigned)m);
@@ -726,15 +656,12 @@ void launch_vb(cudaStream_t s, int m, int P, long n, const unsigned *p, const do
                                          mean_log_lambda, mbar_full);
   const size_t PX = (size_t)(P + 3) / 4 * 4;
   const size_t smem_b = ((size_t)kSub * PX + PX + kSub + (size_t)kVbThreads * 16) * sizeof(T);
-  const size_t smem_f = ((size_t)P * P * 3 + 3 * (size_t)P) * sizeof(double);
   if (smem_b > 48 * 1024) {
     cudaFuncSetAttribute(k_vb_b<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
     cudaFuncSetAttribute(k_vb_b<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
     cudaFuncSetAttribute(k_vb_b<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
     cudaFuncSetAttribute(k_vb_b<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_b);
   }
-  if (smem_f > 48 * 1024)
-    cudaFuncSetAttribute(k_vb_fin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_f);
 #define SGDLM_VB_B(PM)                                                                \
   k_vb_b<T, PM><<<grid, kVbThreads, smem_b, s>>>(m, P, n, chunk, p, w, lambda, theta, mbar_full, \
                                                  scr.part_b)
@@ -764,20 +691,19 @@ void launch_vb(cudaStream_t s, int m, int P, long n, const unsigned *p, const do
   else
     SGDLM_VB_B(64);
 #undef SGDLM_VB_B
-  k_vb_fin<<<m, 32, smem_f, s>>>(m, P, chunks, p, n_t, s_t, scr.part_b, mean_lambda,
+  k_vb_fin<<<m, 32, 0, s>>>(m, P, chunks, p, n_t, s_t, scr.part_b, mean_lambda,
                                  mean_log_lambda, mbar_full, mean_m, mean_C, mean_n,
-                                 mean_s, mean_Q, series_flags);
+                                 mean_s, series_flags);
 }
 
 template void launch_vb<float>(cudaStream_t, int, int, long, const unsigned *,
                                const double *, const double *, const double *,
                                const float *, const float *, VbScratch, double *, double *,
-                               double *, double *, double *, double *, double *, int *,
-                               const double *);
+                               double *, double *, double *, double *, int *, const double *);
 template void launch_vb<double>(cudaStream_t, int, int, long, const unsigned *,
                                 const double *, const double *, const double *,
                                 const double *, const double *, VbScratch, double *,
-                                double *, double *, double *, double *, double *, double *,
-                                int *, const double *);
+                                double *, double *, double *, double *, double *, int *,
+                                const double *);
 
 }  // namespace sgdlm
