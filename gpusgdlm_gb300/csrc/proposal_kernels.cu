@@ -12,40 +12,48 @@ namespace {
 
 constexpr uint32_t TAG_REPLAY = 7u;  // Philox tag of the training batches
 
-// One thread per series.
+// One warp per series: lane k takes coefficient k and parent k; what a series sums over
+// its parents is added in their order by lane 0 (with one thread per series the kernel
+// took 59 us at m = 200: a chain of divisions and dependent loads).
 __global__ void k_features(int m, int P, const unsigned *__restrict__ p,
                            const unsigned *__restrict__ sp, const double *__restrict__ m_t,
                            const double *__restrict__ C_t, const double *__restrict__ n_t,
                            const double *__restrict__ s_t, float *__restrict__ X) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (j >= m) return;
   const int F = proposal_features(P), pj = (int)p[j];
   float *x = X + (size_t)j * F;
-  for (int k = 0; k < P; ++k) {
+  for (int k = lane; k < P; k += 32) {
     const double c = C_t[(size_t)j * P * P + (size_t)k * (P + 1)];
     const bool on = k < pj && c > 0.0;
     x[k] = on ? (float)(m_t[(size_t)j * P + k] / sqrt(c)) : 0.f;
     x[P + k] = on ? (float)log(c) : 0.f;
   }
-  x[2 * P] = (float)log(n_t[j]);
-  x[2 * P + 1] = (float)log(s_t[j]);
-  x[2 * P + 2] = (float)pj / (float)P;
+  if (lane < 2) x[2 * P + lane] = (float)log(lane == 0 ? n_t[j] : s_t[j]);
+  if (lane == 2) x[2 * P + 2] = (float)pj / (float)P;
   // simultaneous parents q of j: sp holds row j + m * q (< m * m)
   const size_t mm = (size_t)m * m;
   double s1 = 0.0, s2 = 0.0;
   int cnt = 0;
-  for (int k = 0; k < P; ++k) {
-    const unsigned pos = sp[(size_t)j * P + k];
-    if ((size_t)pos >= mm) continue;
-    const int q = (int)(pos / (unsigned)m);
-    const int pq = (int)p[q];
+  for (int k0 = 0; k0 < P; k0 += 32) {
+    const unsigned pos = k0 + lane < P ? sp[(size_t)j * P + k0 + lane] : 0xFFFFFFFFu;
+    const bool parent = (size_t)pos < mm;
     double mu = 0.0;
-    for (int l = 0; l < pq; ++l) mu += m_t[(size_t)q * P + l];
-    mu = pq > 0 ? mu / pq : 0.0;
-    s1 += mu;
-    s2 += mu * mu;
-    ++cnt;
+    if (parent) {
+      const int q = (int)(pos / (unsigned)m);
+      const int pq = (int)p[q];
+      for (int l = 0; l < pq; ++l) mu += m_t[(size_t)q * P + l];
+      mu = pq > 0 ? mu / pq : 0.0;
+    }
+    unsigned left = __ballot_sync(0xffffffffu, parent);
+    cnt += __popc(left);
+    for (; left; left &= left - 1) {
+      const double v = __shfl_sync(0xffffffffu, mu, __ffs(left) - 1);
+      s1 += v;
+      s2 += v * v;
+    }
   }
+  if (lane != 0) return;
   const double mean = cnt ? s1 / cnt : 0.0;
   x[2 * P + 3] = (float)mean;
   x[2 * P + 4] = cnt ? (float)fmax(s2 / cnt - mean * mean, 0.0) : 0.f;
@@ -139,8 +147,8 @@ __global__ void k_replay_gather(int B, int F, int O, long count, uint32_t k0, ui
   }
 }
 
-// One thread per series: the proposal's parameters and the constant part of the
-// log density ratio,
+// One warp per series (lane k: coefficient k; one thread per series took 108 us at
+// m = 200): the proposal's parameters and the constant part of the log density ratio,
 //   c_j = [n/2 log(n s/2) - lgamma(n/2) - 1/2 log|C| + p/2 log s]
 //       - [n~/2 log(n~ s~/2) - lgamma(n~/2) - 1/2 log|C~| + p/2 log s~],
 // log|C| = 2 sum log U_kk, log|C~| = log|C| + 2 sum rho_k (k < p_j).
@@ -150,21 +158,21 @@ __global__ void k_params(int m, int P, const unsigned *__restrict__ p, const flo
                          const double *__restrict__ s_t, const double *__restrict__ U64,
                          double *__restrict__ mq, double *__restrict__ nq, double *__restrict__ sq,
                          double *__restrict__ Uq64, T *__restrict__ Uq, double *__restrict__ cst) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), k = threadIdx.x & 31;
   if (j >= m) return;
   const int O = proposal_outputs(P), pj = (int)p[j];
   const float *o = out + (size_t)j * O;
   const double *U = U64 + (size_t)j * P * P;
   double logdetC = 0.0, sum_rho = 0.0;
-  for (int k = 0; k < P; ++k) {
+  static_assert(kProposalMaxP <= 32, "a lane per coefficient");
+  double lg = 0.0, rh = 0.0;
+  bool on = false;
+  if (k < P) {
     const double ukk = U[k + (size_t)P * k];
-    const bool on = k < pj && ukk > 0.0;
+    on = k < pj && ukk > 0.0;
     const double dl = on ? (double)clampf(o[k], kDeltaMax) : 0.0;
-    const double rh = on ? (double)clampf(o[P + k], kRhoMax) : 0.0;
-    if (on) {
-      logdetC += 2.0 * log(ukk);
-      sum_rho += rh;
-    }
+    rh = on ? (double)clampf(o[P + k], kRhoMax) : 0.0;
+    if (on) lg = 2.0 * log(ukk);
     // sqrt(C_kk) = the norm of column k of U
     double ckk = 0.0;
     for (int l = 0; l <= k; ++l) ckk += U[l + (size_t)P * k] * U[l + (size_t)P * k];
@@ -176,6 +184,13 @@ __global__ void k_params(int m, int P, const unsigned *__restrict__ p, const flo
       Uq[(size_t)j * P * P + l + (size_t)P * k] = (T)v;
     }
   }
+  // the sums in the coefficients' order
+  for (unsigned left = __ballot_sync(0xffffffffu, on); left; left &= left - 1) {
+    const int q = __ffs(left) - 1;
+    logdetC += __shfl_sync(0xffffffffu, lg, q);
+    sum_rho += __shfl_sync(0xffffffffu, rh, q);
+  }
+  if (k != 0) return;
   const double n = n_t[j], s = s_t[j];
   const double a = (double)clampf(o[2 * P], kShapeMax), b = (double)clampf(o[2 * P + 1], kShapeMax);
   const double n2 = n * exp(a), s2 = s * exp(b);
@@ -251,8 +266,19 @@ __global__ void k_log_weights(int m, long n, const double *__restrict__ logdet,
                               const double *__restrict__ lr, double *__restrict__ logw) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
+  // added in the series' order, sixteen loads in flight (48 us at m = 200, 10 000 draws,
+  // with one)
   double v = logdet[i];
-  for (int j = 0; j < m; ++j) v += lr[(size_t)j * n + i];
+  constexpr int kAhead = 16;
+  int j = 0;
+  for (; j + kAhead <= m; j += kAhead) {
+    double t[kAhead];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) t[q] = lr[(size_t)(j + q) * n + i];
+#pragma unroll
+    for (int q = 0; q < kAhead; ++q) v += t[q];
+  }
+  for (; j < m; ++j) v += lr[(size_t)j * n + i];
   logw[i] = v;
 }
 
@@ -261,7 +287,7 @@ __global__ void k_log_weights(int m, long n, const double *__restrict__ logdet,
 void launch_proposal_features(cudaStream_t s, int m, int P, const unsigned *p, const unsigned *sp,
                               const double *m_t, const double *C_t, const double *n_t,
                               const double *s_t, float *X) {
-  k_features<<<(m + 127) / 128, 128, 0, s>>>(m, P, p, sp, m_t, C_t, n_t, s_t, X);
+  k_features<<<(m + 3) / 4, 128, 0, s>>>(m, P, p, sp, m_t, C_t, n_t, s_t, X);
 }
 
 void launch_proposal_targets(cudaStream_t s, int m, int P, const unsigned *p, const double *m_t,
@@ -295,7 +321,7 @@ void launch_proposal_params(cudaStream_t s, int m, int P, const unsigned *p, con
                             const double *m_t, const double *n_t, const double *s_t,
                             const double *U64, double *mq, double *nq, double *sq, double *Uq64,
                             T *Uq, double *cst) {
-  k_params<T><<<(m + 127) / 128, 128, 0, s>>>(m, P, p, out, m_t, n_t, s_t, U64, mq, nq, sq, Uq64,
+  k_params<T><<<(m + 3) / 4, 128, 0, s>>>(m, P, p, out, m_t, n_t, s_t, U64, mq, nq, sq, Uq64,
                                               Uq, cst);
 }
 
@@ -309,10 +335,13 @@ void launch_log_ratio(cudaStream_t s, int m, int P, long n, const unsigned *p, c
   if (P <= 8)
     k_log_ratio<T, 8><<<grid, 128, 0, s>>>(m, P, n, p, theta, lambda, m_t, n_t, s_t, U, mq, nq, sq,
                                            Uq, cst, lr);
+  else if (P <= 16)
+    k_log_ratio<T, 16><<<grid, 128, 0, s>>>(m, P, n, p, theta, lambda, m_t, n_t, s_t, U, mq, nq, sq,
+                                            Uq, cst, lr);
   else  // P <= kProposalMaxP (checked by the engine)
     k_log_ratio<T, kProposalMaxP><<<grid, 128, 0, s>>>(m, P, n, p, theta, lambda, m_t, n_t, s_t, U,
                                                        mq, nq, sq, Uq, cst, lr);
-  k_log_weights<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(m, n, logdet, lr, logw);
+  k_log_weights<<<(unsigned)((n + 63) / 64), 64, 0, s>>>(m, n, logdet, lr, logw);
 }
 
 template void launch_proposal_params<float>(cudaStream_t, int, int, const unsigned *, const float *,
