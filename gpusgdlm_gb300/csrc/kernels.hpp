@@ -103,6 +103,8 @@ struct LuPlan {
   int vals_smem;       // the sparse levels' value slots live in shared memory
   int prog_smem;       // the solve phase stages the level programs in shared memory
   int tc;              // trailing updates on the tensor cores (tcgen05)
+  int small_grid;      // > 0: log|det| by k_lu_small on so many blocks ...
+  size_t small_smem;   // ... with this much shared memory each
   size_t scratch_elems_per_cta;  // dense core + per-draw values of the sparse levels
   size_t fb_elems_per_cta;       // the redo's: the above, or a full m_p x m_p slab
   int fb_core_smem;              // the redo factors the dense core in shared memory

@@ -1128,6 +1128,9 @@ __device__ __forceinline__ void gj_load_block(const T *buf, T (&P)[4][4]) {
 __device__ __forceinline__ float log_abs_t(float v) { return logf(fabsf(v)); }
 __device__ __forceinline__ double log_abs_t(double v) { return log(fabs(v)); }
 
+// Super-steps of a last panel at k0 whose inverse is not wanted: its pivot blocks that
+// hold rows of the core (the rest is padding), less the last one's update.
+__device__ __forceinline__ int last_super_steps(int core_n, int k0) { return (core_n - k0 + 3) / 4 - 1; }
 // P^-1 into its slot (row-major after the pivot rows) for the rows of C.
 template <typename T>
 __device__ __forceinline__ void gj_put_inverse(const T (&P)[4][4], T *buf) {
@@ -1139,15 +1142,19 @@ __device__ __forceinline__ void gj_put_inverse(const T (&P)[4][4], T *buf) {
   }
 }
 
-// Warp 0, lane = row of D.  Software-pipelined: super-step K updates positions
+// One warp, lane = row of D.  Short: only short_steps updates (last_super_steps, a last
+// panel whose inverse nobody reads: the rows beyond the core's are rows of the
+// identity, whose pivot blocks contribute nothing to log|det D|).
+// Software-pipelined: super-step K updates positions
 // 4..7 first (they are the next pivot block P_{K+1}), the four next pivot rows
 // put that block into slot K + 1 and every lane reads it back and inverts it,
 // then positions 8..31 are updated and the rest of the pivot rows (and, with
 // Publish, P_{K+1}^-1) complete the slot.  With Publish (rows of C trailing on
 // the named barriers) the slot is then published.  log|det P| accumulates in T
 // on every lane; lane 0 returns the sum.
-template <typename T, bool Publish>
-__device__ __forceinline__ double gj_diag(T (&a)[kB], T *slots, T tau, bool &bad) {
+template <typename T, bool Publish, bool Short = false>
+__device__ __forceinline__ double gj_diag(T (&a)[kB], T *slots, T tau, bool &bad,
+                                          int short_steps = kB / 4) {
   using V = Vec<T>;
   const int lane = threadIdx.x & 31;
   T ld = T(0);
@@ -1170,7 +1177,7 @@ __device__ __forceinline__ double gj_diag(T (&a)[kB], T *slots, T tau, bool &bad
     ld += log_abs_t(det);
   }
 #pragma unroll 1
-  for (int K = 0; K < kB / 4; ++K) {
+  for (int K = 0; K < (Short ? short_steps : kB / 4); ++K) {
     const int c0 = 4 * K;
     const T *buf = slots + K * kGjSlot;
     const bool inK = lane >= c0 && lane < c0 + 4;
@@ -1483,7 +1490,7 @@ __device__ __forceinline__ void level_forward(const EliminationPlan &ep, int lev
 
 // The value slots of draw i before the levels: the constants, the unit diagonal
 // and the level-0 entries -theta (each thread's sixteen gathers in flight at once).
-template <typename T>
+template <typename T, int NT = kThreads>
 __device__ __forceinline__ void build_slots(const EliminationPlan &ep, int m, long i,
                                             const Theta<T> &theta, T *vals) {
   const int tid = threadIdx.x;
@@ -1492,17 +1499,17 @@ __device__ __forceinline__ void build_slots(const EliminationPlan &ep, int m, lo
     vals[kSlotOne] = T(1);
   }
   for (int r = tid; r < m; r += blockDim.x) vals[ep.diag_slot[r]] = T(1);
-  for (int k0 = tid; k0 < ep.nnz0; k0 += 16 * kThreads) {
+  for (int k0 = tid; k0 < ep.nnz0; k0 += 16 * NT) {
     int e[16], sl[16];
 #pragma unroll
     for (int h = 0; h < 16; ++h) {
-      const bool ok = k0 + h * kThreads < ep.nnz0;
-      e[h] = ok ? (theta.g ? 0 : ep.l0_e[k0 + h * kThreads]) : -1;  // the index only without the Gamma copy
-      sl[h] = ok ? ep.l0_slot[k0 + h * kThreads] : 0;
+      const bool ok = k0 + h * NT < ep.nnz0;
+      e[h] = ok ? (theta.g ? 0 : ep.l0_e[k0 + h * NT]) : -1;  // the index only without the Gamma copy
+      sl[h] = ok ? ep.l0_slot[k0 + h * NT] : 0;
     }
     T th[16];
 #pragma unroll
-    for (int h = 0; h < 16; ++h) th[h] = e[h] >= 0 ? theta.gamma(i, k0 + h * kThreads, e[h]) : T(0);
+    for (int h = 0; h < 16; ++h) th[h] = e[h] >= 0 ? theta.gamma(i, k0 + h * NT, e[h]) : T(0);
 #pragma unroll
     for (int h = 0; h < 16; ++h)
       if (e[h] >= 0) vals[sl[h]] = -th[h];
@@ -1518,7 +1525,7 @@ __device__ __forceinline__ void build_slots(const EliminationPlan &ep, int m, lo
 // loads do not wait on a dependent load; kLevFlight chunks are in flight at a
 // time (the plan's words come from L2: the rounds are latency-bound).  With zf,
 // the right-hand side's forward program of each level rides along.
-template <typename T>
+template <typename T, int NW = kWarps>
 __device__ __forceinline__ void run_levels(const EliminationPlan &ep, T *vals, T tau, bool &bad,
                                            double &ld_part, T *zf) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1537,11 +1544,11 @@ __device__ __forceinline__ void run_levels(const EliminationPlan &ep, T *vals, T
     __syncthreads();
     // new entries
     const int c_begin = ep.lev_chunk[lev], c_end = ep.lev_chunk[lev + 1];
-    const int n_w = (c_begin + warp < c_end) ? (c_end - c_begin - warp + kWarps - 1) / kWarps : 0;
+    const int n_w = (c_begin + warp < c_end) ? (c_end - c_begin - warp + NW - 1) / NW : 0;
     for (int base = 0; base < n_w; base += 32) {
       int my_t0 = 0, my_t1 = 0;
       if (base + lane < n_w) {
-        const int ci = c_begin + warp + (base + lane) * kWarps;
+        const int ci = c_begin + warp + (base + lane) * NW;
         my_t0 = ep.chunk_tofs[ci];
         my_t1 = ep.chunk_tofs[ci + 1];
       }
@@ -1555,7 +1562,7 @@ __device__ __forceinline__ void run_levels(const EliminationPlan &ep, T *vals, T
           const int t0 = __shfl_sync(kFull, my_t0, ii & 31);
           const int t1 = __shfl_sync(kFull, my_t1, ii & 31);
           const bool ok = ii < n_here;
-          const int ch = c_begin + warp + (base + ii) * kWarps;
+          const int ch = c_begin + warp + (base + ii) * NW;
           e[h] = ok ? __ldg(ep.ent + (size_t)ch * 32 + lane) : kSlotNone;  // none: no store, base 0
           K[h] = ok ? (t1 - t0) >> 5 : 0;
           toff[h] = t0 + lane;
@@ -2213,6 +2220,231 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
   }
 }
 
+// log|det| of FP32 draws whose dense core has at most 96 nodes (d_p = 32, 64, 96): the
+// arithmetic of k_lu<float, true>, operation by operation, in blocks of 128 threads,
+// four to an SM.
+//
+// k_lu is bound by its dependent chains (levels' barriers and L2 latencies, the pivot
+// blocks of a panel), of which two blocks of 256 threads run per SM (registers, tensor
+// memory).  At these sizes a draw needs half of that: thread t owns row t of the core,
+// which is tensor-memory lane t in every panel, so rows never move and no slab in
+// global memory is needed.  Panel kb: warp kb inverts its own rows' diagonal block (the
+// chain moves from one SM sub-partition to the next), the warps below split their rows
+// of C and one column of B each; L = C D^-1 and -L B on the tensor cores; then each
+// thread has its row's next 32 columns in registers, the rest stays in tensor memory
+// (columns 0..63: column c - 32 of the core; 64..127: -L B, before it L in 96..127).
+// 10 000 draws: m = 100 (core 33) 725 -> 326 us, m = 200 (87) 1161 -> 593 us; 4 999 at
+// m = 133 (45) 383 -> 191 us.
+constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32, kSmallMaxDp = 96;
+constexpr int kSmallTmem = 128, kSmallTmemU = 64, kSmallTmemL = 96;
+constexpr int kBs = kB + 1;  // stride of the staged columns of B
+struct SmallSmem {
+  size_t off_B, off_D, off_prow, off_Lt, off_Ut, off_vals, off_red, total;
+  static constexpr size_t part_L = (kSmallMaxDp) * 64, part_U = (kSmallMaxDp - kB) * 64;
+  __host__ __device__ explicit SmallSmem(int nv) {
+    size_t o = 0;
+    auto take = [&](size_t bytes) {
+      const size_t at = o;
+      o += (bytes + 15) & ~(size_t)15;
+      return at;
+    };
+    // B's columns, then (they are split by then) D^-1 split as a B operand
+    off_B = take((size_t)(kSmallMaxDp - kB) * kBs * sizeof(float));
+    off_D = take((size_t)kB * kDs * sizeof(float));
+    off_prow = take((size_t)(kB / 4) * kGjSlot * sizeof(float));
+    // the level value slots, then the split rows of C / L (rows 32.. of the core) and
+    // columns of B
+    const size_t panels = 3 * (part_L + part_U), vals = (size_t)nv * sizeof(float);
+    o = (o + 127) & ~(size_t)127;
+    off_vals = off_Lt = take(panels > vals ? panels : vals);
+    off_Ut = off_Lt + 3 * part_L;
+    off_red = take(64 * sizeof(double));
+    total = o;
+  }
+};
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+      "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+      "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])),
+      "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+      "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
+      "r"(__float_as_uint(v[15])));
+}
+
+__global__ void __launch_bounds__(kSmallThreads, 4)
+    k_lu_small(int m, int P, int dp, long n, EliminationPlan ep, const float *__restrict__ theta_g,
+               double *__restrict__ logdet, int *__restrict__ draw_flags,
+               int *__restrict__ pivot_list) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const SmallSmem S(ep.nv);
+  float *Bs = reinterpret_cast<float *>(smem_raw + S.off_B);
+  unsigned char *Dt = smem_raw + S.off_B;
+  float *D = reinterpret_cast<float *>(smem_raw + S.off_D);
+  float *prow = reinterpret_cast<float *>(smem_raw + S.off_prow);
+  float *vals = reinterpret_cast<float *>(smem_raw + S.off_vals);
+  // the A operand's tile of 128 rows begins 32 rows before the first one that exists
+  // (lanes 0..31 get products of whatever lies there; nobody reads them)
+  unsigned char *Lt = smem_raw + S.off_Lt - kB * 64, *Ut = smem_raw + S.off_Ut;
+  double *red = reinterpret_cast<double *>(smem_raw + S.off_red);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = tid;
+  const int nbk = dp / kB;
+  const float tau = (float)kPivotThreshold;
+  const Theta<float> theta{nullptr, theta_g, m, P, ep.nnz0, n};
+  __shared__ int sflag;
+  __shared__ uint32_t s_tmem;
+  __shared__ __align__(8) MmaSync s_mbar;
+  uint32_t mphase = 0;
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 128;" ::"r"(
+        smem_u32(&s_tmem)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  if (tid == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&s_mbar.bar)));
+    s_mbar.dead = 0;
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = s_tmem, trow = tmem + ((uint32_t)(warp * 32) << 16);
+  auto issue = [&](uint32_t d, const unsigned char *b, size_t part_b, uint32_t idesc) {
+    if (tid == 0 && mma_live(&s_mbar)) {
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      umma_split_tile(d, smem_u32(Lt), SmallSmem::part_L, smem_u32(b), part_b, idesc, false);
+      asm volatile(
+          "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+              smem_u32(&s_mbar.bar)));
+    }
+  };
+  // shared memory written, tensor memory read: before the next MMAs and reads
+  auto operands_ready = [&]() {
+    asm volatile("fence.proxy.async.shared::cta;");
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+  };
+  for (long i = blockIdx.x; i < n; i += gridDim.x) {
+    if (tid == 0) sflag = 0;
+    bool bad = false;
+    double ld_part = 0.0;
+    build_slots<float, kSmallThreads>(ep, m, i, theta, vals);
+    __syncthreads();
+    run_levels<float, kSmallWarps>(ep, vals, tau, bad, ld_part, nullptr);
+    // ---- the core's rows: 32 columns in registers, the rest in tensor memory (or, of
+    // the first panel's rows, staged as B)
+    float a[kB];
+    if (warp < nbk) {
+#pragma unroll
+      for (int q = 0; q < kB; ++q) a[q] = vals[ep.core_map[row + dp * q]];
+      for (int c0 = kB; c0 < dp; c0 += 16) {
+        float e[16];
+#pragma unroll
+        for (int q = 0; q < 16; ++q) e[q] = vals[ep.core_map[row + dp * (c0 + q)]];
+        if (warp == 0) {
+#pragma unroll
+          for (int q = 0; q < 16; ++q) Bs[(c0 - kB + q) * kBs + lane] = e[q];
+        } else {
+          tmem_st16(trow + (uint32_t)(c0 - kB), e);
+        }
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;");
+    }
+    __syncthreads();  // the slots are dead
+    for (int kb = 0; kb < nbk; ++kb) {
+      const int k0 = kb * kB, r0 = k0 + kB, R = dp - r0;
+      const bool below = warp > kb && warp < nbk;
+      if (warp == kb) {
+        ld_part += gj_diag<float, false, true>(a, prow, tau, bad,
+                                               R > 0 ? kB / 4 : last_super_steps(ep.core_n, k0));
+#pragma unroll
+        for (int q = 0; q < kB; q += 4) Vec<float>::st(D + lane * kDs + q, a + q);
+      } else if (below) {
+        write_split_row(Lt, SmallSmem::part_L, row, a);
+        float b[kB];
+        const int col = (warp - kb - 1) * 32 + lane;  // of B, from r0 on
+#pragma unroll
+        for (int q = 0; q < kB; ++q) b[q] = Bs[(r0 - kB + col) * kBs + q];
+        write_split_row(Ut, SmallSmem::part_U, col, b);
+      }
+      if (R == 0) break;
+      __syncthreads();
+      {  // Dt row `lane` = column `lane` of D^-1, values 8 warp .. 8 warp + 7
+        float col[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) col[e] = D[(8 * warp + e) * kDs + lane];
+        write_split_chunk(Dt, (size_t)kB * 64, lane, warp, col);
+      }
+      operands_ready();
+      issue(tmem + kSmallTmemL, Dt, (size_t)kB * 64, umma_idesc(kB, false));
+      mma_wait(&s_mbar, mphase, bad);
+      if (below) {
+        float l[kB];
+#pragma unroll
+        for (int h = 0; h < kB; h += 16) {
+          uint32_t v[16];
+          tmem_ld16(trow + (uint32_t)(kSmallTmemL + h), v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+          for (int q = 0; q < 16; ++q) {
+            l[h + q] = __uint_as_float(v[q]);
+            bad |= !(fabsf(l[h + q]) <= tau);
+          }
+        }
+        write_split_row(Lt, SmallSmem::part_L, row, l);
+      }
+      operands_ready();
+      issue(tmem + kSmallTmemU, Ut, SmallSmem::part_U, umma_idesc(R));
+      mma_wait(&s_mbar, mphase, bad);
+      if (below) {
+#pragma unroll
+        for (int h = 0; h < kB; h += 16) {  // the next panel's columns
+          uint32_t e[16], u[16];
+          tmem_ld16(trow + (uint32_t)(r0 - kB + h), e);
+          tmem_ld16(trow + (uint32_t)(kSmallTmemU + h), u);
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+          for (int q = 0; q < 16; ++q) a[h + q] = __fadd_rn(__uint_as_float(e[q]), __uint_as_float(u[q]));
+        }
+        for (int c = kB; c < R; c += 16) {
+          uint32_t e[16], u[16];
+          tmem_ld16(trow + (uint32_t)(r0 - kB + c), e);
+          tmem_ld16(trow + (uint32_t)(kSmallTmemU + c), u);
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
+          float s[16];
+#pragma unroll
+          for (int q = 0; q < 16; ++q) s[q] = __fadd_rn(__uint_as_float(e[q]), __uint_as_float(u[q]));
+          if (warp == kb + 1) {
+#pragma unroll
+            for (int q = 0; q < 16; ++q) Bs[(r0 - kB + c + q) * kBs + lane] = s[q];
+          } else {
+            tmem_st16(trow + (uint32_t)(r0 - kB + c), s);
+          }
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;");
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;");
+      __syncthreads();
+      asm volatile("tcgen05.fence::after_thread_sync;");
+    }
+    if (bad) atomicOr(&sflag, 1);
+    const double ld_total = block_sum_det(ld_part, red);  // contains __syncthreads
+    if (tid == 0) {
+      logdet[i] = ld_total;
+      if (sflag != 0) {
+        atomicOr(&draw_flags[i], DRAW_FLAG_PIVOT);
+        const int q = atomicAdd(pivot_list, 1);
+        if (q < n) pivot_list[1 + q] = (int)i;
+      }
+    }
+    __syncthreads();
+  }
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem));
+}
+
 // Pivoting redo of the draws the fast pass flagged.  The sparse levels' pivots
 // are diagonal entries of (I - Gamma) as updated by earlier levels, eliminated
 // without pivoting as in the fast pass (their multipliers only feed the
@@ -2732,6 +2964,15 @@ LuPlan plan_lu(int m, int P, long n, int num_sms, int core_n, int nv, int n_solv
   }
   int ctas_per_sm = pl.smem <= smem_budget(2) ? 2 : 1;
   if (sizeof(T) == 8) ctas_per_sm = 1;
+  // small cores of FP32 draws: k_lu_small while at least three of its blocks fit an SM
+  pl.small_grid = 0;
+  if (pl.tc && nv > 0 && pl.dp <= kSmallMaxDp) {
+    pl.small_smem = SmallSmem(nv).total;
+    for (int c = 4; c >= 3 && pl.small_grid == 0; --c)
+      if (pl.small_smem + 128 <= smem_budget(c)) pl.small_grid = num_sms * c;
+    if (opt.max_grid > 0) pl.small_grid = std::min(pl.small_grid, opt.max_grid);
+    pl.small_grid = (int)std::min<long>(pl.small_grid, n);
+  }
   long grid = (long)num_sms * ctas_per_sm;
   if (opt.max_grid > 0 && grid > opt.max_grid) grid = opt.max_grid;
   if (grid > n) grid = n;
@@ -2769,6 +3010,12 @@ void launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &
                                               nu_in, pivot_list, draw_list);
   };
   if constexpr (sizeof(T) == 4) {
+    if (pl.small_grid > 0 && !x && !draw_list && theta_g && pivot_list) {
+      cudaFuncSetAttribute(k_lu_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.small_smem);
+      k_lu_small<<<pl.small_grid, kSmallThreads, pl.small_smem, s>>>(pl.m, pl.P, pl.dp, n, ep, theta_g,
+                                                                     logdet, draw_flags, pivot_list);
+      return;
+    }
     if (pl.tc) {
       run(k_lu<T, true>);
       return;

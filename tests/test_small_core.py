@@ -1,0 +1,79 @@
+"""log|det| of FP32 draws with a dense core of at most 96 nodes: the kernel that takes
+four blocks per SM against the one it replaces there, which forecasts still take when
+the iterative solve is switched off (the same operations, so the same factors: the
+forecasts' log|det| of the same draws agree to the rounding of the FP64 sum of the
+pivots' logarithms), at cores of one node, below, at and above each panel, and around
+the largest; and draws that need pivoting.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from gpusgdlm_gb300 import SGDLM
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(m, kmax, seed, spread):
+    import bench
+
+    wl = bench.make_workload(m=m, kmax=kmax, T=2, seed=seed)
+    P = wl["P"]
+    s = SGDLM(1, strict=True)
+    s.setSimultaneousParents(wl["p"], np.where(wl["sp"] >= m * m, np.nan, wl["sp"]).astype(float))
+    s.setDiscountFactors(np.full(m, 0.97), np.full((P, P, m), 0.98))
+    rng = np.random.default_rng(seed)
+    par = (rng.uniform(-spread, spread, size=(P, m)),
+           np.repeat((1e-6 * np.eye(P))[:, :, None], m, axis=2), np.full(m, 50.0), np.full(m, 1.0))
+    return s, wl, par
+
+
+def _both(s, wl, par, n, seed):
+    s.setPosteriorParameters(*par)
+    s.setRngState(seed, 0)
+    s.computeVBPosterior(n, n)
+    flags = s.getStats()["draws_pivoted"]
+    d = s.getDraws()
+    s.setPriorParameters(*par)
+    s.setForecastSolver(False)
+    s.setRngState(seed, 0)
+    s.computeForecast(n, n, np.zeros((wl["P"], wl["m"])))
+    f = s.getDraws()
+    np.testing.assert_array_equal(d["thetas"], f["thetas"])
+    return d, f, flags
+
+
+@pytest.mark.parametrize("m,kmax,n", [
+    (33, 1, 3), (40, 9, 700), (60, 17, 300), (90, 12, 1300), (120, 9, 200), (150, 12, 333),
+    (170, 12, 200), (180, 13, 150), (200, 13, 100), (210, 13, 100)])
+def test_matches_the_large_kernel(built_lib, m, kmax, n):
+    s, wl, par = _engine(m, kmax, 3 + m, min(0.3, 0.8 / kmax))
+    d, f, flags = _both(s, wl, par, n, 5)
+    assert flags == 0
+    np.testing.assert_allclose(d["log_dets"], f["log_dets"], rtol=0, atol=1e-12)
+    ld = oracle.logdet(wl["sp"], np.asfortranarray(d["thetas"][:, :, :16].transpose(0, 2, 1)))
+    np.testing.assert_allclose(d["log_dets"][:16], ld, rtol=0, atol=1e-4)
+    s.close()
+
+
+def test_cores_cover_the_panels(built_lib):
+    """The sizes above reach every panel count of the kernel and the first one beyond."""
+    cores = set()
+    for m, kmax in ((33, 1), (90, 12), (120, 9), (150, 12), (180, 13), (210, 13)):
+        s, _, _ = _engine(m, kmax, 3 + m, 0.1)
+        cores.add((s.getEliminationInfo()["core_n"] + 31) // 32)
+        s.close()
+    assert {1, 2, 3, 4} <= cores
+
+
+def test_draws_that_need_pivoting(built_lib):
+    s, wl, par = _engine(100, 10, 8, 3.0)
+    s.setPosteriorParameters(*par)
+    s.computeVBPosterior(64, 64)
+    assert s.getStats()["draws_pivoted"] > 0
+    d = s.getDraws()
+    ld = oracle.logdet(wl["sp"], np.asfortranarray(d["thetas"].transpose(0, 2, 1)))
+    # partial pivoting in FP32: growth and condition of these draws (spectral radius far
+    # above one) leave about four digits
+    np.testing.assert_allclose(d["log_dets"], ld, rtol=0, atol=5e-2)
+    s.close()
