@@ -227,6 +227,54 @@ EliminationPlanHost plan_elimination(int m, int P, const std::vector<unsigned> &
   return pl;
 }
 
+LevelStreamHost level_stream(const EliminationPlanHost &pl, int lanes) {
+  LevelStreamHost st;
+  auto add_rows = [&](size_t n) {
+    st.rows.resize(st.rows.size() + n * (size_t)lanes * 2, 0u);
+    return st.rows.size() - n * (size_t)lanes * 2;
+  };
+  for (int l = 0; l < pl.nlev; ++l) {
+    const int p0 = pl.lev_piv[l], np = pl.lev_piv[l + 1] - p0;
+    const int s0 = pl.lev_scale[l], ns = pl.lev_scale[l + 1] - s0;
+    const int first = (std::max(np, ns) + lanes - 1) / lanes;
+    const size_t at = add_rows(first);
+    for (int q = 0; q < np; ++q) st.rows[at + 2 * (size_t)q] = (unsigned)pl.piv[p0 + q];
+    for (int q = 0; q < ns; ++q) st.rows[at + 2 * (size_t)q + 1] = pl.scale[s0 + q];
+    st.n_first.push_back(first);
+    // the level's entries, by decreasing term count: entry e on thread e % lanes, pass
+    // after pass over those that have a k-th term
+    std::vector<unsigned> ent;
+    std::vector<std::vector<unsigned>> terms;
+    for (int ch = pl.lev_chunk[l]; ch < pl.lev_chunk[l + 1]; ++ch)
+      for (int lane = 0; lane < 32; ++lane) {
+        const unsigned e = pl.ent[(size_t)ch * 32 + lane];
+        if ((e & 0xFFFFu) == kSlotNone) continue;
+        std::vector<unsigned> t;
+        for (int k = pl.chunk_tofs[ch]; k < pl.chunk_tofs[ch + 1]; k += 32)
+          if (pl.terms[k + lane] != pack16(kSlotZero, kSlotZero)) t.push_back(pl.terms[k + lane]);
+        ent.push_back(e);
+        terms.push_back(std::move(t));
+      }
+    int second = 0;
+    for (size_t k = 0;; ++k) {
+      size_t n = 0;
+      while (n < ent.size() && terms[n].size() > k) ++n;  // (decreasing term counts)
+      if (n == 0) break;
+      const int rows = (int)((n + lanes - 1) / lanes);
+      const size_t a = add_rows(rows);
+      for (size_t e = 0; e < n; ++e) {
+        const unsigned out = ent[e] & 0xFFFFu;
+        st.rows[a + 2 * e] = k == 0 ? ent[e] : pack16(out, out);
+        st.rows[a + 2 * e + 1] = terms[e][k];
+      }
+      second += rows;
+    }
+    st.n_second.push_back(second);
+  }
+  add_rows(kStreamAhead);
+  return st;
+}
+
 namespace {
 // A level takes the independent nodes whose Markowitz cost is at most kCostFactor
 // times the smallest one plus kCostSlack (more per level: fewer levels and barriers,

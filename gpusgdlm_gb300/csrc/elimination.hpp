@@ -39,6 +39,7 @@ namespace sgdlm {
 constexpr unsigned kSlotZero = 0, kSlotOne = 1, kSlotDiag0 = 2;
 constexpr unsigned kSlotNone = 0xFFFFu;  // padding lane of a chunk: no store
 constexpr int kMaxSlots = 0xFFFF;        // slots 0 .. 0xFFFE
+constexpr int kMaxLevels = 16;           // levels a caller may ask for
 
 inline unsigned pack16(unsigned lo, unsigned hi) { return (lo & 0xFFFFu) | (hi << 16); }
 
@@ -80,6 +81,29 @@ struct EliminationPlanHost {
   size_t n_terms = 0;                // unpadded term count (for reporting)
 };
 
+// The levels' program as rows of one 8-byte word per thread of a block of `lanes`
+// threads, in the order in which they are worked off, so that a thread reads its words
+// one after the other, ahead of the barriers between phases:
+//   first phase of a level: x = slot of a pivot (0: none), y = a multiplier (slot
+//     M[r][t] | slot M[t][t] << 16; 0: none);
+//   second phase: x = out slot | base slot << 16 (out 0: none), y = slot L | slot U << 16:
+//     vals[out] = vals[base] - vals[L] vals[U].  An entry's further terms follow in the
+//     same thread's later rows, with the entry itself as base.
+// Row t of phase p of level l: rows[(sum of the counts before + t) * lanes + thread];
+// kStreamAhead empty rows at the end (they are read, never used).
+constexpr int kStreamAhead = 3;
+struct LevelStreamHost {
+  std::vector<unsigned> rows;  // x, y pairs
+  std::vector<int> n_first, n_second;
+};
+LevelStreamHost level_stream(const EliminationPlanHost &pl, int lanes);
+struct LevelStream {
+  const uint2 *rows;
+  // rows of each phase and pivots of each level (a level's pivots are the first words
+  // of its first phase's rows)
+  unsigned short n_first[kMaxLevels], n_second[kMaxLevels], n_piv[kMaxLevels];
+};
+
 // Device copy of the plan (pointers into one allocation owned by the engine).
 // core_map == nullptr means "no plan": the whole matrix is the dense core.
 struct EliminationPlan {
@@ -100,6 +124,10 @@ struct EliminationPlan {
   // run of prog_len ints starting at prog, so that a kernel can stage them
   const int *prog;
   int prog_len;
+  // for blocks of 128 threads (k_lu_small): the levels, and the slots of the core's
+  // cells (row, 4 q) .. (row, 4 q + 3), 16 bits each, at small_map[128 q + row]
+  LevelStream small_stream;
+  const uint2 *small_map;
 };
 
 // Builds the plan from the parental sets (sp: max_p x m, entries < m*m address

@@ -413,6 +413,16 @@ int upload_elimination(sgdlm_engine *h) {
   put(pl.bwd.data(), pl.bwd.size());
   put(pl.core_node.data(), pl.core_node.size());
   put(pl.core_map.data(), (pl.core_map.size() + 1) / 2);  // two 16-bit slots per int
+  const LevelStreamHost small = level_stream(pl, 128);
+  put(small.rows.data(), small.rows.size());
+  std::vector<uint16_t> cells;
+  if (pl.nlev > 0 && pl.dp <= 128) {
+    cells.assign((size_t)128 * pl.dp, (uint16_t)kSlotZero);
+    for (int c = 0; c < pl.dp; ++c)
+      for (int r = 0; r < pl.dp; ++r)
+        cells[((size_t)(c / 4) * 128 + r) * 4 + c % 4] = pl.core_map[(size_t)r + (size_t)pl.dp * c];
+  }
+  put(cells.data(), cells.size() / 2);
   while (buf.size() % 4) buf.push_back(0);
   CK(h->elim_buf.alloc(buf.size()));
   CK(cudaMemcpy(h->elim_buf.ptr, buf.data(), buf.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -453,6 +463,14 @@ int upload_elimination(sgdlm_engine *h) {
   d.core_node = b + offs[k++];
   // without levels the whole matrix is the dense core, built from the parental sets
   d.core_map = pl.nlev > 0 ? reinterpret_cast<const uint16_t *>(b + offs[k]) : nullptr;
+  ++k;
+  d.small_stream.rows = reinterpret_cast<const uint2 *>(b + offs[k]);
+  for (int l = 0; l < pl.nlev; ++l) {
+    d.small_stream.n_first[l] = (unsigned short)small.n_first[l];
+    d.small_stream.n_second[l] = (unsigned short)small.n_second[l];
+    d.small_stream.n_piv[l] = (unsigned short)(pl.lev_piv[l + 1] - pl.lev_piv[l]);
+  }
+  d.small_map = reinterpret_cast<const uint2 *>(b + offs[++k]);
   return SGDLM_OK;
 }
 
@@ -1698,7 +1716,7 @@ int sgdlm_set_precision(sgdlm_handle h, int precision) {
 }
 int sgdlm_set_elimination_levels(sgdlm_handle h, int levels) {
   HCHECK(h);
-  if (levels < 0 || levels > 16) return h->fail(SGDLM_ERR_BAD_ARG, "levels must be in 0..16");
+  if (levels < 0 || levels > kMaxLevels) return h->fail(SGDLM_ERR_BAD_ARG, "levels must be in 0..16");
   h->elim_levels = levels;
   if (!h->mem_init) return SGDLM_OK;
   cudaStreamSynchronize(h->stream);

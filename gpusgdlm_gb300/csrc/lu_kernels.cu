@@ -1597,6 +1597,55 @@ __device__ __forceinline__ void run_levels(const EliminationPlan &ep, T *vals, T
   }
 }
 
+// The same levels from their stream (elimination.hpp, LevelStream) by a block of NT
+// threads: per row and warp one 8-byte load, three shared loads, one FMA and one store,
+// where the chunks cost about twice the instructions (shuffled offsets, two words, all
+// eight chunks of a round stepping through the longest one's terms).  The next
+// kStreamAhead rows' words are always on their way.  logs receives the pivots'
+// logarithms, level after level (their FP64 sum, on the narrow pipe, is left to one
+// warp); returns their number.
+template <int NT>
+__device__ __forceinline__ int run_stream(const LevelStream &st, int nlev, float *vals, float tau,
+                                          bool &bad, float *logs) {
+  const uint2 *next = st.rows + threadIdx.x;
+  uint2 q[kStreamAhead];
+#pragma unroll
+  for (int h = 0; h < kStreamAhead; ++h, next += NT) q[h] = __ldg(next);
+  auto take = [&]() {
+    const uint2 w = q[0];
+#pragma unroll
+    for (int h = 0; h + 1 < kStreamAhead; ++h) q[h] = q[h + 1];
+    q[kStreamAhead - 1] = __ldg(next);
+    next += NT;
+    return w;
+  };
+  int n_logs = 0;
+  for (int lev = 0; lev < nlev; ++lev) {
+    const int rows = st.n_first[lev];
+    for (int r = 0; r < rows; ++r) {
+      const uint2 w = take();
+      if (w.x) {
+        const float pv = vals[w.x];
+        if (!(finite_t(pv) && pv != 0.f)) bad = true;
+        logs[n_logs + r * NT + threadIdx.x] = logf(fabsf(pv));
+      }
+      if (w.y) {
+        const float l = vals[lo16(w.y)] / vals[hi16(w.y)];
+        if (!(dabs(l) <= tau)) bad = true;
+        vals[lo16(w.y)] = l;
+      }
+    }
+    n_logs += st.n_piv[lev];
+    __syncthreads();
+    for (int r = st.n_second[lev]; r > 0; --r) {
+      const uint2 w = take();
+      if (lo16(w.x)) vals[lo16(w.x)] = vals[hi16(w.x)] - vals[lo16(w.y)] * vals[hi16(w.y)];
+    }
+    __syncthreads();
+  }
+  return n_logs;
+}
+
 // The dense core (d_p x d_p, column-major) from the value slots through the
 // plan's slot map: four 16-bit slots per 8-byte word of the map, eight words in flight
 // per thread.
@@ -2233,15 +2282,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
 // of C and one column of B each; L = C D^-1 and -L B on the tensor cores; then each
 // thread has its row's next 32 columns in registers, the rest stays in tensor memory
 // (columns 0..63: column c - 32 of the core; 64..127: -L B, before it L in 96..127).
-// 10 000 draws: m = 100 (core 33) 725 -> 326 us, m = 200 (87) 1161 -> 593 us; 4 999 at
-// m = 133 (45) 383 -> 191 us.
+// 10 000 draws, us (k_lu; with the chunks' program of the levels; now): m = 100 (core 33)
+// 725, 325, 230; m = 133 (45) 765, 358, 258; m = 200 (87) 1161, 595, 489.
 constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32, kSmallMaxDp = 96;
 constexpr int kSmallTmem = 128, kSmallTmemU = 64, kSmallTmemL = 96;
 constexpr int kBs = kB + 1;  // stride of the staged columns of B
 struct SmallSmem {
-  size_t off_B, off_D, off_prow, off_Lt, off_Ut, off_vals, off_red, total;
+  size_t off_B, off_D, off_prow, off_Lt, off_Ut, off_vals, off_logs, total;
   static constexpr size_t part_L = (kSmallMaxDp) * 64, part_U = (kSmallMaxDp - kB) * 64;
-  __host__ __device__ explicit SmallSmem(int nv) {
+  __host__ __device__ SmallSmem(int nv, int m) {
     size_t o = 0;
     auto take = [&](size_t bytes) {
       const size_t at = o;
@@ -2258,7 +2307,8 @@ struct SmallSmem {
     o = (o + 127) & ~(size_t)127;
     off_vals = off_Lt = take(panels > vals ? panels : vals);
     off_Ut = off_Lt + 3 * part_L;
-    off_red = take(64 * sizeof(double));
+    // the logarithms of the pivots: one per eliminated node, one sum per panel
+    off_logs = take((size_t)(m + kSmallMaxDp / kB) * sizeof(float));
     total = o;
   }
 };
@@ -2280,7 +2330,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
                double *__restrict__ logdet, int *__restrict__ draw_flags,
                int *__restrict__ pivot_list) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const SmallSmem S(ep.nv);
+  const SmallSmem S(ep.nv, m);
   float *Bs = reinterpret_cast<float *>(smem_raw + S.off_B);
   unsigned char *Dt = smem_raw + S.off_B;
   float *D = reinterpret_cast<float *>(smem_raw + S.off_D);
@@ -2289,7 +2339,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
   // the A operand's tile of 128 rows begins 32 rows before the first one that exists
   // (lanes 0..31 get products of whatever lies there; nobody reads them)
   unsigned char *Lt = smem_raw + S.off_Lt - kB * 64, *Ut = smem_raw + S.off_Ut;
-  double *red = reinterpret_cast<double *>(smem_raw + S.off_red);
+  float *logs = reinterpret_cast<float *>(smem_raw + S.off_logs);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, row = tid;
   const int nbk = dp / kB;
   const float tau = (float)kPivotThreshold;
@@ -2330,20 +2380,28 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
   for (long i = blockIdx.x; i < n; i += gridDim.x) {
     if (tid == 0) sflag = 0;
     bool bad = false;
-    double ld_part = 0.0;
     build_slots<float, kSmallThreads>(ep, m, i, theta, vals);
     __syncthreads();
-    run_levels<float, kSmallWarps>(ep, vals, tau, bad, ld_part, nullptr);
+    const int n_logs = run_stream<kSmallThreads>(ep.small_stream, ep.nlev, vals, tau, bad, logs);
     // ---- the core's rows: 32 columns in registers, the rest in tensor memory (or, of
     // the first panel's rows, staged as B)
     float a[kB];
     if (warp < nbk) {
+      const uint2 *cells = ep.small_map + row;
 #pragma unroll
-      for (int q = 0; q < kB; ++q) a[q] = vals[ep.core_map[row + dp * q]];
+      for (int q = 0; q < kB; q += 4) {
+        const uint2 w = __ldg(cells + (q / 4) * kSmallThreads);
+        a[q] = vals[lo16(w.x)], a[q + 1] = vals[hi16(w.x)];
+        a[q + 2] = vals[lo16(w.y)], a[q + 3] = vals[hi16(w.y)];
+      }
       for (int c0 = kB; c0 < dp; c0 += 16) {
         float e[16];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) e[q] = vals[ep.core_map[row + dp * (c0 + q)]];
+        for (int q = 0; q < 16; q += 4) {
+          const uint2 w = __ldg(cells + ((c0 + q) / 4) * kSmallThreads);
+          e[q] = vals[lo16(w.x)], e[q + 1] = vals[hi16(w.x)];
+          e[q + 2] = vals[lo16(w.y)], e[q + 3] = vals[hi16(w.y)];
+        }
         if (warp == 0) {
 #pragma unroll
           for (int q = 0; q < 16; ++q) Bs[(c0 - kB + q) * kBs + lane] = e[q];
@@ -2358,8 +2416,9 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
       const int k0 = kb * kB, r0 = k0 + kB, R = dp - r0;
       const bool below = warp > kb && warp < nbk;
       if (warp == kb) {
-        ld_part += gj_diag<float, false, true>(a, prow, tau, bad,
-                                               R > 0 ? kB / 4 : last_super_steps(ep.core_n, k0));
+        const double ld = gj_diag<float, false, true>(a, prow, tau, bad,
+                                                      R > 0 ? kB / 4 : last_super_steps(ep.core_n, k0));
+        if (lane == 0) logs[n_logs + kb] = (float)ld;  // (an FP32 sum)
 #pragma unroll
         for (int q = 0; q < kB; q += 4) Vec<float>::st(D + lane * kDs + q, a + q);
       } else if (below) {
@@ -2431,16 +2490,20 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
       asm volatile("tcgen05.fence::after_thread_sync;");
     }
     if (bad) atomicOr(&sflag, 1);
-    const double ld_total = block_sum_det(ld_part, red);  // contains __syncthreads
-    if (tid == 0) {
-      logdet[i] = ld_total;
-      if (sflag != 0) {
-        atomicOr(&draw_flags[i], DRAW_FLAG_PIVOT);
-        const int q = atomicAdd(pivot_list, 1);
-        if (q < n) pivot_list[1 + q] = (int)i;
+    __syncthreads();
+    if (warp == 0) {  // (the other warps go on to the next draw)
+      double ld = 0.0;
+      for (int q = lane; q < n_logs + nbk; q += 32) ld += (double)logs[q];
+      ld = warp_sum_d(ld);
+      if (lane == 0) {
+        logdet[i] = ld;
+        if (sflag != 0) {
+          atomicOr(&draw_flags[i], DRAW_FLAG_PIVOT);
+          const int q = atomicAdd(pivot_list, 1);
+          if (q < n) pivot_list[1 + q] = (int)i;
+        }
       }
     }
-    __syncthreads();
   }
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 128;" ::"r"(tmem));
 }
@@ -2967,7 +3030,7 @@ LuPlan plan_lu(int m, int P, long n, int num_sms, int core_n, int nv, int n_solv
   // small cores of FP32 draws: k_lu_small while at least three of its blocks fit an SM
   pl.small_grid = 0;
   if (pl.tc && nv > 0 && pl.dp <= kSmallMaxDp) {
-    pl.small_smem = SmallSmem(nv).total;
+    pl.small_smem = SmallSmem(nv, m).total;
     for (int c = 4; c >= 3 && pl.small_grid == 0; --c)
       if (pl.small_smem + 128 <= smem_budget(c)) pl.small_grid = num_sms * c;
     if (opt.max_grid > 0) pl.small_grid = std::min(pl.small_grid, opt.max_grid);
