@@ -128,6 +128,7 @@ struct EliminationPlan {
   // cells (row, 4 q) .. (row, 4 q + 3), 16 bits each, at small_map[128 q + row]
   LevelStream small_stream;
   const uint2 *small_map;
+  LevelStream stream;  // the levels for blocks of 256 threads (k_lu, FP32 draws, log|det|)
 };
 
 // Builds the plan from the parental sets (sp: max_p x m, entries < m*m address

@@ -413,7 +413,7 @@ int upload_elimination(sgdlm_engine *h) {
   put(pl.bwd.data(), pl.bwd.size());
   put(pl.core_node.data(), pl.core_node.size());
   put(pl.core_map.data(), (pl.core_map.size() + 1) / 2);  // two 16-bit slots per int
-  const LevelStreamHost small = level_stream(pl, 128);
+  const LevelStreamHost small = level_stream(pl, 128), large = level_stream(pl, 256);
   put(small.rows.data(), small.rows.size());
   std::vector<uint16_t> cells;
   if (pl.nlev > 0 && pl.dp <= 128) {
@@ -423,6 +423,7 @@ int upload_elimination(sgdlm_engine *h) {
         cells[((size_t)(c / 4) * 128 + r) * 4 + c % 4] = pl.core_map[(size_t)r + (size_t)pl.dp * c];
   }
   put(cells.data(), cells.size() / 2);
+  put(large.rows.data(), large.rows.size());
   while (buf.size() % 4) buf.push_back(0);
   CK(h->elim_buf.alloc(buf.size()));
   CK(cudaMemcpy(h->elim_buf.ptr, buf.data(), buf.size() * sizeof(int), cudaMemcpyHostToDevice));
@@ -464,13 +465,17 @@ int upload_elimination(sgdlm_engine *h) {
   // without levels the whole matrix is the dense core, built from the parental sets
   d.core_map = pl.nlev > 0 ? reinterpret_cast<const uint16_t *>(b + offs[k]) : nullptr;
   ++k;
-  d.small_stream.rows = reinterpret_cast<const uint2 *>(b + offs[k]);
-  for (int l = 0; l < pl.nlev; ++l) {
-    d.small_stream.n_first[l] = (unsigned short)small.n_first[l];
-    d.small_stream.n_second[l] = (unsigned short)small.n_second[l];
-    d.small_stream.n_piv[l] = (unsigned short)(pl.lev_piv[l + 1] - pl.lev_piv[l]);
-  }
-  d.small_map = reinterpret_cast<const uint2 *>(b + offs[++k]);
+  auto set_stream = [&](LevelStream &st, const LevelStreamHost &sh, size_t at) {
+    st.rows = reinterpret_cast<const uint2 *>(b + offs[at]);
+    for (int l = 0; l < pl.nlev; ++l) {
+      st.n_first[l] = (unsigned short)sh.n_first[l];
+      st.n_second[l] = (unsigned short)sh.n_second[l];
+      st.n_piv[l] = (unsigned short)(pl.lev_piv[l + 1] - pl.lev_piv[l]);
+    }
+  };
+  set_stream(d.small_stream, small, k++);
+  d.small_map = reinterpret_cast<const uint2 *>(b + offs[k++]);
+  set_stream(d.stream, large, k);
   return SGDLM_OK;
 }
 

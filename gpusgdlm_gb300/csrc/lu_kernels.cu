@@ -1892,9 +1892,19 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
       }
     }
     __syncthreads();
-    // ---- sparse levels (the loop of run_levels, kept inline here: through the
-    // function this kernel measured 2 % slower)
-    for (int lev = 0; lev < ep.nlev; ++lev) {
+    // ---- sparse levels: log|det| alone from the stream; else the loop of run_levels
+    // (kept inline here: through the function this kernel measured 2 % slower)
+    int n_logs = 0;
+    bool streamed = false;
+    if constexpr (TC) {
+      if (planned && vals_smem && !solve) {
+        // the pivots' logarithms take nu's place (no right-hand side here)
+        n_logs = run_stream<kThreads>(ep.stream, ep.nlev, reinterpret_cast<float *>(vals), tau, bad,
+                                      reinterpret_cast<float *>(nu));
+        streamed = true;
+      }
+    }
+    for (int lev = streamed ? ep.nlev : 0; lev < ep.nlev; ++lev) {
       for (int q = ep.lev_piv[lev] + tid; q < ep.lev_piv[lev + 1]; q += blockDim.x) {
         const T pv = vals[ep.piv[q]];
         if (!(finite_t(pv) && pv != T(0))) bad = true;
@@ -2171,6 +2181,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
       __syncthreads();
     }
     if (bad) atomicOr(&sflag, 1);
+    for (int q = tid; q < n_logs; q += kThreads) ld_part += (double)reinterpret_cast<float *>(nu)[q];
     const double ld_total = block_sum_det(ld_part, red);  // contains __syncthreads
     const bool flagged = (sflag != 0);
     if (tid == 0) {
