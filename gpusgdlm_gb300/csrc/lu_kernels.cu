@@ -1152,6 +1152,7 @@ __device__ __forceinline__ void gj_put_inverse(const T (&P)[4][4], T *buf) {
 // Publish, P_{K+1}^-1) complete the slot.  With Publish (rows of C trailing on
 // the named barriers) the slot is then published.  log|det P| accumulates in T
 // on every lane; lane 0 returns the sum.
+// Without Publish two slots are used in turn.
 template <typename T, bool Publish, bool Short = false>
 __device__ __forceinline__ double gj_diag(T (&a)[kB], T *slots, T tau, bool &bad,
                                           int short_steps = kB / 4) {
@@ -1179,7 +1180,7 @@ __device__ __forceinline__ double gj_diag(T (&a)[kB], T *slots, T tau, bool &bad
 #pragma unroll 1
   for (int K = 0; K < (Short ? short_steps : kB / 4); ++K) {
     const int c0 = 4 * K;
-    const T *buf = slots + K * kGjSlot;
+    const T *buf = slots + (Short ? (K & 1) : K) * kGjSlot;
     const bool inK = lane >= c0 && lane < c0 + 4;
     // g = f P^-1, f = this row's pivot-column entries (unit vector for pivot rows)
     T f[4];
@@ -1199,7 +1200,7 @@ __device__ __forceinline__ double gj_diag(T (&a)[kB], T *slots, T tau, bool &bad
     }
     gj_update_range<4, 8>(a, g, buf, inK);  // a[0..3]: the next pivot block's columns
     if (K + 1 < kB / 4) {
-      T *nb = slots + (K + 1) * kGjSlot;
+      T *nb = slots + (Short ? ((K + 1) & 1) : K + 1) * kGjSlot;
       const bool next = lane >= c0 + 4 && lane < c0 + 8;
       if (next) {
 #pragma unroll
@@ -2280,7 +2281,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
   }
 }
 
-// log|det| of FP32 draws whose dense core has at most 96 nodes (d_p = 32, 64, 96): the
+// log|det| of FP32 draws whose dense core has at most 128 nodes (d_p = 32 .. 128): the
 // arithmetic of k_lu<float, true>, operation by operation, in blocks of 128 threads,
 // four to an SM.
 //
@@ -2291,16 +2292,20 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
 // global memory is needed.  Panel kb: warp kb inverts its own rows' diagonal block (the
 // chain moves from one SM sub-partition to the next), the warps below split their rows
 // of C and one column of B each; L = C D^-1 and -L B on the tensor cores; then each
-// thread has its row's next 32 columns in registers, the rest stays in tensor memory
-// (columns 0..63: column c - 32 of the core; 64..127: -L B, before it L in 96..127).
+// thread has its row's next 32 columns in registers, the rest stays in tensor memory.
+// Its 128 columns hold the core's column blocks 1, 2 at 0 and 32, -L B at 64..127 and
+// before it L at 96..127.  At d_p = 128 the first panel has three blocks: 2, 3 lie at 0
+// and 32 and block 1 at 64, whose -L B goes to 96..127 alone; then 64..127 are free.
 // 10 000 draws, us (k_lu; with the chunks' program of the levels; now): m = 100 (core 33)
-// 725, 325, 230; m = 133 (45) 765, 358, 258; m = 200 (87) 1161, 595, 489.
-constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32, kSmallMaxDp = 96;
+// 725, 325, 230; m = 133 (45) 765, 358, 258; m = 200 (87) 1161, 595, 489; m = 250 (128)
+// 1545, -, 855.
+constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32, kSmallMaxDp = 128;
 constexpr int kSmallTmem = 128, kSmallTmemU = 64, kSmallTmemL = 96;
 constexpr int kBs = kB + 1;  // stride of the staged columns of B
 struct SmallSmem {
   size_t off_B, off_D, off_prow, off_Lt, off_Ut, off_vals, off_logs, total;
-  static constexpr size_t part_L = (kSmallMaxDp) * 64, part_U = (kSmallMaxDp - kB) * 64;
+  // rows 32.. of the core, columns 32.. of the core
+  static constexpr size_t part_L = (kSmallMaxDp - kB) * 64, part_U = (kSmallMaxDp - kB) * 64;
   __host__ __device__ SmallSmem(int nv, int m) {
     size_t o = 0;
     auto take = [&](size_t bytes) {
@@ -2311,7 +2316,7 @@ struct SmallSmem {
     // B's columns, then (they are split by then) D^-1 split as a B operand
     off_B = take((size_t)(kSmallMaxDp - kB) * kBs * sizeof(float));
     off_D = take((size_t)kB * kDs * sizeof(float));
-    off_prow = take((size_t)(kB / 4) * kGjSlot * sizeof(float));
+    off_prow = take((size_t)2 * kGjSlot * sizeof(float));
     // the level value slots, then the split rows of C / L (rows 32.. of the core) and
     // columns of B
     const size_t panels = 3 * (part_L + part_U), vals = (size_t)nv * sizeof(float);
@@ -2372,6 +2377,11 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = s_tmem, trow = tmem + ((uint32_t)(warp * 32) << 16);
+  // tensor-memory column of the core's column c
+  auto ecol = [&](int c) {
+    const int block = c / kB, at = dp <= 96 ? block - 1 : (block == 1 ? 2 : block - 2);
+    return (uint32_t)(at * kB + (c & (kB - 1)));
+  };
   auto issue = [&](uint32_t d, const unsigned char *b, size_t part_b, uint32_t idesc) {
     if (tid == 0 && mma_live(&s_mbar)) {
       asm volatile("tcgen05.fence::after_thread_sync;");
@@ -2417,7 +2427,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
 #pragma unroll
           for (int q = 0; q < 16; ++q) Bs[(c0 - kB + q) * kBs + lane] = e[q];
         } else {
-          tmem_st16(trow + (uint32_t)(c0 - kB), e);
+          tmem_st16(trow + ecol(c0), e);
         }
       }
       asm volatile("tcgen05.wait::st.sync.aligned;");
@@ -2467,22 +2477,33 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
         write_split_row(Lt, SmallSmem::part_L, row, l);
       }
       operands_ready();
-      issue(tmem + kSmallTmemU, Ut, SmallSmem::part_U, umma_idesc(R));
+      const bool two = R > 64;  // block 1 first, alone
+      const int u0 = two ? kSmallTmemL : kSmallTmemU;
+      issue(tmem + u0, Ut, SmallSmem::part_U, umma_idesc(two ? kB : R));
       mma_wait(&s_mbar, mphase, bad);
       if (below) {
 #pragma unroll
         for (int h = 0; h < kB; h += 16) {  // the next panel's columns
           uint32_t e[16], u[16];
-          tmem_ld16(trow + (uint32_t)(r0 - kB + h), e);
-          tmem_ld16(trow + (uint32_t)(kSmallTmemU + h), u);
+          tmem_ld16(trow + ecol(r0 + h), e);
+          tmem_ld16(trow + (uint32_t)(u0 + h), u);
           asm volatile("tcgen05.wait::ld.sync.aligned;");
 #pragma unroll
           for (int q = 0; q < 16; ++q) a[h + q] = __fadd_rn(__uint_as_float(e[q]), __uint_as_float(u[q]));
         }
+      }
+      if (two) {
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        issue(tmem + kSmallTmemU, Ut + kB * 64, SmallSmem::part_U, umma_idesc(R - kB));
+        mma_wait(&s_mbar, mphase, bad);
+      }
+      if (below) {
         for (int c = kB; c < R; c += 16) {
           uint32_t e[16], u[16];
-          tmem_ld16(trow + (uint32_t)(r0 - kB + c), e);
-          tmem_ld16(trow + (uint32_t)(kSmallTmemU + c), u);
+          tmem_ld16(trow + ecol(r0 + c), e);
+          tmem_ld16(trow + (uint32_t)(kSmallTmemU + (two ? c - kB : c)), u);
           asm volatile("tcgen05.wait::ld.sync.aligned;");
           float s[16];
 #pragma unroll
@@ -2491,7 +2512,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
 #pragma unroll
             for (int q = 0; q < 16; ++q) Bs[(r0 - kB + c + q) * kBs + lane] = s[q];
           } else {
-            tmem_st16(trow + (uint32_t)(r0 - kB + c), s);
+            tmem_st16(trow + ecol(r0 + c), s);
           }
         }
         asm volatile("tcgen05.wait::st.sync.aligned;");

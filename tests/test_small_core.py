@@ -1,4 +1,4 @@
-"""log|det| of FP32 draws with a dense core of at most 96 nodes: the kernel that takes
+"""log|det| of FP32 draws with a dense core of at most 128 nodes: the kernel that takes
 four blocks per SM against the one it replaces there, which forecasts still take when
 the iterative solve is switched off (the same operations, so the same factors: the
 forecasts' log|det| of the same draws agree to the rounding of the FP64 sum of the
@@ -45,7 +45,8 @@ def _both(s, wl, par, n, seed):
 
 @pytest.mark.parametrize("m,kmax,n", [
     (33, 1, 3), (40, 9, 700), (60, 17, 300), (90, 12, 1300), (120, 9, 200), (150, 12, 333),
-    (170, 12, 200), (180, 13, 150), (200, 13, 100), (210, 13, 100)])
+    (170, 12, 200), (180, 13, 150), (200, 13, 100), (210, 13, 100), (240, 17, 300),
+    (255, 17, 100), (275, 17, 60)])
 def test_matches_the_large_kernel(built_lib, m, kmax, n):
     s, wl, par = _engine(m, kmax, 3 + m, min(0.3, 0.8 / kmax))
     d, f, flags = _both(s, wl, par, n, 5)
@@ -59,11 +60,11 @@ def test_matches_the_large_kernel(built_lib, m, kmax, n):
 def test_cores_cover_the_panels(built_lib):
     """The sizes above reach every panel count of the kernel and the first one beyond."""
     cores = set()
-    for m, kmax in ((33, 1), (90, 12), (120, 9), (150, 12), (180, 13), (210, 13)):
+    for m, kmax in ((33, 1), (90, 12), (120, 9), (150, 12), (180, 13), (210, 13), (275, 17)):
         s, _, _ = _engine(m, kmax, 3 + m, 0.1)
         cores.add((s.getEliminationInfo()["core_n"] + 31) // 32)
         s.close()
-    assert {1, 2, 3, 4} <= cores
+    assert {1, 2, 3, 4, 5} <= cores
 
 
 def test_draws_that_need_pivoting(built_lib):
