@@ -161,6 +161,12 @@ void launch_lu(cudaStream_t s, const LuPlan &plan, long n, const EliminationPlan
                int *pivot_list = nullptr,
                // the same form: only the listed draws are factored, or nullptr: all
                const int *draw_list = nullptr);
+// log|det| of unplanned FP32 draws (levels off, d_p above the tensor-core path's) by a
+// cluster of blocks per draw, where scratch holds only `slabs` matrices (d_p x d_p).
+// false: not launched (sizes for which launch_lu is the better choice, or no cluster fits).
+bool launch_lu_cluster(cudaStream_t s, const LuPlan &plan, long n, int slabs, int num_sms,
+                       const unsigned *sp, const float *theta, float *scratch, double *logdet,
+                       int *draw_flags);
 // log|det| of FP64 draws by the deep elimination of elimination.hpp (logdet64.cu).
 // Draws whose elimination needs pivoting are appended to pivot_list; next: the
 // blocks' work counter, zero on entry.

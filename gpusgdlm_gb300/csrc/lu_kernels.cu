@@ -1785,6 +1785,44 @@ __device__ __forceinline__ void copy_vals(T *__restrict__ dst, const T *__restri
   }
 }
 
+// (b) of the panel: rows Rg .. R of C, Lp <- C D^-1 in place; warp (half, quarter) owns
+// 32 rows x 8 columns of each 64-row round, a round reads its rows before writing them.
+// Ends on a barrier.
+template <typename T>
+__device__ __forceinline__ void block_multipliers_rest(T *Lp, const T *D, int Rg, int R, int Rmax, T tau,
+                                                       bool &bad) {
+  constexpr int W = Vec<T>::W;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int qc = (warp >> 1) * 8;
+  for (int t0 = Rg; t0 < R; t0 += 64) {
+    const int t = t0 + (warp & 1) * 32 + lane;
+    const bool act = t < R;
+    T o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = T(0);
+    if (act) {
+#pragma unroll 8
+      for (int c = 0; c < kB; ++c) {
+        const T lv = Lp[c * Rmax + t];
+        T dv[8];
+#pragma unroll
+        for (int j = 0; j < 8; j += W) Vec<T>::ld(D + c * kDs + qc + j, dv + j);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += lv * dv[j];
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (!(dabs(o[j]) <= tau)) bad = true;
+    }
+    __syncthreads();
+    if (act) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) Lp[(qc + j) * Rmax + t] = o[j];
+    }
+  }
+  __syncthreads();
+}
+
 // TC: trailing updates on the tensor cores (FP32 draws, d_p <= 224); a separate
 // instantiation, so that the FFMA path's register tiles do not weigh on it.
 template <typename T, bool TC>
@@ -2128,37 +2166,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
       cp_async_wait_all();
       __syncthreads();
       if (R > Rg) {
-        // (b) rows of C beyond Rg: Lp <- C D^-1 in place; warp (half, quarter) owns
-        // 32 rows x 8 columns of each 64-row round, a round reads its rows before
-        // writing them.
-        const int qc = (warp >> 1) * 8;
-        for (int t0 = Rg; t0 < R; t0 += 64) {
-          const int t = t0 + (warp & 1) * 32 + lane;
-          const bool act = t < R;
-          T o[8];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = T(0);
-          if (act) {
-#pragma unroll 8
-            for (int c = 0; c < kB; ++c) {
-              const T lv = Lp[c * Rmax + t];
-              T dv[8];
-#pragma unroll
-              for (int j = 0; j < 8; j += W) V::ld(D + c * kDs + qc + j, dv + j);
-#pragma unroll
-              for (int j = 0; j < 8; ++j) o[j] += lv * dv[j];
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (!(dabs(o[j]) <= tau)) bad = true;
-          }
-          __syncthreads();
-          if (act) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) Lp[(qc + j) * Rmax + t] = o[j];
-          }
-        }
-        __syncthreads();
+        block_multipliers_rest(Lp, D, Rg, R, Rmax, tau, bad);
         if (solve) {
           const int RW = (R - Rg) / W;
           for (int u = tid; u < kB * RW; u += blockDim.x) {
@@ -2278,6 +2286,125 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
   }
   if constexpr (TC) {
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
+  }
+}
+
+// log|det| of FP32 draws without a plan (the whole matrix is the dense core) where the
+// scratch holds far fewer matrices than the GPU has SMs: a cluster of blocks per draw.
+// The arithmetic of k_lu<float, false>, operation by operation: every block inverts the
+// panel's diagonal block for itself, in step with its half of the rows of C, and updates
+// that half's share of the columns; a cluster barrier per panel orders the matrix in
+// global memory (L2).  What bounds it is the panels' chain of pivot blocks (11 at m = 333,
+// 8 800 of a panel's 22 000 cycles; 8 100 in the trailing update).  1 999 draws at m = 333
+// on 16 MiB (33 matrices): 12.6 ms with a block per draw; with four 7.2 ms, and 9.4 ms
+// with two, 7.8 ms with eight (two blocks to an SM, which slows the chain); with eight
+// that split the columns alone 8.0 ms, the rows alone 9.2 ms (8.2 ms with four).
+__device__ __forceinline__ unsigned cluster_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kThreads, 2)
+    k_lu_cluster(int m, int P, int dp, int cl, long n, const unsigned *__restrict__ sp,
+                 const float *__restrict__ theta_sm, float *__restrict__ scratch,
+                 double *__restrict__ logdet, int *__restrict__ draw_flags) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const Theta<float> theta{theta_sm, nullptr, m, P, 0, n};
+  const Smem L(dp, m, sizeof(float), 0, false);
+  float *D = reinterpret_cast<float *>(smem_raw + L.off_D);
+  float *prow = reinterpret_cast<float *>(smem_raw + L.off_prow);
+  float *Lp = reinterpret_cast<float *>(smem_raw + L.off_Lp);
+  float *Up = reinterpret_cast<float *>(smem_raw + L.off_Up);
+  double *red = reinterpret_cast<double *>(smem_raw + L.off_red);
+  const int Rmax = L.Rmax;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rank = (int)cluster_rank(), cid = (int)(blockIdx.x / (unsigned)cl);
+  float *A = scratch + (size_t)cid * dp * dp;
+  const float tau = (float)kPivotThreshold;
+  __shared__ int sflag;
+  for (long i = cid; i < n; i += gridDim.x / (unsigned)cl) {
+    if (tid == 0) sflag = 0;
+    bool bad = false;
+    double ld_part = 0.0;
+    // ---- the matrix (as build_full), a share each
+    {
+      const size_t n16 = (size_t)dp * dp / 4;
+      float4 *A16 = reinterpret_cast<float4 *>(A);
+      for (size_t e = (size_t)rank * kThreads + tid; e < n16; e += (size_t)cl * kThreads)
+        A16[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      cluster_sync();
+      for (int r = rank * kThreads + tid; r < dp; r += cl * kThreads) A[(size_t)r * dp + r] = 1.f;
+      const size_t mm = (size_t)m * m;
+      for (int e = rank * kThreads + tid; e < m * P; e += cl * kThreads) {
+        const unsigned pos = sp[e];
+        if ((size_t)pos < mm) {
+          const int row = (int)(pos % (unsigned)m), col = (int)(pos / (unsigned)m);
+          A[row + (size_t)dp * col] = -theta.at(i, e);
+        }
+      }
+      cluster_sync();
+    }
+    for (int kb = 0; kb < dp / kB; ++kb) {
+      const int k0 = kb * kB, r0 = k0 + kB, R = dp - r0;
+      // this block's part of the trailing matrix (multiples of 8): rows t0 .. t0 + Rl and
+      // columns c0 .. c1 of the R;
+      // the first kGjRows of the R go through the Gauss-Jordan, the others through D^-1
+      const int rr = rank & 1, rc = rank >> 1, nc = cl >> 1;
+      const int t0 = R / 8 * rr / 2 * 8, Rl = R / 8 * (rr + 1) / 2 * 8 - t0;
+      const int c0 = R / 8 * rc / nc * 8, c1 = R / 8 * (rc + 1) / nc * 8;
+      const int Rg = min(Rl, max(0, kGjRows - t0));
+      const float *C = A + (size_t)(r0 + t0) + (size_t)dp * k0;
+      // rows of C beyond Rg, and B, on their way
+      if (Rl > 0 && c1 > c0) {
+        const int RW = (Rl - Rg) / 4;
+        for (int u = tid; u < kB * RW; u += kThreads) {
+          const int c = u / RW, t = Rg + (u - c * RW) * 4;
+          cp_async16(Lp + c * Rmax + t, C + t + (size_t)dp * c);
+        }
+        for (int u = c0 * 8 + tid; u < c1 * 8; u += kThreads) {
+          const int t = u / 8, q = u - t * 8;
+          cp_async16(Up + t * kUs + q * 4, A + (size_t)(k0 + q * 4) + (size_t)dp * (r0 + t));
+        }
+      }
+      {
+        const int t = (warp - 1) * 32 + lane;  // row of C (warps 1..7)
+        const bool active = (warp == 0) || t < Rg;
+        const float *rowp = warp == 0 ? A + (size_t)(k0 + lane) + (size_t)dp * k0 : C + t;
+        float a[kB];
+#pragma unroll
+        for (int q = 0; q < kB; ++q) a[q] = active ? rowp[(size_t)dp * q] : 0.f;
+        if (warp == 0)
+          ld_part += gj_diag<float, true>(a, prow, tau, bad);
+        else
+          gj_rows<float>(a, active, (warp - 1) * 32 < Rg, prow, tau, bad);
+        if (warp == 0) {
+#pragma unroll
+          for (int q = 0; q < kB; q += 4) Vec<float>::st(D + lane * kDs + q, a + q);
+        } else if (active) {
+#pragma unroll
+          for (int q = 0; q < kB; ++q) Lp[q * Rmax + t] = a[q];
+        }
+      }
+      cp_async_wait_all();
+      __syncthreads();
+      if (Rl > Rg) block_multipliers_rest(Lp, D, Rg, Rl, Rmax, tau, bad);
+      // (the matrix shifted down by t0 rows)
+      if (Rl > 0 && c1 > c0)
+        trailing_update<float>(A + t0, dp, r0, Rl, c0, c1 - c0, Lp, Up + c0 * kUs, Rmax);
+      cluster_sync();  // (also the block's barrier before the panel buffers' next use)
+    }
+    if (bad) atomicOr(&sflag, 1);
+    const double ld_total = block_sum_det(ld_part, red);  // contains __syncthreads
+    if (tid == 0) {
+      if (rank == 0) logdet[i] = ld_total;
+      if (sflag != 0) atomicOr(&draw_flags[i], DRAW_FLAG_PIVOT);
+    }
+    __syncthreads();
   }
 }
 
@@ -3117,6 +3244,49 @@ void launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &
     }
   }
   run(k_lu<T, false>);
+}
+
+bool launch_lu_cluster(cudaStream_t s, const LuPlan &pl, long n, int slabs, int num_sms,
+                       const unsigned *sp, const float *theta, float *scratch, double *logdet,
+                       int *draw_flags) {
+  if (pl.tc || pl.dp <= kB) return false;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  cudaLaunchConfig_t cfg{};
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = pl.smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(k_lu_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem) !=
+      cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  // blocks per draw: as many as the slabs leave room for with a block per SM (33 slabs:
+  // four, 7.2 ms; eight, two blocks per SM: 7.8 ms); a cluster lies within a part of the
+  // GPU, so the clusters that are resident at once are asked for
+  for (int cl = 8; cl >= 2; cl /= 2) {
+    long clusters = std::min<long>(slabs, n);
+    if (clusters * cl > num_sms + cl) continue;
+    attr.val.clusterDim = {(unsigned)cl, 1u, 1u};
+    cfg.gridDim = dim3((unsigned)(clusters * cl));
+    int resident = 0;
+    if (cudaOccupancyMaxActiveClusters(&resident, k_lu_cluster, &cfg) != cudaSuccess || resident < 1) {
+      (void)cudaGetLastError();
+      continue;
+    }
+    // (at least three quarters of the slabs in use)
+    if (4L * resident < 3 * clusters) continue;
+    clusters = std::min<long>(clusters, resident);
+    cfg.gridDim = dim3((unsigned)(clusters * cl));
+    if (cudaLaunchKernelEx(&cfg, k_lu_cluster, pl.m, pl.P, pl.dp, cl, n, sp, theta, scratch, logdet,
+                           draw_flags) == cudaSuccess)
+      return true;
+    (void)cudaGetLastError();
+    return false;
+  }
+  return false;
 }
 
 template <typename T>

@@ -147,9 +147,13 @@ extern "C" int sgdlm_log_det_noalloc(size_t m, size_t max_p, size_t n, const flo
   no_plan.m = (int)m;
   no_plan.P = (int)max_p;
   no_plan.core_n = (int)m;
-  launch_lu<float>(s, pl, (long)n, no_plan, d_sp, d_theta, nullptr, (float *)scratch, d_log_det,
-                   d_flags,
-                   nullptr, nullptr, no_key, false, nullptr, no_rows);
+  // the array holds few matrices (33 at m = 333): several blocks per draw where one per
+  // draw would leave most of the GPU idle
+  if (max_ctas >= sms || !launch_lu_cluster(s, pl, (long)n, (int)max_ctas, sms, d_sp, d_theta,
+                                            (float *)scratch, d_log_det, d_flags))
+    launch_lu<float>(s, pl, (long)n, no_plan, d_sp, d_theta, nullptr, (float *)scratch, d_log_det,
+                     d_flags,
+                     nullptr, nullptr, no_key, false, nullptr, no_rows);
   launch_lu_fallback<float>(s, pl, (long)n, no_plan, d_sp, d_theta, nullptr, (float *)scratch, d_log_det,
                             d_flags,
                             nullptr, nullptr, no_key, nullptr, no_rows);

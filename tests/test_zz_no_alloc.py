@@ -92,6 +92,24 @@ def test_noalloc_matches_oracle_m400():
         assert np.all(fl >= 0)
 
 
+@pytest.mark.parametrize("m,kmax,n", [(225, 6, 70), (256, 5, 1), (257, 9, 130), (333, 11, 67), (460, 4, 40),
+                                      (736, 3, 10)])
+def test_noalloc_several_blocks_per_draw(m, kmax, n):
+    """Matrices of which the 16 MiB array holds fewer than the GPU has SMs: a cluster of
+    blocks shares each draw (column shares of every width, one draw, more draws than
+    matrices).  The same operations as the allocating entry point's dense LU."""
+    import bench
+
+    wl = bench.make_workload(m=m, kmax=kmax, T=3, seed=m)
+    P = wl["P"]
+    sp = np.where(wl["sp"] >= m * m, np.nan, wl["sp"]).astype(float)
+    d, st = _engine_draws(m, P, wl["p"], sp, np.full((P, m), 0.05), np.repeat((0.001 * np.eye(P))[:, :, None], m, axis=2), n)
+    th = _series_major(d["thetas"])
+    for ld, fl in _call_noalloc(m, P, n, th, wl["sp"]):
+        np.testing.assert_allclose(ld, d["log_dets"], rtol=0, atol=1e-9)
+        assert (np.asarray(fl) != 0).sum() == st["draws_pivoted"]
+
+
 def test_noalloc_matches_oracle_with_pivoting():
     m, P, n = 3, 1, 300
     sp = np.array([[0 + 3 * 1, 1 + 3 * 0, 2 + 3 * 0]], dtype=np.float64)
