@@ -11,6 +11,8 @@
 // contiguous coalesced run.  From the same staged rows the block writes its draws'
 // Gamma entries to the draw-major Gamma copy (GammaDraws), which the LU and
 // iterative-solve kernels read as one run per draw.
+#include <type_traits>
+
 #include "kernels.hpp"
 #include "rng.cuh"
 
@@ -56,7 +58,51 @@ __device__ __forceinline__ void write_gamma_runs(const GammaDraws<T> &gd, int P,
   }
 }
 
-template <typename T, int PMAX>
+// W values of 16 bytes (aligned).
+template <typename T> struct V16 {
+  static constexpr int W = (int)(16 / sizeof(T));
+  __device__ static __forceinline__ void ld(const T *p, T *o) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(p);
+    const T *t = reinterpret_cast<const T *>(&v);
+#pragma unroll
+    for (int b = 0; b < W; ++b) o[b] = t[b];
+  }
+  __device__ static __forceinline__ void st(T *p, const T *o) {
+    uint4 v;
+    T *t = reinterpret_cast<T *>(&v);
+#pragma unroll
+    for (int b = 0; b < W; ++b) t[b] = o[b];
+    *reinterpret_cast<uint4 *>(p) = v;
+  }
+};
+
+// sum_{l <= k} U[l + P k] z[l] in increasing l; VEC: P is a multiple of V16<T>::W, so that
+// every column of U starts on 16 bytes (the padding behind l = k is read, not used).
+template <typename T, bool VEC>
+__device__ __forceinline__ T column_dot(const T *Us, int P, int k, const T *z) {
+  constexpr int W = V16<T>::W;
+  T acc = T(0);
+  if constexpr (VEC) {
+#pragma unroll
+    for (int l = 0; l <= k; l += W) {
+      T u[W];
+      V16<T>::ld(Us + l + P * k, u);
+#pragma unroll
+      for (int b = 0; b < W; ++b)
+        if (l + b <= k) acc += u[b] * z[l + b];
+    }
+  } else {
+#pragma unroll
+    for (int l = 0; l <= k; ++l) acc += Us[l + P * k] * z[l];
+  }
+  return acc;
+}
+
+// Both kernels: VEC (P a multiple of four FP32 or two FP64 values) reads U's columns and
+// the staged rows 16 bytes at a time.  A row of P = 20 FP32 values read and written value by
+// value meets four-way bank conflicts (20 l mod 32 takes eight values), as 16-byte accesses
+// none; an odd P has none either way.
+template <typename T, int PMAX, bool VEC>
 __global__ void __launch_bounds__(kSampleThreads)
     k_sample(int m, int P, long n, const double *__restrict__ m_t,
              const double *__restrict__ n_t, const double *__restrict__ s_t,
@@ -111,15 +157,25 @@ __global__ void __launch_bounds__(kSampleThreads)
     // one reciprocal instead of P divisions (within 1-2 ulp of the quotients)
     const T rden = T(1) / dev_sqrt(ser[1] * lam);
     T *row = stage + (size_t)threadIdx.x * P;
+    constexpr int W = VEC ? V16<T>::W : 1;
 #pragma unroll
-    for (int k = 0; k < PMAX; ++k) {
+    for (int k = 0; k < PMAX; k += W) {
       if (k < P) {
-        T acc = T(0);
-        if (k < pj) {
+        T o[W];
+        if constexpr (VEC)
+          V16<T>::ld(ms + k, o);
+        else
+          o[0] = ms[k];
 #pragma unroll
-          for (int l = 0; l <= k; ++l) acc += Us[l + P * k] * z[l];
+        for (int b = 0; b < W; ++b) {
+          T acc = T(0);
+          if (k + b < pj) acc = column_dot<T, VEC>(Us, P, k + b, z);
+          o[b] = o[b] + acc * rden;
         }
-        row[k] = ms[k] + acc * rden;
+        if constexpr (VEC)
+          V16<T>::st(row + k, o);
+        else
+          row[k] = o[0];
       }
     }
     lambda[(size_t)j * n + i] = lam;
@@ -144,7 +200,12 @@ __global__ void __launch_bounds__(kSampleThreads)
 // make_beta, kernel_functions.cuh:644-798); lambda *= eta (batchedMultiply
 // :458-466); omega ~ N(0, I) scaled by 1/sqrt(c lambda) and cut at p
 // (scale_omegas :986-1001); theta += U_W' omega (SGDLM.cu:755-758).
-template <typename T, int PMAX>
+// Bound by the instructions of a (draw, series) pair, most of them the random numbers'.
+// The series' inactive coefficients (k >= p_j: U_W is zero outside its leading block, their
+// omega is cut) take no normals, quotients or products; the rows of theta are on their way
+// (cp.async) while the gammas are drawn.  m = 400, P = 20 (11.9 active on average), 10 000
+// draws, FP32: 752 us with all of it over P coefficients, 522 us so.
+template <typename T, int PMAX, bool VEC>
 __global__ void __launch_bounds__(kSampleThreads)
     k_evolve(int m, int P, long n, const unsigned *__restrict__ p,
              const double *__restrict__ r_t, const double *__restrict__ c_t,
@@ -159,6 +220,8 @@ __global__ void __launch_bounds__(kSampleThreads)
   __shared__ int gks[64], gcnt, gq0;  // the series' Gamma coefficients (gamma_row_of)
   __shared__ GammaShape<T> shapes[2];  // of the Beta draw's two gammas
   const int j = blockIdx.y;
+  // the reference's unscaled omegas are not cut at p_j: all P take part then
+  const int na = compat_unscaled ? P : min(P, (int)p[j]);
   if (threadIdx.x < 64 && threadIdx.x % 32 == 0) {  // one thread of warps 0 and 1 each
     const double bj = beta[j], rj = r_t[j];
     const bool second = threadIdx.x == 32;
@@ -172,13 +235,26 @@ __global__ void __launch_bounds__(kSampleThreads)
   for (int e = threadIdx.x; e < P * P; e += blockDim.x) Us[e] = UW[(size_t)j * P * P + e];
   if (G)
     for (int e = threadIdx.x; e < P * P; e += blockDim.x) Gs[e] = G[(size_t)j * P * P + e];
-  for (long e = threadIdx.x; e < cnt; e += blockDim.x) stage[e] = src[e];
+  const bool run16 = ((size_t)j * n + i0) * P * sizeof(T) % 16 == 0 && cnt * sizeof(T) % 16 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(stage) | reinterpret_cast<uintptr_t>(theta)) & 15) == 0;
+  if (run16) {
+    constexpr int W16 = V16<T>::W;
+    for (long e = (long)threadIdx.x * W16; e < cnt; e += (long)blockDim.x * W16)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
+                       (unsigned)__cvta_generic_to_shared(stage + e)),
+                   "l"(src + e)
+                   : "memory");
+  } else {
+    for (long e = threadIdx.x; e < cnt; e += blockDim.x) stage[e] = src[e];
+  }
   __syncthreads();
   const long i = i0 + threadIdx.x;
+  T w[PMAX];
+  bool fail = false;
   if (i < n) {
     const uint32_t ep = key_epoch(key);
+    const T lam0 = lambda[(size_t)j * n + i];
     const double bj = beta[j];
-    bool fail = false;
     T eta = T(1);
     if (bj != 1.0) {
       const T ga = gamma_mt<T>(shapes[0], (uint32_t)i, (uint32_t)j, TAG_BETA_A, ep, key.k0, key.k1,
@@ -187,12 +263,11 @@ __global__ void __launch_bounds__(kSampleThreads)
                                key.tab, &fail);
       eta = (ga / (ga + gb)) / (T)bj;
     }
-    const T lam = lambda[(size_t)j * n + i] * eta;
+    const T lam = lam0 * eta;
     lambda[(size_t)j * n + i] = lam;
-    T w[PMAX];
 #pragma unroll
     for (int q = 0; q < PMAX / 4; ++q) {
-      if (4 * q < P) {
+      if (4 * q < na) {
         const U4 r = philox((uint32_t)i, (uint32_t)j, tag_sub(TAG_OMEGA, q), ep, key.k0, key.k1);
         box_muller<T>(r.x, r.y, w[4 * q], w[4 * q + 1], key.tab);
         box_muller<T>(r.z, r.w, w[4 * q + 2], w[4 * q + 3], key.tab);
@@ -210,6 +285,10 @@ __global__ void __launch_bounds__(kSampleThreads)
 #pragma unroll
       for (int k = 0; k < PMAX; ++k) w[k] = ((unsigned)k < pj) ? w[k] / den : T(0);
     }
+  }
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncthreads();  // the staged rows
+  if (i < n) {
     T *row = stage + (size_t)threadIdx.x * P;
     if (G) {
       // theta = G theta over the full max_p x max_p product (SGDLM.cu:729-740)
@@ -225,24 +304,64 @@ __global__ void __launch_bounds__(kSampleThreads)
       for (int k = 0; k < PMAX; ++k)
         if (k < P) row[k] = g[k];
     }
+    constexpr int W = VEC ? V16<T>::W : 1;
 #pragma unroll
-    for (int k = 0; k < PMAX; ++k) {
+    for (int k = 0; k < PMAX; k += W) {
       if (k < P) {
-        T acc = T(0);
+        T o[W];
+        if constexpr (VEC)
+          V16<T>::ld(row + k, o);
+        else
+          o[0] = row[k];
 #pragma unroll
-        for (int l = 0; l <= k; ++l) acc += Us[l + P * k] * w[l];
-        row[k] = acc + row[k];
+        for (int b = 0; b < W; ++b) {
+          T acc = T(0);
+          if (k + b < na) acc = column_dot<T, VEC>(Us, P, k + b, w);
+          o[b] = acc + o[b];
+        }
+        if constexpr (VEC)
+          V16<T>::st(row + k, o);
+        else
+          row[k] = o[0];
       }
     }
     if (fail) atomicOr(&draw_flags[i], DRAW_FLAG_GAMMA_CAP);
   }
   __syncthreads();
   if (gd.v) write_gamma_runs<T>(gd, P, i0, (int)min((long)blockDim.x, n - i0), stage, gks, gcnt, gq0);
-  for (long e = threadIdx.x; e < cnt; e += blockDim.x) src[e] = stage[e];
+  if (run16) {
+    constexpr int W16 = V16<T>::W;
+    for (long e = (long)threadIdx.x * W16; e < cnt; e += (long)blockDim.x * W16)
+      *reinterpret_cast<uint4 *>(src + e) = *reinterpret_cast<const uint4 *>(stage + e);
+  } else {
+    for (long e = threadIdx.x; e < cnt; e += blockDim.x) src[e] = stage[e];
+  }
 }
 
 template <typename T> size_t sample_smem(int P) {
   return ((size_t)P * P + P + (size_t)kSampleThreads * P) * sizeof(T);
+}
+
+// The instantiation for P coefficients: registers for 8, 16, 24, 32 or 64 of them, and
+// 16-byte accesses where P allows them (above 32 the unrolled products are instructions
+// enough once).
+template <typename T, typename F> void by_width(int P, F f) {
+  const auto pick = [&](auto pm) {
+    if (P % V16<T>::W == 0)
+      f(pm, std::true_type{});
+    else
+      f(pm, std::false_type{});
+  };
+  if (P <= 8)
+    pick(std::integral_constant<int, 8>{});
+  else if (P <= 16)
+    pick(std::integral_constant<int, 16>{});
+  else if (P <= 24)
+    pick(std::integral_constant<int, 24>{});
+  else if (P <= 32)
+    pick(std::integral_constant<int, 32>{});
+  else
+    f(std::integral_constant<int, 64>{}, std::false_type{});
 }
 
 }  // namespace
@@ -253,28 +372,11 @@ void launch_sample(cudaStream_t s, int m, int P, long n, const double *m_t,
                    T *lambda, T *theta, GammaDraws<T> gd, int *draw_flags, const unsigned *p) {
   dim3 grid((unsigned)((n + kSampleThreads - 1) / kSampleThreads), (unsigned)m);
   const size_t smem = sample_smem<T>(P);
-  if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(k_sample<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_sample<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_sample<T, 24>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_sample<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_sample<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
-  if (P <= 8)
-    k_sample<T, 8><<<grid, kSampleThreads, smem, s>>>(m, P, n, m_t, n_t, s_t, U, key,
-                                                      lambda, theta, gd, draw_flags, p);
-  else if (P <= 16)
-    k_sample<T, 16><<<grid, kSampleThreads, smem, s>>>(m, P, n, m_t, n_t, s_t, U, key,
-                                                       lambda, theta, gd, draw_flags, p);
-  else if (P <= 24)
-    k_sample<T, 24><<<grid, kSampleThreads, smem, s>>>(m, P, n, m_t, n_t, s_t, U, key,
-                                                       lambda, theta, gd, draw_flags, p);
-  else if (P <= 32)
-    k_sample<T, 32><<<grid, kSampleThreads, smem, s>>>(m, P, n, m_t, n_t, s_t, U, key,
-                                                       lambda, theta, gd, draw_flags, p);
-  else
-    k_sample<T, 64><<<grid, kSampleThreads, smem, s>>>(m, P, n, m_t, n_t, s_t, U, key,
-                                                       lambda, theta, gd, draw_flags, p);
+  by_width<T>(P, [&](auto pm, auto vec) {
+    auto *f = k_sample<T, pm.value, vec.value>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    f<<<grid, kSampleThreads, smem, s>>>(m, P, n, m_t, n_t, s_t, U, key, lambda, theta, gd, draw_flags, p);
+  });
 }
 
 template <typename T>
@@ -286,26 +388,12 @@ void launch_evolve(cudaStream_t s, int m, int P, long n, const unsigned *p,
   dim3 grid((unsigned)((n + kSampleThreads - 1) / kSampleThreads), (unsigned)m);
   const size_t smem =
       ((size_t)P * P * (G ? 2 : 1) + (size_t)kSampleThreads * P) * sizeof(T);
-  if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(k_evolve<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_evolve<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_evolve<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_evolve<T, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
-#define SGDLM_EVOLVE(PM)                                                              \
-  k_evolve<T, PM><<<grid, kSampleThreads, smem, s>>>(m, P, n, p, r_t, c_t, beta, UW, \
-                                                     key, compat_unscaled_omega,      \
-                                                     compat_beta_no_boost, lambda,    \
-                                                     theta, gd, draw_flags, G)
-  if (P <= 8)
-    SGDLM_EVOLVE(8);
-  else if (P <= 16)
-    SGDLM_EVOLVE(16);
-  else if (P <= 32)
-    SGDLM_EVOLVE(32);
-  else
-    SGDLM_EVOLVE(64);
-#undef SGDLM_EVOLVE
+  by_width<T>(P, [&](auto pm, auto vec) {
+    auto *f = k_evolve<T, pm.value, vec.value>;
+    if (smem > 48 * 1024) cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    f<<<grid, kSampleThreads, smem, s>>>(m, P, n, p, r_t, c_t, beta, UW, key, compat_unscaled_omega,
+                                         compat_beta_no_boost, lambda, theta, gd, draw_flags, G);
+  });
 }
 
 template void launch_sample<float>(cudaStream_t, int, int, long, const double *,
