@@ -26,8 +26,12 @@
 // both.  The sweeps are bound by the gathers' shared-memory wavefronts (bank
 // conflicts: 32 scattered 4-byte loads take about 3.5, two 16-lane phases of 8-byte
 // loads about 6 for two draws) and by issue slots.  10 000 FP32 draws at m = 400: one
-// draw per block 908 us, two 833 us, four 949 us (the registers leave one block per
-// SM); FP64 draws: two 1.52 ms, four 1.87 ms, and 94.5 ms with FP64 factors.
+// draw per block 908 us, two 833 us, four 949 us (one block per SM each); two with the
+// registers cut to 72 a thread, so that two blocks share an SM and one sweeps while the
+// other waits at its barrier (K <= 20, a few spilled words outside the sweeps), 758 us;
+// and with the residual's conversions to FP64, three FP64-rate instructions per entry
+// before, down to one, 628 us.  FP64 draws: two 1.52 ms, four 1.87 ms, and 94.5 ms with
+// FP64 factors.
 #include <algorithm>
 
 #include "kernels.hpp"
@@ -37,6 +41,7 @@ namespace {
 
 constexpr int kJacMaxThreads = 1024;  // one row per thread: m <= 1024
 constexpr int kJacGroupThreads = 512;  // two draws per block: m <= 512 (registers)
+constexpr int kJacPairThreads = 448;   // and two such blocks on an SM: m <= 448
 constexpr int kMaxSweeps = 128;
 // The first solve stops at max|dy| <= 2^-20 max|y|; the FP32 draws' correction,
 // whose size is that of y's error, needs only 2^-10 of its own size: y + d is then
@@ -49,7 +54,7 @@ constexpr double kDoneTol = 1.4551915228366852e-11;  // 2^-36: FP64 draws' last 
 constexpr int kMaxCorrections = 4;                    // FP64 draws
 
 struct JacSmem {
-  size_t yd, xa, xb, yv, red, total;
+  size_t yd, xa, xb, red, total;
   __host__ __device__ JacSmem(int m, int nb) {
     size_t o = 0;
     auto take = [&](size_t bytes) {
@@ -60,7 +65,6 @@ struct JacSmem {
     yd = take((size_t)m * nb * sizeof(double));
     xa = take((size_t)m * nb * sizeof(float));
     xb = take((size_t)m * nb * sizeof(float));
-    yv = take((size_t)m * nb * sizeof(float));
     red = take(4 * (size_t)nb * sizeof(unsigned));
     total = o;
   }
@@ -94,6 +98,18 @@ template <int NB> __device__ __forceinline__ void st_row(double *x, int r, const
     reinterpret_cast<double2 *>(x)[r] = make_double2(v[0], v[1]);
   else
     x[r] = v[0];
+}
+
+// (double)f of a finite f that is zero or a normal number, in integer instructions: the
+// conversion instruction runs at the FP64 rate.
+__device__ __forceinline__ double widen(float f) {
+  const unsigned b = __float_as_uint(f), a = b & 0x7FFFFFFFu;
+  const unsigned hi = (a >> 3) + (a ? (1023u - 127u) << 20 : 0u);
+  return __hiloint2double((int)(hi | (b & 0x80000000u)), (int)(b << 29));
+}
+__device__ __forceinline__ bool is_tiny(float f) {  // not zero, below the normal numbers
+  const unsigned a = __float_as_uint(f) & 0x7FFFFFFFu;
+  return a - 1u < 0x007FFFFFu;
 }
 
 // A non-negative float as an ordered integer key; a NaN counts as infinity.
@@ -209,8 +225,11 @@ __device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row
   return conv;
 }
 
-template <typename T, int K, int NB>
-__global__ void __launch_bounds__(NB > 1 ? kJacGroupThreads : kJacMaxThreads)
+// FULL: one block of up to kJacMaxThreads (one draw) or kJacGroupThreads (two) per SM;
+// otherwise (two draws, m <= kJacPairThreads) registers for two blocks.
+template <typename T, int K, int NB, bool FULL>
+__global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairThreads) : kJacMaxThreads,
+                                  FULL ? 1 : 2)
     k_forecast_jacobi(int m, long n, GammaRows rows, const T *__restrict__ theta_g, int nnz,
                       const double *__restrict__ nu, double *__restrict__ y,
                       double *__restrict__ logdet, int *__restrict__ list,
@@ -222,7 +241,6 @@ __global__ void __launch_bounds__(NB > 1 ? kJacGroupThreads : kJacMaxThreads)
   double *yds = reinterpret_cast<double *>(smem_raw + L.yd);
   float *xa = reinterpret_cast<float *>(smem_raw + L.xa);
   float *xb = reinterpret_cast<float *>(smem_raw + L.xb);
-  float *yv = reinterpret_cast<float *>(smem_raw + L.yv);
   unsigned *red = reinterpret_cast<unsigned *>(smem_raw + L.red);
   const int tid = threadIdx.x;
   const bool mine = tid < m;
@@ -259,19 +277,38 @@ __global__ void __launch_bounds__(NB > 1 ? kJacGroupThreads : kJacMaxThreads)
       for (int b = 0; b < NB; ++b) c[b] = (float)nud[b];
       ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kSweepTol, ok, yo);
       if (ok) {
-        // residual in FP64 and its correction by the same iteration
-        if (mine) st_row<NB>(yv, r, yo);
+        // residual in FP64 and its correction by the same iteration.  The iterates are
+        // widened once per row, the Gamma entries without the conversion instruction
+        // (those of a draw that is still solved here are finite)
+        double v[NB], yw[NB];
+        bool tiny = false;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          yw[b] = (double)yo[b];
+          v[b] = nud[b] - yw[b];
+#pragma unroll
+          for (int q = 0; q < K; ++q) tiny |= is_tiny(R.val[b][q]);
+        }
+        if (mine) st_row<NB>(yds, r, yw);
         __syncthreads();
-        double v[NB];
+        if (!__any_sync(0xffffffffu, tiny)) {
 #pragma unroll
-        for (int b = 0; b < NB; ++b) v[b] = nud[b] - (double)yo[b];
+          for (int q = 0; q < K; ++q) {
+            if (q >= wlen) break;
+            double u[NB];
+            ld_row<NB>(yds, R.c(q), u);
 #pragma unroll
-        for (int q = 0; q < K; ++q) {
-          if (q >= wlen) break;
-          float u[NB];
-          ld_row<NB>(yv, R.c(q), u);
+            for (int b = 0; b < NB; ++b) v[b] += widen(R.val[b][q]) * u[b];
+          }
+        } else {
 #pragma unroll
-          for (int b = 0; b < NB; ++b) v[b] += (double)R.val[b][q] * (double)u[b];
+          for (int q = 0; q < K; ++q) {
+            if (q >= wlen) break;
+            double u[NB];
+            ld_row<NB>(yds, R.c(q), u);
+#pragma unroll
+            for (int b = 0; b < NB; ++b) v[b] += (double)R.val[b][q] * u[b];
+          }
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) c[b] = (float)v[b];
@@ -388,15 +425,19 @@ __global__ void __launch_bounds__(NB > 1 ? kJacGroupThreads : kJacMaxThreads)
 
 // ELL widths: the smallest of these that holds the longest row
 constexpr int kJacWidths[] = {8, 12, 16, 18, 20, 24, 32};
+// and the widest of those whose FP32 kernels fit 72 registers with few spills
+constexpr int kJacPairWidth = 20;
 
 // Calls f with the kernel of type T, width K and draws per block (group: two).
-template <typename T, typename F> void with_jacobi_kernel(int K, bool group, F f) {
-#define SGDLM_JACOBI(KK)                  \
-  case KK:                                \
-    if (group)                            \
-      f(k_forecast_jacobi<T, KK, 2>, 2);  \
-    else                                  \
-      f(k_forecast_jacobi<T, KK, 1>, 1);  \
+template <typename T, typename F> void with_jacobi_kernel(int K, bool group, int threads, F f) {
+#define SGDLM_JACOBI(KK)                                                           \
+  case KK:                                                                         \
+    if (group && threads <= kJacPairThreads && sizeof(T) == 4 && KK <= kJacPairWidth) \
+      f(k_forecast_jacobi<T, KK, 2, (sizeof(T) > 4 || KK > kJacPairWidth)>, 2);    \
+    else if (group)                                                                \
+      f(k_forecast_jacobi<T, KK, 2, true>, 2);                                     \
+    else                                                                           \
+      f(k_forecast_jacobi<T, KK, 1, true>, 1);                                     \
     break
   switch (K) {
     SGDLM_JACOBI(8);
@@ -427,7 +468,7 @@ template <typename T> JacobiPlan plan_jacobi(int m, int max_row, int num_sms) {
     if (g == 1 && jp.threads > kJacGroupThreads) break;
     int per_sm = 0;
     cudaError_t e = cudaSuccess;
-    with_jacobi_kernel<T>(jp.nnz, g == 1, [&](auto kernel, int nb) {
+    with_jacobi_kernel<T>(jp.nnz, g == 1, jp.threads, [&](auto kernel, int nb) {
       jp.draws[g] = nb;
       jp.smem[g] = JacSmem(m, nb).total;
       if (jp.smem[g] > 48 * 1024)
@@ -457,7 +498,7 @@ void launch_forecast_jacobi(cudaStream_t s, const JacobiPlan &jp, int m, long n,
   const int g = jp.draws[1] > 0 && n >= (long)jp.grid[1] * jp.draws[1] / 2 ? 1 : 0;
   const long blocks = (n + jp.draws[g] - 1) / jp.draws[g];
   const unsigned grid = (unsigned)std::max<long>(std::min<long>(jp.grid[g], blocks), 1);
-  with_jacobi_kernel<T>(jp.nnz, g == 1, [&](auto kernel, int) {
+  with_jacobi_kernel<T>(jp.nnz, g == 1, jp.threads, [&](auto kernel, int) {
     if (jp.smem[g] > 48 * 1024)
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jp.smem[g]);
     kernel<<<grid, (unsigned)jp.threads, jp.smem[g], s>>>(m, n, rows, theta_g, nnz, nu, y, logdet, list,

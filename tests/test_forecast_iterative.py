@@ -76,3 +76,25 @@ def test_draws_do_not_depend_on_their_block(built_lib, precision, m):
     few = _forecast(s, wl, 3, x, True)
     np.testing.assert_array_equal(few, many[:, :3])
     s.close()
+
+
+@pytest.mark.parametrize("m,kmax,mean", [(31, 4, 0.05), (447, 17, 0.05), (448, 20, 0.05), (449, 17, 0.05),
+                                         (448, 17, 1e-40), (200, 8, 0.0)])
+def test_fp32_two_blocks_per_sm(built_lib, m, kmax, mean):
+    """FP32 draws at and beside the largest system of the form with two blocks on an SM,
+    with Gamma entries below the normal FP32 numbers and at zero: both paths correct an FP32
+    solve (relative error 2^-20 at most) by a solve of its FP64 residual, so they are within
+    about 2^-30 of the solution; 1e-8 leaves a factor of five for each."""
+    s, wl = _engine(m, kmax, "mixed")
+    P = wl["P"]
+    rng = np.random.default_rng(m)
+    s.setPriorParameters(rng.uniform(-mean, mean, size=(P, m)),
+                         np.repeat(((1e-4 if mean > 1e-9 else 1e-90) * np.eye(P))[:, :, None], m, axis=2),
+                         np.full(m, 20.0), np.full(m, 1.0))
+    x = wl["F_of"](2, False)
+    y = _forecast(s, wl, 5001, x, True)
+    assert s.getStats()["forecast_draws_factored"] == 0
+    ref = _forecast(s, wl, 5001, x, False)
+    err = np.abs(y - ref).max(axis=0) / np.abs(ref).max(axis=0)
+    assert err.max() <= 1e-8
+    s.close()
