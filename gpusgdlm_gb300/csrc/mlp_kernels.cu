@@ -20,64 +20,148 @@
 namespace sgdlm {
 namespace {
 
-constexpr int kTile = 32;
-
-template <typename T> __device__ __forceinline__ float to_f(T v);
-template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
-template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) {
-  return __bfloat162float(v);
-}
-
-// C[i, j] (+)= sum_k A(i, k) B(k, j), A(i, k) = A[i*sai + k*sak],
-// B(k, j) = B[k*sbk + j*sbj], C row-major with leading dimension ldc; 32 x 32
-// output tiles, 16 x 16 threads with 2 x 2 outputs each, K in chunks of 32
-// staged in shared memory, FP32 accumulation.  Optional epilogue: + bias[j],
-// store the pre-activation to Z, apply GELU; or times GELU'(Zg) (the backward's
+// C[i, j] = sum_k A[i, k] B(k, j), A row-major (M x K), B BF16: the N x K row-major matrix
+// (BT) or the K x N one; C row-major with leading dimension ldc.  Optional epilogue:
+// + bias[j], store the pre-activation to Z, apply GELU; or times GELU'(Zg) (the backward's
 // dZ = dA * GELU'(Z)).
-template <typename TB>
-__global__ void __launch_bounds__(256)
-    k_matmul(int M, int N, int K, const float *__restrict__ A, long sai, long sak,
-             const TB *__restrict__ B, long sbk, long sbj, float *__restrict__ C, int ldc,
-             const float *__restrict__ bias, float *__restrict__ Z, int gelu,
-             const float *__restrict__ Zg) {
-  __shared__ float As[kTile][kTile + 1];
-  __shared__ float Bs[kTile][kTile + 1];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int i0 = blockIdx.y * kTile, j0 = blockIdx.x * kTile;
-  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-  for (int k0 = 0; k0 < K; k0 += kTile) {
-    for (int e = threadIdx.x; e < kTile * kTile; e += blockDim.x) {
-      const int r = e / kTile, c = e % kTile;
+//
+// FP32 sums in increasing k, one thread per output, as long as the network is this narrow
+// (K, N <= 128: a layer of 4 096 rows is 67 MFMA, 2 us of the FP32 pipe, and 1 us of
+// memory).  Bound by shared-memory loads and by the latency of the K chunks' loads: 32 x 64
+// outputs per block of 128 threads, 4 x 4 each (two 16-byte loads per 16 FMAs), so that a
+// layer of 4 096 rows is 256 blocks and one of 200 series still 14; the next chunk's values
+// come into registers while the current one is multiplied, two buffers, one barrier per
+// chunk.  4 096 x 128 x 128: 15.7 us with 2 x 2 outputs per thread and 32 x 32 tiles,
+// 10.1 us (11.2 us with GELU') so; 200 rows: 12.4 us, 9.1 us.
+constexpr int kTileM = 32, kTileN = 64, kTileK = 32, kMatThreads = 128;
+template <bool BT>
+__global__ void __launch_bounds__(kMatThreads)
+    k_matmul(int M, int N, int K, const float *__restrict__ A, const __nv_bfloat16 *__restrict__ B,
+             float *__restrict__ C, int ldc, const float *__restrict__ bias, float *__restrict__ Z,
+             int gelu, const float *__restrict__ Zg) {
+  __shared__ __align__(16) float As[2][kTileM][kTileK + 4];  // [i][k]
+  __shared__ __align__(16) float Bs[2][kTileK][kTileN + 4];  // [k][j]
+  constexpr int NA = kTileM * kTileK / kMatThreads, NB = kTileK * kTileN / kMatThreads;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int i0 = blockIdx.y * kTileM, j0 = blockIdx.x * kTileN;
+  float ra[NA], rb[NB];
+  // the thread's e-th value of A's and B's chunk: A by rows; B by rows of j, or (BT) eight
+  // k by four j per 32 values (distinct banks in Bs)
+  auto at_a = [&](int e, int &r, int &c) {
+    r = (e * kMatThreads + tid) / kTileK;
+    c = tid % kTileK;
+  };
+  auto at_b = [&](int e, int &k, int &j) {
+    if (BT) {
+      const int g = e * (kMatThreads / 32) + tid / 32;
+      k = g % (kTileK / 8) * 8 + tid % 8;
+      j = g / (kTileK / 8) * 4 + tid % 32 / 8;
+    } else {
+      k = (e * kMatThreads + tid) / kTileN;
+      j = tid % kTileN;
+    }
+  };
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int e = 0; e < NA; ++e) {
+      int r, c;
+      at_a(e, r, c);
       const int i = i0 + r, k = k0 + c;
-      As[r][c] = (i < M && k < K) ? A[(long)i * sai + (long)k * sak] : 0.f;
-      const int kk = k0 + r, j = j0 + c;
-      Bs[r][c] = (kk < K && j < N) ? to_f(B[(long)kk * sbk + (long)j * sbj]) : 0.f;
+      ra[e] = (i < M && k < K) ? A[(long)i * K + k] : 0.f;
     }
-    __syncthreads();
-#pragma unroll 8
-    for (int k = 0; k < kTile; ++k) {
-      const float a0 = As[ty][k], a1 = As[ty + 16][k];
-      const float b0 = Bs[k][tx], b1 = Bs[k][tx + 16];
-      acc[0][0] = fmaf(a0, b0, acc[0][0]);
-      acc[0][1] = fmaf(a0, b1, acc[0][1]);
-      acc[1][0] = fmaf(a1, b0, acc[1][0]);
-      acc[1][1] = fmaf(a1, b1, acc[1][1]);
+#pragma unroll
+    for (int e = 0; e < NB; ++e) {
+      int k, j;
+      at_b(e, k, j);
+      k += k0, j += j0;
+      rb[e] = (k < K && j < N) ? __bfloat162float(B[BT ? (long)j * K + k : (long)k * N + j]) : 0.f;
     }
-    __syncthreads();
+  };
+  float acc[4][4] = {};
+  fetch(0);
+  // this thread's outputs: rows i .. i + 3, columns j .. j + 3, 16 bytes at a time where
+  // the rows of C, Z and Zg allow it; Zg is on its way during the products
+  const int i = i0 + 4 * ty, j = j0 + 4 * tx;
+  const bool vec = j + 3 < N && ldc % 4 == 0 &&
+                   ((reinterpret_cast<uintptr_t>(C) | reinterpret_cast<uintptr_t>(Z) |
+                     reinterpret_cast<uintptr_t>(Zg)) & 15) == 0;
+  float zg[4][4] = {};
+  if (Zg) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (i + u >= M) break;
+      const float *src = Zg + (long)(i + u) * ldc + j;
+      if (vec) {
+        const float4 v = *reinterpret_cast<const float4 *>(src);
+        zg[u][0] = v.x, zg[u][1] = v.y, zg[u][2] = v.z, zg[u][3] = v.w;
+      } else {
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (j + v < N) zg[u][v] = src[v];
+      }
+    }
   }
+  int buf = 0;
+  for (int k0 = 0; k0 < K; k0 += kTileK, buf ^= 1) {
+    // (the buffer was read two chunks ago, before the last barrier)
 #pragma unroll
-  for (int u = 0; u < 2; ++u)
-#pragma unroll
-    for (int v = 0; v < 2; ++v) {
-      const int i = i0 + ty + 16 * u, j = j0 + tx + 16 * v;
-      if (i >= M || j >= N) continue;
-      float x = acc[u][v];
-      if (bias) x += bias[j];
-      if (Z) Z[(long)i * ldc + j] = x;
-      if (gelu) x = gelu_f(x);
-      if (Zg) x *= gelu_grad_f(Zg[(long)i * ldc + j]);
-      C[(long)i * ldc + j] = x;
+    for (int e = 0; e < NA; ++e) {
+      int r, c;
+      at_a(e, r, c);
+      As[buf][r][c] = ra[e];
     }
+#pragma unroll
+    for (int e = 0; e < NB; ++e) {
+      int k, j;
+      at_b(e, k, j);
+      Bs[buf][k][j] = rb[e];
+    }
+    __syncthreads();
+    if (k0 + kTileK < K) fetch(k0 + kTileK);
+#pragma unroll
+    for (int k = 0; k < kTileK; k += 4) {
+      float av[4][4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float4 a = *reinterpret_cast<const float4 *>(&As[buf][4 * ty + u][k]);
+        av[u][0] = a.x, av[u][1] = a.y, av[u][2] = a.z, av[u][3] = a.w;
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 b = *reinterpret_cast<const float4 *>(&Bs[buf][k + q][4 * tx]);
+        const float bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(av[u][q], bv[v], acc[u][v]);
+      }
+    }
+  }
+  auto put = [&](float *dst, const float (&x)[4]) {
+    if (vec) {
+      *reinterpret_cast<float4 *>(dst) = make_float4(x[0], x[1], x[2], x[3]);
+    } else {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (j + v < N) dst[v] = x[v];
+    }
+  };
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    if (i + u >= M) break;
+    if (bias) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (j + v < N) acc[u][v] += bias[j + v];
+    }
+    if (Z) put(Z + (long)(i + u) * ldc + j, acc[u]);
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      if (gelu) acc[u][v] = gelu_f(acc[u][v]);
+      if (Zg) acc[u][v] *= gelu_grad_f(zg[u][v]);
+    }
+    put(C + (long)(i + u) * ldc + j, acc[u]);
+  }
 }
 
 // Weight and bias gradients dW = dZ' A, db = colsum dZ of the three layers in one
@@ -225,13 +309,13 @@ __global__ void k_to_bf16(long n, const float *__restrict__ w, __nv_bfloat16 *__
     w16[e] = __float2bfloat16_rn(w[e]);
 }
 
-template <typename TB>
-void matmul(cudaStream_t s, int M, int N, int K, const float *A, long sai, long sak, const TB *B,
-            long sbk, long sbj, float *C, int ldc, const float *bias, float *Z, bool gelu,
+// B is N x K row-major if b_transposed, else K x N
+void matmul(cudaStream_t s, int M, int N, int K, const float *A, const __nv_bfloat16 *B,
+            bool b_transposed, float *C, int ldc, const float *bias, float *Z, bool gelu,
             const float *Zg = nullptr) {
-  const dim3 grid((N + kTile - 1) / kTile, (M + kTile - 1) / kTile);
-  k_matmul<TB><<<grid, 256, 0, s>>>(M, N, K, A, sai, sak, B, sbk, sbj, C, ldc, bias, Z,
-                                    gelu ? 1 : 0, Zg);
+  const dim3 grid((N + kTileN - 1) / kTileN, (M + kTileM - 1) / kTileM);
+  auto *f = b_transposed ? k_matmul<true> : k_matmul<false>;
+  f<<<grid, kMatThreads, 0, s>>>(M, N, K, A, B, C, ldc, bias, Z, gelu ? 1 : 0, Zg);
 }
 
 int grid_for(long n) {
@@ -258,13 +342,10 @@ MlpLayout mlp_layout(int F, int O) {
 
 void mlp_forward(cudaStream_t s, const MlpLayout &L, int B, const float *X, const float *w,
                  const __nv_bfloat16 *w16, MlpActs a) {
-  // Z1 = X W1' + b1, A1 = GELU(Z1): W1 is H x F row-major, B(k, j) = W1[j*F + k]
-  matmul<__nv_bfloat16>(s, B, L.H, L.F, X, L.F, 1, w16 + L.w1, 1, L.F, a.A1, L.H, w + L.b1, a.Z1,
-                        true);
-  matmul<__nv_bfloat16>(s, B, L.H, L.H, a.A1, L.H, 1, w16 + L.w2, 1, L.H, a.A2, L.H, w + L.b2,
-                        a.Z2, true);
-  matmul<__nv_bfloat16>(s, B, L.O, L.H, a.A2, L.H, 1, w16 + L.w3, 1, L.H, a.Out, L.O, w + L.b3,
-                        nullptr, false);
+  // Z1 = X W1' + b1, A1 = GELU(Z1): W1 is H x F row-major
+  matmul(s, B, L.H, L.F, X, w16 + L.w1, true, a.A1, L.H, w + L.b1, a.Z1, true);
+  matmul(s, B, L.H, L.H, a.A1, w16 + L.w2, true, a.A2, L.H, w + L.b2, a.Z2, true);
+  matmul(s, B, L.O, L.H, a.A2, w16 + L.w3, true, a.Out, L.O, w + L.b3, nullptr, false);
 }
 
 namespace {
@@ -287,10 +368,8 @@ void mlp_loss_backward(cudaStream_t s, const MlpLayout &L, int B, const float *X
   k_mse_sums<<<mse_blocks, kMseThreads, 0, s>>>(nO, a.Out, Y, mask, sums);
   k_mse_grad<<<mse_blocks, kMseThreads, 0, s>>>(nO, a.Out, Y, mask, sums, a.dOut, loss);
   // dZ2 = (dOut W3) GELU'(Z2), dZ1 = (dZ2 W2) GELU'(Z1)
-  matmul<__nv_bfloat16>(s, B, L.H, L.O, a.dOut, L.O, 1, w16 + L.w3, L.H, 1, a.dA, L.H, nullptr,
-                        nullptr, false, a.Z2);
-  matmul<__nv_bfloat16>(s, B, L.H, L.H, a.dA, L.H, 1, w16 + L.w2, L.H, 1, a.dA2, L.H, nullptr,
-                        nullptr, false, a.Z1);
+  matmul(s, B, L.H, L.O, a.dOut, w16 + L.w3, false, a.dA, L.H, nullptr, nullptr, false, a.Z2);
+  matmul(s, B, L.H, L.H, a.dA, w16 + L.w2, false, a.dA2, L.H, nullptr, nullptr, false, a.Z1);
   // dW3 = dOut' A2, dW2 = dZ2' A1, dW1 = dZ1' X and the bias gradients
   GradLayers g{};
   auto layer = [&](int q, const float *dZ, const float *A, int M, int N, long w, long b) {
