@@ -109,45 +109,64 @@ __global__ void k_prior(int m, int P, const unsigned *__restrict__ p,
 // Upper Cholesky factor with the reference's update order
 // (kernel_functions.cuh:845-902), warp per series.  Each element receives the
 // same sequence of floating-point operations as the reference's one-thread
-// loop, so the factor is bit-identical to it.
+// loop, so the factor is bit-identical to it.  Bound by its chain: per column a square
+// root and a reciprocal on the FP64 pipe (about 14 of its 64-cycle slots), then the
+// update, whose elements (k, l > k) are enumerated column by column, so that the first
+// rem (rem - 1) / 2 entries of one table serve every step: no index division, no lane on
+// an element of the lower triangle.  m = 400, max_p = 20: 31.6 us with the square
+// rem x rem enumerated by divisions, 24.2 us so; m = 133, max_p = 11: 17, 14.3 us.
+__device__ __forceinline__ int chol_stride(int P) { return P | 1; }  // (odd: distinct banks)
 __global__ void k_cholesky(int m, int P, const unsigned *__restrict__ p,
                            const double *__restrict__ C, double *__restrict__ U64,
                            float *__restrict__ U32) {
   extern __shared__ double sh[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int S = chol_stride(P);
+  // tri[q] = (k, l), k < l: 8 bits each
+  unsigned short *tri = reinterpret_cast<unsigned short *>(sh + (size_t)(blockDim.x >> 5) * P * S);
+  for (int l = threadIdx.x; l < P; l += blockDim.x)
+    for (int k = 0; k < l; ++k) tri[l * (l - 1) / 2 + k] = (unsigned short)(k | l << 8);
+  __syncthreads();
   const int j = blockIdx.x * (blockDim.x >> 5) + warp;
   if (j >= m) return;
-  double *a = sh + (size_t)warp * P * P;  // a[row + P*col]
+  double *a = sh + (size_t)warp * P * S;  // a[row + S*col]
   const double *Cj = C + (size_t)j * P * P;
   const int pj = (int)min((unsigned)P, p[j]);
-  for (int ix = lane; ix < P * P; ix += 32) {
-    const int r = ix % P, c = ix / P;
-    a[ix] = (r < pj && c < pj && c >= r) ? Cj[ix] : 0.0;
-  }
+  for (int r = lane; r < P; r += 32)
+#pragma unroll 4
+    for (int c = 0; c < P; ++c) a[r + S * c] = (c < pj && c >= r) ? Cj[r + P * c] : 0.0;
   __syncwarp();
   for (int n = 0; n < pj; ++n) {
-    const double d = sqrt(a[n + P * n]);
+    const double d = sqrt(a[n + S * n]);
     const double inv = 1.0 / d;
     __syncwarp();
-    if (lane == 0) a[n + P * n] = d;
+    if (lane == 0) a[n + S * n] = d;
     for (int k = n + 1 + lane; k < pj; k += 32) {
-      const double v = a[n + P * k] * inv;
-      a[n + P * k] = v;
-      a[k + P * k] -= v * v;
+      const double v = a[n + S * k] * inv;
+      a[n + S * k] = v;
+      a[k + S * k] -= v * v;
     }
     __syncwarp();
-    const int rem = pj - n - 1;
-    for (int q = lane; q < rem * rem; q += 32) {
-      const int k = n + 1 + q % rem, l = n + 1 + q / rem;
-      if (l > k) a[k + P * l] -= a[n + P * k] * a[n + P * l];
+    const int rem = pj - n - 1, cnt = rem * (rem - 1) / 2;
+    double *b = a + (n + 1) * (S + 1);  // the trailing matrix
+    const double *row = a + n + S * (n + 1);
+    for (int q = lane; q < cnt; q += 64) {
+      const int t0 = tri[q], t1 = tri[min(q + 32, cnt - 1)];
+      const int k0 = t0 & 255, l0 = t0 >> 8, k1 = t1 & 255, l1 = t1 >> 8;
+      double v0 = b[k0 + S * l0], v1 = b[k1 + S * l1];
+      v0 -= row[S * k0] * row[S * l0];
+      v1 -= row[S * k1] * row[S * l1];
+      b[k0 + S * l0] = v0;
+      if (q + 32 < cnt) b[k1 + S * l1] = v1;
     }
     __syncwarp();
   }
-  for (int ix = lane; ix < P * P; ix += 32) {
-    const double v = a[ix];
-    U64[(size_t)j * P * P + ix] = v;
-    if (U32) U32[(size_t)j * P * P + ix] = (float)v;
-  }
+  for (int r = lane; r < P; r += 32)
+    for (int c = 0; c < P; ++c) {
+      const double v = a[r + S * c];
+      U64[(size_t)j * P * P + r + (size_t)P * c] = v;
+      if (U32) U32[(size_t)j * P * P + r + (size_t)P * c] = (float)v;
+    }
 }
 
 __global__ void k_gate(int m, int P, const double *__restrict__ stats, double threshold,
@@ -255,10 +274,12 @@ void launch_to_float(cudaStream_t s, size_t n, const double *src, float *dst) {
 
 void launch_cholesky(cudaStream_t s, int m, int P, const unsigned *p, const double *C,
                      double *U64, float *U32) {
-  // one P x P FP64 slice per warp; keep the block under the default 48 KB
-  const size_t per_warp = (size_t)P * P * sizeof(double);
-  const int warps = (int)std::max<size_t>(1, std::min<size_t>(4, (48 * 1024) / per_warp));
-  const size_t smem = (size_t)warps * per_warp;
+  // one P x P FP64 slice per warp (its columns an odd number of values apart) and the
+  // triangle's table; keep the block under the default 48 KB
+  const size_t per_warp = (size_t)P * (P | 1) * sizeof(double);
+  const size_t table = ((size_t)P * (P - 1) / 2 + 1) * sizeof(unsigned short);
+  const int warps = (int)std::max<size_t>(1, std::min<size_t>(4, (48 * 1024 - table) / per_warp));
+  const size_t smem = (size_t)warps * per_warp + table;
   k_cholesky<<<(m + warps - 1) / warps, warps * 32, smem, s>>>(m, P, p, C, U64, U32);
 }
 
