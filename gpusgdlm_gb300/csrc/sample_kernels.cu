@@ -158,7 +158,10 @@ __global__ void __launch_bounds__(kSampleThreads)
       if (4 * q < pj) {
         const U4 r = philox((uint32_t)i, (uint32_t)j, tag_sub(TAG_THETA, q), ep, key.k0, key.k1);
         box_muller<T>(r.x, r.y, z[4 * q], z[4 * q + 1], key.tab);
-        box_muller<T>(r.z, r.w, z[4 * q + 2], z[4 * q + 3], key.tab);
+        if (4 * q + 2 < pj)
+          box_muller<T>(r.z, r.w, z[4 * q + 2], z[4 * q + 3], key.tab);
+        else
+          z[4 * q + 2] = z[4 * q + 3] = T(0);
       } else {
         z[4 * q] = z[4 * q + 1] = z[4 * q + 2] = z[4 * q + 3] = T(0);
       }
@@ -280,7 +283,10 @@ __global__ void __launch_bounds__(kSampleThreads)
       if (4 * q < na) {
         const U4 r = philox((uint32_t)i, (uint32_t)j, tag_sub(TAG_OMEGA, q), ep, key.k0, key.k1);
         box_muller<T>(r.x, r.y, w[4 * q], w[4 * q + 1], key.tab);
-        box_muller<T>(r.z, r.w, w[4 * q + 2], w[4 * q + 3], key.tab);
+        if (4 * q + 2 < na)
+          box_muller<T>(r.z, r.w, w[4 * q + 2], w[4 * q + 3], key.tab);
+        else
+          w[4 * q + 2] = w[4 * q + 3] = T(0);
       } else {
         w[4 * q] = w[4 * q + 1] = w[4 * q + 2] = w[4 * q + 3] = T(0);
       }
