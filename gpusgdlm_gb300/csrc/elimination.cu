@@ -243,29 +243,29 @@ LevelStreamHost level_stream(const EliminationPlanHost &pl, int lanes) {
     st.n_first.push_back(first);
     // the level's entries, by decreasing term count: entry e on thread e % lanes, pass
     // after pass over those that have a k-th term
-    std::vector<unsigned> ent;
-    std::vector<std::vector<unsigned>> terms;
+    std::vector<unsigned> ent, terms;  // entry e's terms: first_term[e] .. first_term[e + 1]
+    std::vector<int> first_term;
     for (int ch = pl.lev_chunk[l]; ch < pl.lev_chunk[l + 1]; ++ch)
       for (int lane = 0; lane < 32; ++lane) {
         const unsigned e = pl.ent[(size_t)ch * 32 + lane];
         if ((e & 0xFFFFu) == kSlotNone) continue;
-        std::vector<unsigned> t;
-        for (int k = pl.chunk_tofs[ch]; k < pl.chunk_tofs[ch + 1]; k += 32)
-          if (pl.terms[k + lane] != pack16(kSlotZero, kSlotZero)) t.push_back(pl.terms[k + lane]);
         ent.push_back(e);
-        terms.push_back(std::move(t));
+        first_term.push_back((int)terms.size());
+        for (int k = pl.chunk_tofs[ch]; k < pl.chunk_tofs[ch + 1]; k += 32)
+          if (pl.terms[k + lane] != pack16(kSlotZero, kSlotZero)) terms.push_back(pl.terms[k + lane]);
       }
+    first_term.push_back((int)terms.size());
     int second = 0;
     for (size_t k = 0;; ++k) {
       size_t n = 0;
-      while (n < ent.size() && terms[n].size() > k) ++n;  // (decreasing term counts)
+      while (n < ent.size() && (size_t)(first_term[n + 1] - first_term[n]) > k) ++n;  // (decreasing term counts)
       if (n == 0) break;
       const int rows = (int)((n + lanes - 1) / lanes);
       const size_t a = add_rows(rows);
       for (size_t e = 0; e < n; ++e) {
         const unsigned out = ent[e] & 0xFFFFu;
         st.rows[a + 2 * e] = k == 0 ? ent[e] : pack16(out, out);
-        st.rows[a + 2 * e + 1] = terms[e][k];
+        st.rows[a + 2 * e + 1] = terms[first_term[e] + k];
       }
       second += rows;
     }

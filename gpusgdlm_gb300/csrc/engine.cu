@@ -413,15 +413,17 @@ int upload_elimination(sgdlm_engine *h) {
   put(pl.bwd.data(), pl.bwd.size());
   put(pl.core_node.data(), pl.core_node.size());
   put(pl.core_map.data(), (pl.core_map.size() + 1) / 2);  // two 16-bit slots per int
-  const LevelStreamHost small = level_stream(pl, 128), large = level_stream(pl, 256);
-  put(small.rows.data(), small.rows.size());
+  const LevelStreamHost large = level_stream(pl, 256);
+  LevelStreamHost small;  // for cores of k_lu_small only
   std::vector<uint16_t> cells;
   if (pl.nlev > 0 && pl.dp <= 128) {
+    small = level_stream(pl, 128);
     cells.assign((size_t)128 * pl.dp, (uint16_t)kSlotZero);
     for (int c = 0; c < pl.dp; ++c)
       for (int r = 0; r < pl.dp; ++r)
         cells[((size_t)(c / 4) * 128 + r) * 4 + c % 4] = pl.core_map[(size_t)r + (size_t)pl.dp * c];
   }
+  put(small.rows.data(), small.rows.size());
   put(cells.data(), cells.size() / 2);
   put(large.rows.data(), large.rows.size());
   while (buf.size() % 4) buf.push_back(0);
@@ -467,7 +469,7 @@ int upload_elimination(sgdlm_engine *h) {
   ++k;
   auto set_stream = [&](LevelStream &st, const LevelStreamHost &sh, size_t at) {
     st.rows = reinterpret_cast<const uint2 *>(b + offs[at]);
-    for (int l = 0; l < pl.nlev; ++l) {
+    for (int l = 0; l < pl.nlev && !sh.n_first.empty(); ++l) {
       st.n_first[l] = (unsigned short)sh.n_first[l];
       st.n_second[l] = (unsigned short)sh.n_second[l];
       st.n_piv[l] = (unsigned short)(pl.lev_piv[l + 1] - pl.lev_piv[l]);

@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kSampleThreads)
 // The series' inactive coefficients (k >= p_j: U_W is zero outside its leading block, their
 // omega is cut) take no normals, quotients or products; the rows of theta are on their way
 // (cp.async) while the gammas are drawn.  m = 400, P = 20 (11.9 active on average), 10 000
-// draws, FP32: 752 us with all of it over P coefficients, 522 us so.
+// draws, FP32: 752 us with all of it over P coefficients, 500 us so.
 template <typename T, int PMAX, bool VEC>
 __global__ void __launch_bounds__(kSampleThreads)
     k_evolve(int m, int P, long n, const unsigned *__restrict__ p,
