@@ -425,15 +425,17 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
 
 // ELL widths: the smallest of these that holds the longest row
 constexpr int kJacWidths[] = {8, 12, 16, 18, 20, 24, 32};
-// and the widest of those whose FP32 kernels fit 72 registers with few spills
-constexpr int kJacPairWidth = 20;
+// and the widest rows of that form: FP32 kernels fit 72 registers with few spills up to 20;
+// FP64 ones gain up to 12 (m = 100: 231 us, 209 so) and lose beyond (m = 400, 18: 1505, 1525)
+constexpr int kJacPairWidth = 20, kJacPairWidth64 = 12;
 
 // Calls f with the kernel of type T, width K and draws per block (group: two).
 template <typename T, typename F> void with_jacobi_kernel(int K, bool group, int threads, F f) {
+  constexpr int pair_width = sizeof(T) == 4 ? kJacPairWidth : kJacPairWidth64;
 #define SGDLM_JACOBI(KK)                                                           \
   case KK:                                                                         \
-    if (group && threads <= kJacPairThreads && sizeof(T) == 4 && KK <= kJacPairWidth) \
-      f(k_forecast_jacobi<T, KK, 2, (sizeof(T) > 4 || KK > kJacPairWidth)>, 2);    \
+    if (group && threads <= kJacPairThreads && KK <= pair_width)                    \
+      f(k_forecast_jacobi<T, KK, 2, (KK > pair_width)>, 2);                        \
     else if (group)                                                                \
       f(k_forecast_jacobi<T, KK, 2, true>, 2);                                     \
     else                                                                           \
