@@ -825,14 +825,17 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
       launch_logdet64(h->stream, h->deep_launch, n, h->deep_dev, as<T>(h->theta_g),
                       as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, pivot_list, next);
   }
-  if (!deep) launch_lu<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
-               as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x, as<T>(h->lambda), key,
-               refine, y, rows, x ? h->nu_fc.ptr : nullptr, pivot_list,
-               iterative ? h->jac_list.ptr : nullptr);
+  int lu_launches = 1;
+  if (!deep)
+    lu_launches = launch_lu<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
+                               as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr,
+                               h->draw_flags.ptr, x, as<T>(h->lambda), key, refine, y, rows,
+                               x ? h->nu_fc.ptr : nullptr, pivot_list,
+                               iterative ? h->jac_list.ptr : nullptr);
   launch_lu_fallback<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
                         as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x,
                         as<T>(h->lambda), key, y, rows, pivot_list);
-  h->launches += 2;
+  h->launches += 1 + lu_launches;
   return SGDLM_OK;
 }
 

@@ -105,6 +105,9 @@ struct LuPlan {
   int tc;              // trailing updates on the tensor cores (tcgen05)
   int small_grid;      // > 0: log|det| by k_lu_small on so many blocks ...
   size_t small_smem;   // ... with this much shared memory each
+  int tail_draws;      // > 0: log|det| by k_lu up to the core's last 128 rows, these by
+  int tail_grid;       // k_lu_small on so many blocks, tail_draws draws at a time through
+  size_t tail_offset;  // slabs from this element of the scratch on
   size_t scratch_elems_per_cta;  // dense core + per-draw values of the sparse levels
   size_t fb_elems_per_cta;       // the redo's: the above, or a full m_p x m_p slab
   int fb_core_smem;              // the redo factors the dense core in shared memory
@@ -146,8 +149,9 @@ void launch_lu_warp(cudaStream_t s, int m, long n, int num_sms, GammaRows rows, 
 struct EliminationPlan;
 template <typename T>
 // theta: the draws series-major; theta_g: their Gamma entries (GammaDraws layout,
-// ep.nnz0 per draw), or nullptr (then gathered from theta).
-void launch_lu(cudaStream_t s, const LuPlan &plan, long n, const EliminationPlan &ep,
+// ep.nnz0 per draw), or nullptr (then gathered from theta).  Returns the number of kernels
+// launched.
+int launch_lu(cudaStream_t s, const LuPlan &plan, long n, const EliminationPlan &ep,
                const unsigned *sp, const T *theta, const T *theta_g, T *scratch,
                double *logdet, int *draw_flags,
                // forecast solve (x == nullptr: log|det| only)

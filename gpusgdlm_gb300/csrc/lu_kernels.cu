@@ -868,7 +868,8 @@ __device__ __forceinline__ void tc_preload_tile0(const float *A, int dp, int r0,
 // r0 .. r0 + 31 of the updated matrix) into dnext (shared, row-major, stride
 // kDs) instead of storing it and returns, so that the next panel's Gauss-Jordan
 // overlaps the rest of this update and the other warps' splits and preload of the
-// next panel; warps 1..7 meet on a named barrier at the end.
+// next panel; warps 1..7 meet on a named barrier at the end.  hand_over: the updated
+// matrix goes there (R x R) instead of back to E, no panel of this block follows.
 // Two tiles (R > 128): the product of each tile goes to columns 0 .. R-1 and E
 // comes from global memory (tmem_add_e); warp 4 would carry lanes 0..31 alone
 // through both tiles, so lanes 0..31 are split in halves as the other quarters,
@@ -877,7 +878,8 @@ __device__ __forceinline__ void tc_preload_tile0(const float *A, int dp, int r0,
 __device__ void tc_trailing_update(float *__restrict__ A, int dp, int r0, int R,
                                    const unsigned char *Lt, const unsigned char *Ut,
                                    size_t part_L, size_t part_U, uint32_t tmem, MmaSync *mbar,
-                                   uint32_t &mphase, bool &bad, float *dnext) {
+                                   uint32_t &mphase, bool &bad, float *dnext,
+                                   float *hand_over = nullptr) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int quarter = warp & 3;
   const bool two = R > 128;
@@ -914,11 +916,12 @@ __device__ void tc_trailing_update(float *__restrict__ A, int dp, int r0, int R,
       asm volatile("tcgen05.fence::before_thread_sync;");
       // warp 4 may overwrite lanes 0..31 now, in the next panel's preload (there
       // is one when R > 32)
-      if (R > kB) named_arrive_n(kBarQuarter0, 64);
+      if (R > kB && !hand_over) named_arrive_n(kBarQuarter0, 64);
       __syncwarp();
       return;
     }
-    if (quarter * 32 < R) tmem_sum_to_e(E, dp, R, row, cb, ce, tlane);
+    if (quarter * 32 < R)
+      tmem_sum_to_e(hand_over ? hand_over : E, hand_over ? R : dp, R, row, cb, ce, tlane);
     asm volatile("tcgen05.fence::before_thread_sync;");
     named_sync_n(kBarRest, kThreads - 32);
     asm volatile("tcgen05.fence::after_thread_sync;");
@@ -1823,9 +1826,21 @@ __device__ __forceinline__ void block_multipliers_rest(T *Lp, const T *D, int Rg
   __syncthreads();
 }
 
+// What k_lu<float, true, true> leaves of a draw to k_lu_small<true>: the last 128 x 128 of
+// the core after the panels before (column-major), then whether a check failed.
+constexpr int kSmallMaxDp = 128;
+constexpr size_t kTailElems = (size_t)kSmallMaxDp * kSmallMaxDp + 32;
+// ... for so many draws at a time: 1 GiB, one part up to 16 384 draws
+constexpr long kTailDraws = 16384;
+
 // TC: trailing updates on the tensor cores (FP32 draws, d_p <= 224); a separate
 // instantiation, so that the FFMA path's register tiles do not weigh on it.
-template <typename T, bool TC>
+// Front: log|det| of the draws first .. first + count - 1 only, and only the panels before
+// the core's last 128 rows, which k_lu_small<true> finishes: there a draw needs 128
+// threads, and four draws' chains of pivot blocks run on an SM instead of two.  10 000
+// draws at m = 400 (core of 215): 3.62 ms by one kernel, 2.84 + 0.52 ms so; the 64 KB per
+// draw in between, 0.2 ms of memory traffic, go on beside the chains.
+template <typename T, bool TC, bool Front = false>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     k_lu(int m, int P, int dp, size_t per_cta, int vals_smem, int prog_smem, long n,
          EliminationPlan ep,
@@ -1834,8 +1849,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
          double *__restrict__ logdet, int *__restrict__ draw_flags,
          const double *__restrict__ x, const T *__restrict__ lambda, RngKey key, bool refine,
          double *__restrict__ y, GammaRows rows, const double *__restrict__ nu_in,
-         int *__restrict__ pivot_list, const int *__restrict__ draw_list) {
+         int *__restrict__ pivot_list, const int *__restrict__ draw_list,
+         float *__restrict__ tail = nullptr, long first = 0, long count = 0) {
   static_assert(!TC || sizeof(T) == 4, "tensor-core path: FP32 draws");
+  static_assert(TC || !Front, "");
   using V = Vec<T>;
   constexpr int W = V::W;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1860,7 +1877,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
   const bool planned = (ep.core_map != nullptr);
   T *vals = vals_smem ? reinterpret_cast<T *>(smem_raw + L.off_vals) : vals_g;
   const int nbk = dp / kB;
-  const bool solve = (x != nullptr);
+  const bool solve = Front ? false : (x != nullptr);
   const T tau = (T)kPivotThreshold;
   __shared__ int sflag;
   // tensor-core trailing updates (FP32 draws, d_p <= 224): 256 columns of tensor
@@ -1884,9 +1901,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
   }
   const uint32_t tmem = TC ? s_tmem : 0u;
 
-  const long n_todo = draw_list ? min((long)draw_list[0], n) : n;
+  const long n_todo = Front ? count : (draw_list ? min((long)draw_list[0], n) : n);
   for (long it = blockIdx.x; it < n_todo; it += gridDim.x) {
-    const long i = draw_list ? (long)draw_list[1 + it] : it;
+    const long i = Front ? first + it : (draw_list ? (long)draw_list[1 + it] : it);
     if (tid == 0) sflag = 0;
     bool bad = false;
     double ld_part = 0.0;  // this thread's share of sum log|pivot| (levels and core)
@@ -2048,7 +2065,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
         // other warps' splits of the next panel.
         unsigned char *Lt = smem_raw + L.off_Lt, *Ut = smem_raw + L.off_Ut;
         unsigned char *Dt = smem_raw + L.off_Dt;
-        for (int kb = 0; kb < nbk; ++kb) {
+        const int nb_here = Front ? nbk - kSmallMaxDp / kB : nbk;
+        for (int kb = 0; kb < nb_here; ++kb) {
           const int k0 = kb * kB, r0 = k0 + kB, R = dp - r0;
           if (warp == 0) {
             // the rows of D (the first panel's from the core, later ones as the
@@ -2120,10 +2138,16 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
             tc_block_multipliers(reinterpret_cast<float *>(A), dp, k0, r0, R, Lt, L.part_L, Dt, tmem,
                                  &s_mbar, mphase, tau, reinterpret_cast<float *>(z), solve, bad);
             tc_trailing_update(reinterpret_cast<float *>(A), dp, r0, R, Lt, Ut, L.part_L,
-                               L.part_U, tmem, &s_mbar, mphase, bad, reinterpret_cast<float *>(D));
+                               L.part_U, tmem, &s_mbar, mphase, bad, reinterpret_cast<float *>(D),
+                               Front && kb + 1 == nb_here ? tail + (size_t)it * kTailElems : nullptr);
           } else {
             __syncthreads();
           }
+        }
+        if (Front && warp == 0) {  // the diagonal block that the last update left in D
+          float *dst = tail + (size_t)it * kTailElems + lane;
+#pragma unroll 8
+          for (int q = 0; q < kB; ++q) dst[(size_t)kSmallMaxDp * q] = (float)D[lane * kDs + q];
         }
       }
     }
@@ -2193,7 +2217,12 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     for (int q = tid; q < n_logs; q += kThreads) ld_part += (double)reinterpret_cast<float *>(nu)[q];
     const double ld_total = block_sum_det(ld_part, red);  // contains __syncthreads
     const bool flagged = (sflag != 0);
-    if (tid == 0) {
+    if constexpr (Front) {
+      if (tid == 0) {
+        logdet[i] = ld_total;
+        tail[(size_t)it * kTailElems + kSmallMaxDp * kSmallMaxDp] = flagged ? 1.f : 0.f;
+      }
+    } else if (tid == 0) {
       logdet[i] = ld_total;
       if (flagged) {
         atomicOr(&draw_flags[i], DRAW_FLAG_PIVOT);
@@ -2203,7 +2232,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
         }
       }
     }
-    if (solve && !flagged) {
+    if (!Front && solve && !flagged) {
       EliminationPlan eps = ep;  // the solve programs, staged in shared memory when they fit
       if (planned && vals_smem) {
         copy_vals<T>(vals, vals_g, ep.n_solve);
@@ -2283,6 +2312,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
       }
     }
     __syncthreads();
+    // (the next draw's first panel may write tensor memory that this one's last has read)
+    if constexpr (Front) asm volatile("tcgen05.fence::after_thread_sync;");
   }
   if constexpr (TC) {
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;" ::"r"(tmem));
@@ -2426,7 +2457,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // 10 000 draws, us (k_lu; with the chunks' program of the levels; now): m = 100 (core 33)
 // 725, 325, 230; m = 133 (45) 765, 358, 258; m = 200 (87) 1161, 595, 489; m = 250 (128)
 // 1545, -, 855.
-constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32, kSmallMaxDp = 128;
+constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32;
 constexpr int kSmallTmem = 128, kSmallTmemU = 64, kSmallTmemL = 96;
 constexpr int kBs = kB + 1;  // stride of the staged columns of B
 struct SmallSmem {
@@ -2468,12 +2499,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
       "r"(__float_as_uint(v[15])));
 }
 
+// Tail: of the draws first .. first + count - 1, whose larger core's panels before the last
+// 128 rows are done (k_lu<float, true, true>): dp = 128, core_n counts the rows of these.
+template <bool Tail>
 __global__ void __launch_bounds__(kSmallThreads, 4)
     k_lu_small(int m, int P, int dp, long n, EliminationPlan ep, const float *__restrict__ theta_g,
                double *__restrict__ logdet, int *__restrict__ draw_flags,
-               int *__restrict__ pivot_list) {
+               int *__restrict__ pivot_list, int core_n, const float *__restrict__ tail, long first,
+               long count) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  const SmallSmem S(ep.nv, m);
+  const SmallSmem S(Tail ? 0 : ep.nv, Tail ? 0 : m);
   float *Bs = reinterpret_cast<float *>(smem_raw + S.off_B);
   unsigned char *Dt = smem_raw + S.off_B;
   float *D = reinterpret_cast<float *>(smem_raw + S.off_D);
@@ -2525,31 +2560,40 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
   };
-  for (long i = blockIdx.x; i < n; i += gridDim.x) {
-    if (tid == 0) sflag = 0;
+  for (long it = blockIdx.x; it < (Tail ? count : n); it += gridDim.x) {
+    const long i = Tail ? first + it : it;
+    const float *rest = tail + (size_t)it * kTailElems;
+    if (tid == 0) sflag = Tail ? (int)rest[kSmallMaxDp * kSmallMaxDp] : 0;
     bool bad = false;
-    build_slots<float, kSmallThreads>(ep, m, i, theta, vals);
-    __syncthreads();
-    const int n_logs = run_stream<kSmallThreads>(ep.small_stream, ep.nlev, vals, tau, bad, logs);
+    int n_logs = 0;
+    if constexpr (!Tail) {
+      build_slots<float, kSmallThreads>(ep, m, i, theta, vals);
+      __syncthreads();
+      n_logs = run_stream<kSmallThreads>(ep.small_stream, ep.nlev, vals, tau, bad, logs);
+    }
     // ---- the core's rows: 32 columns in registers, the rest in tensor memory (or, of
     // the first panel's rows, staged as B)
     float a[kB];
-    if (warp < nbk) {
-      const uint2 *cells = ep.small_map + row;
+    auto cells_of = [&](int c0, float *e) {  // row's columns c0 .. c0 + 15
+      if constexpr (Tail) {
 #pragma unroll
-      for (int q = 0; q < kB; q += 4) {
-        const uint2 w = __ldg(cells + (q / 4) * kSmallThreads);
-        a[q] = vals[lo16(w.x)], a[q + 1] = vals[hi16(w.x)];
-        a[q + 2] = vals[lo16(w.y)], a[q + 3] = vals[hi16(w.y)];
-      }
-      for (int c0 = kB; c0 < dp; c0 += 16) {
-        float e[16];
+        for (int q = 0; q < 16; ++q) e[q] = rest[row + (size_t)kSmallMaxDp * (c0 + q)];
+      } else {
+        const uint2 *cells = ep.small_map + row;
 #pragma unroll
         for (int q = 0; q < 16; q += 4) {
           const uint2 w = __ldg(cells + ((c0 + q) / 4) * kSmallThreads);
           e[q] = vals[lo16(w.x)], e[q + 1] = vals[hi16(w.x)];
           e[q + 2] = vals[lo16(w.y)], e[q + 3] = vals[hi16(w.y)];
         }
+      }
+    };
+    if (warp < nbk) {
+      cells_of(0, a);
+      cells_of(16, a + 16);
+      for (int c0 = kB; c0 < dp; c0 += 16) {
+        float e[16];
+        cells_of(c0, e);
         if (warp == 0) {
 #pragma unroll
           for (int q = 0; q < 16; ++q) Bs[(c0 - kB + q) * kBs + lane] = e[q];
@@ -2559,13 +2603,22 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
       }
       asm volatile("tcgen05.wait::st.sync.aligned;");
     }
+    if constexpr (Tail) {
+      // this block's next 64 KB on their way to L2
+      if (it + gridDim.x < count) {
+        const float *ahead = tail + (size_t)(it + gridDim.x) * kTailElems + 32 * tid;
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(ahead + 32 * kSmallThreads * h));
+      }
+    }
     __syncthreads();  // the slots are dead
     for (int kb = 0; kb < nbk; ++kb) {
       const int k0 = kb * kB, r0 = k0 + kB, R = dp - r0;
       const bool below = warp > kb && warp < nbk;
       if (warp == kb) {
         const double ld = gj_diag<float, false, true>(a, prow, tau, bad,
-                                                      R > 0 ? kB / 4 : last_super_steps(ep.core_n, k0));
+                                                      R > 0 ? kB / 4 : last_super_steps(core_n, k0));
         if (lane == 0) logs[n_logs + kb] = (float)ld;  // (an FP32 sum)
 #pragma unroll
         for (int q = 0; q < kB; q += 4) Vec<float>::st(D + lane * kDs + q, a + q);
@@ -2655,7 +2708,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
       for (int q = lane; q < n_logs + nbk; q += 32) ld += (double)logs[q];
       ld = warp_sum_d(ld);
       if (lane == 0) {
-        logdet[i] = ld;
+        logdet[i] = Tail ? logdet[i] + ld : ld;
         if (sflag != 0) {
           atomicOr(&draw_flags[i], DRAW_FLAG_PIVOT);
           const int q = atomicAdd(pivot_list, 1);
@@ -3195,13 +3248,32 @@ LuPlan plan_lu(int m, int P, long n, int num_sms, int core_n, int nv, int n_solv
     if (opt.max_grid > 0) pl.small_grid = std::min(pl.small_grid, opt.max_grid);
     pl.small_grid = (int)std::min<long>(pl.small_grid, n);
   }
+  // larger ones on the tensor cores: the last 128 rows by k_lu_small<true>, from slabs
+  // behind k_lu's (16 systems of m = 20 .. 400, 10 000 draws each, whole steps: 37.9 ms
+  // without, 33.7 ms with the split)
+  pl.tail_draws = 0;
+  if (pl.tc && pl.vals_smem && pl.dp > kSmallMaxDp) {
+    pl.small_smem = SmallSmem(0, 0).total;
+    pl.tail_grid = num_sms * 4;
+    if (opt.max_grid > 0) pl.tail_grid = std::min(pl.tail_grid, opt.max_grid);
+    pl.tail_draws = (int)std::min<long>(n, kTailDraws);
+  }
   long grid = (long)num_sms * ctas_per_sm;
   if (opt.max_grid > 0 && grid > opt.max_grid) grid = opt.max_grid;
   if (grid > n) grid = n;
   if (grid < 1) grid = 1;
   pl.grid = (int)grid;
   pl.scratch_elems_per_cta = (size_t)pl.dp * pl.dp + (((size_t)nv + 3) / 4) * 4;
-  const size_t total = pl.scratch_elems_per_cta * pl.grid;
+  size_t total = pl.scratch_elems_per_cta * pl.grid;
+  if (pl.tail_draws > 0) {
+    // (no fewer draws than one per resident block: with those the split gains nothing)
+    if (n > pl.grid) {
+      pl.tail_offset = (total + 31) / 32 * 32;
+      total = pl.tail_offset + (size_t)pl.tail_draws * kTailElems;
+    } else {
+      pl.tail_draws = 0;
+    }
+  }
   // the redo needs the dense core and the value slots, or a full m_p x m_p slab,
   // per CTA; it shares the slab array, which grows to one slab per SM for it
   const size_t full = std::max((size_t)pl.mp * pl.mp, pl.scratch_elems_per_cta);
@@ -3215,7 +3287,7 @@ LuPlan plan_lu(int m, int P, long n, int num_sms, int core_n, int nv, int n_solv
 }
 
 template <typename T>
-void launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &ep,
+int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &ep,
                const unsigned *sp, const T *theta, const T *theta_g, T *scratch,
                double *logdet, int *draw_flags,
                const double *x, const T *lambda, RngKey key, bool refine, double *y,
@@ -3229,21 +3301,43 @@ void launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &
                                               pl.vals_smem, pl.prog_smem, n, ep, sp, theta,
                                               theta_g, scratch,
                                               logdet, draw_flags, x, lambda, key, refine, y, rows,
-                                              nu_in, pivot_list, draw_list);
+                                              nu_in, pivot_list, draw_list, nullptr, 0, 0);
   };
   if constexpr (sizeof(T) == 4) {
     if (pl.small_grid > 0 && !x && !draw_list && theta_g && pivot_list) {
-      cudaFuncSetAttribute(k_lu_small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.small_smem);
-      k_lu_small<<<pl.small_grid, kSmallThreads, pl.small_smem, s>>>(pl.m, pl.P, pl.dp, n, ep, theta_g,
-                                                                     logdet, draw_flags, pivot_list);
-      return;
+      auto *f = k_lu_small<false>;
+      cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.small_smem);
+      f<<<pl.small_grid, kSmallThreads, pl.small_smem, s>>>(pl.m, pl.P, pl.dp, n, ep, theta_g, logdet,
+                                                            draw_flags, pivot_list, ep.core_n, nullptr, 0, 0);
+      return 1;
+    }
+    if (pl.tail_draws > 0 && n > pl.grid && !x && !draw_list && theta_g && pivot_list) {
+      auto *front = k_lu<T, true, true>;
+      auto *rest = k_lu_small<true>;
+      cudaFuncSetAttribute(front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
+      cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.small_smem);
+      float *tail = scratch + pl.tail_offset;
+      // equal parts of at most tail_draws
+      const long parts = (n + pl.tail_draws - 1) / pl.tail_draws, per = (n + parts - 1) / parts;
+      for (long first = 0; first < n; first += per) {
+        const long count = std::min(per, n - first);
+        front<<<(unsigned)std::min<long>(pl.grid, count), pl.block, pl.smem, s>>>(
+            pl.m, pl.P, pl.dp, pl.scratch_elems_per_cta, pl.vals_smem, pl.prog_smem, n, ep, sp, theta,
+            theta_g, scratch, logdet, draw_flags, nullptr, nullptr, key, false, nullptr, rows, nullptr,
+            nullptr, nullptr, tail, first, count);
+        rest<<<(unsigned)std::min<long>(pl.tail_grid, count), kSmallThreads, pl.small_smem, s>>>(
+            pl.m, pl.P, kSmallMaxDp, n, ep, theta_g, logdet, draw_flags, pivot_list,
+            ep.core_n - (pl.dp - kSmallMaxDp), tail, first, count);
+      }
+      return (int)(2 * parts);
     }
     if (pl.tc) {
       run(k_lu<T, true>);
-      return;
+      return 1;
     }
   }
   run(k_lu<T, false>);
+  return 1;
 }
 
 bool launch_lu_cluster(cudaStream_t s, const LuPlan &pl, long n, int slabs, int num_sms,
@@ -3314,12 +3408,12 @@ void launch_lu_fallback(cudaStream_t s, const LuPlan &pl, long n, const Eliminat
 
 template LuPlan plan_lu<float>(int, int, long, int, int, int, int, int, LuOptions);
 template LuPlan plan_lu<double>(int, int, long, int, int, int, int, int, LuOptions);
-template void launch_lu<float>(cudaStream_t, const LuPlan &, long, const EliminationPlan &,
+template int launch_lu<float>(cudaStream_t, const LuPlan &, long, const EliminationPlan &,
                                const unsigned *, const float *, const float *, float *,
                                double *, int *,
                                const double *, const float *, RngKey, bool, double *, GammaRows,
                                const double *, int *, const int *);
-template void launch_lu<double>(cudaStream_t, const LuPlan &, long, const EliminationPlan &,
+template int launch_lu<double>(cudaStream_t, const LuPlan &, long, const EliminationPlan &,
                                 const unsigned *, const double *, const double *, double *,
                                 double *, int *,
                                 const double *, const double *, RngKey, bool, double *,

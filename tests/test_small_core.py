@@ -78,3 +78,35 @@ def test_draws_that_need_pivoting(built_lib):
     # above one) leave about four digits
     np.testing.assert_allclose(d["log_dets"], ld, rtol=0, atol=5e-2)
     s.close()
+
+
+@pytest.mark.parametrize("m,kmax,n", [(275, 17, 305), (290, 17, 700), (345, 17, 400), (400, 17, 611)])
+def test_last_rows_by_the_small_kernel(built_lib, m, kmax, n):
+    """Cores of 160, 192 and 224 rows with more draws than the large kernel has blocks: it
+    leaves their last 128 rows to the small one."""
+    s, wl, par = _engine(m, kmax, 3 + m, min(0.3, 0.8 / kmax))
+    assert 128 < s.getEliminationInfo()["core_n"] <= 224
+    d, f, flags = _both(s, wl, par, n, 5)
+    assert flags == 0
+    np.testing.assert_allclose(d["log_dets"], f["log_dets"], rtol=0, atol=1e-12)
+    s.close()
+
+
+@pytest.mark.parametrize("m,spread", [(275, 1.0), (275, 3.0), (345, 3.0)])
+def test_last_rows_of_draws_that_need_pivoting(built_lib, m, spread):
+    """A check that fails before or in the last 128 rows sends the draw to the redo: the
+    first of many draws (two kernels) against the same draws alone (one kernel), whose
+    operations are the same up to the FP64 sum of the logarithms."""
+    s, wl, par = _engine(m, 17, 3 + m, spread)
+    got = []
+    for n in (200, 330):
+        s.setPosteriorParameters(*par)
+        s.setRngState(5, 0)
+        s.computeVBPosterior(n, n)
+        got.append((s.getStats()["draws_pivoted"], s.getDraws()))
+    (few_flags, few), (many_flags, many) = got
+    np.testing.assert_array_equal(few["thetas"], many["thetas"][..., :200])
+    np.testing.assert_allclose(few["log_dets"], many["log_dets"][:200], rtol=0, atol=1e-10)
+    assert few_flags <= many_flags <= few_flags + 130
+    assert spread < 3.0 or few_flags > 0
+    s.close()
