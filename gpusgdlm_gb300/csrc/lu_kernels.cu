@@ -1826,7 +1826,7 @@ __device__ __forceinline__ void block_multipliers_rest(T *Lp, const T *D, int Rg
   __syncthreads();
 }
 
-// What k_lu<float, true, true> leaves of a draw to k_lu_small<true>: the last 128 x 128 of
+// What k_lu<float, true, kFront> leaves of a draw to k_lu_small<true>: the last 128 x 128 of
 // the core after the panels before (column-major), then whether a check failed.
 constexpr int kSmallMaxDp = 128;
 constexpr size_t kTailElems = (size_t)kSmallMaxDp * kSmallMaxDp + 32;
@@ -1835,12 +1835,17 @@ constexpr long kTailDraws = 16384;
 
 // TC: trailing updates on the tensor cores (FP32 draws, d_p <= 224); a separate
 // instantiation, so that the FFMA path's register tiles do not weigh on it.
-// Front: log|det| of the draws first .. first + count - 1 only, and only the panels before
+// Mode kPlain: log|det| of whole matrices without a plan (the allocation-free entry point),
+// without the code of the levels and the solves, whose registers it would share (1 200
+// draws, m = 220: 1189 us in the general kernel, 1113 us so; m = 130: 366, 350).
+// Mode kFront: log|det| of the draws first .. first + count - 1 only, and only the panels before
 // the core's last 128 rows, which k_lu_small<true> finishes: there a draw needs 128
 // threads, and four draws' chains of pivot blocks run on an SM instead of two.  10 000
-// draws at m = 400 (core of 215): 3.62 ms by one kernel, 2.84 + 0.52 ms so; the 64 KB per
+// draws at m = 400 (core of 215): 3.62 ms by one kernel, 2.52 + 0.52 ms so (2.84 with the
+// general kernel's code for solves and unplanned matrices in it); the 64 KB per
 // draw in between, 0.2 ms of memory traffic, go on beside the chains.
-template <typename T, bool TC, bool Front = false>
+constexpr int kAny = 0, kFront = 1, kPlain = 2;
+template <typename T, bool TC, int Mode = kAny>
 __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     k_lu(int m, int P, int dp, size_t per_cta, int vals_smem, int prog_smem, long n,
          EliminationPlan ep,
@@ -1852,6 +1857,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
          int *__restrict__ pivot_list, const int *__restrict__ draw_list,
          float *__restrict__ tail = nullptr, long first = 0, long count = 0) {
   static_assert(!TC || sizeof(T) == 4, "tensor-core path: FP32 draws");
+  constexpr bool Front = Mode == kFront;
   static_assert(TC || !Front, "");
   using V = Vec<T>;
   constexpr int W = V::W;
@@ -1874,10 +1880,10 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   T *A = scratch + (size_t)blockIdx.x * per_cta;
   T *vals_g = A + (size_t)dp * dp;
-  const bool planned = (ep.core_map != nullptr);
-  T *vals = vals_smem ? reinterpret_cast<T *>(smem_raw + L.off_vals) : vals_g;
+  const bool planned = Mode == kPlain ? false : (Mode == kFront ? true : ep.core_map != nullptr);
+  T *vals = Mode == kFront || vals_smem ? reinterpret_cast<T *>(smem_raw + L.off_vals) : vals_g;
   const int nbk = dp / kB;
-  const bool solve = Front ? false : (x != nullptr);
+  const bool solve = Mode == kAny ? x != nullptr : false;
   const T tau = (T)kPivotThreshold;
   __shared__ int sflag;
   // tensor-core trailing updates (FP32 draws, d_p <= 224): 256 columns of tensor
@@ -1953,14 +1959,14 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
     int n_logs = 0;
     bool streamed = false;
     if constexpr (TC) {
-      if (planned && vals_smem && !solve) {
+      if (planned && (Front || vals_smem) && !solve) {
         // the pivots' logarithms take nu's place (no right-hand side here)
         n_logs = run_stream<kThreads>(ep.stream, ep.nlev, reinterpret_cast<float *>(vals), tau, bad,
                                       reinterpret_cast<float *>(nu));
         streamed = true;
       }
     }
-    for (int lev = streamed ? ep.nlev : 0; lev < ep.nlev; ++lev) {
+    for (int lev = Mode != kAny || streamed ? ep.nlev : 0; lev < ep.nlev; ++lev) {
       for (int q = ep.lev_piv[lev] + tid; q < ep.lev_piv[lev + 1]; q += blockDim.x) {
         const T pv = vals[ep.piv[q]];
         if (!(finite_t(pv) && pv != T(0))) bad = true;
@@ -2232,7 +2238,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
         }
       }
     }
-    if (!Front && solve && !flagged) {
+    if (Mode == kAny && solve && !flagged) {
       EliminationPlan eps = ep;  // the solve programs, staged in shared memory when they fit
       if (planned && vals_smem) {
         copy_vals<T>(vals, vals_g, ep.n_solve);
@@ -2500,7 +2506,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) 
 }
 
 // Tail: of the draws first .. first + count - 1, whose larger core's panels before the last
-// 128 rows are done (k_lu<float, true, true>): dp = 128, core_n counts the rows of these.
+// 128 rows are done (k_lu<float, true, kFront>): dp = 128, core_n counts the rows of these.
 template <bool Tail>
 __global__ void __launch_bounds__(kSmallThreads, 4)
     k_lu_small(int m, int P, int dp, long n, EliminationPlan ep, const float *__restrict__ theta_g,
@@ -3250,7 +3256,7 @@ LuPlan plan_lu(int m, int P, long n, int num_sms, int core_n, int nv, int n_solv
   }
   // larger ones on the tensor cores: the last 128 rows by k_lu_small<true>, from slabs
   // behind k_lu's (16 systems of m = 20 .. 400, 10 000 draws each, whole steps: 37.9 ms
-  // without, 33.7 ms with the split)
+  // without, 30.6 ms with the split)
   pl.tail_draws = 0;
   if (pl.tc && pl.vals_smem && pl.dp > kSmallMaxDp) {
     pl.small_smem = SmallSmem(0, 0).total;
@@ -3312,7 +3318,7 @@ int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &e
       return 1;
     }
     if (pl.tail_draws > 0 && n > pl.grid && !x && !draw_list && theta_g && pivot_list) {
-      auto *front = k_lu<T, true, true>;
+      auto *front = k_lu<T, true, kFront>;
       auto *rest = k_lu_small<true>;
       cudaFuncSetAttribute(front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
       cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.small_smem);
@@ -3332,7 +3338,10 @@ int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &e
       return (int)(2 * parts);
     }
     if (pl.tc) {
-      run(k_lu<T, true>);
+      if (!x && !ep.core_map)
+        run(k_lu<T, true, kPlain>);
+      else
+        run(k_lu<T, true>);
       return 1;
     }
   }
