@@ -119,7 +119,7 @@ struct LuPlan {
 struct LuOptions {
   int allow_tc = 1;
   int max_grid = 0;
-  int allow_warp = 1;  // m <= kWarpLuMaxM: one warp per draw (launch_lu_warp)
+  int allow_warp = 1;  // m <= kWarpLuMaxM: 4 to 32 lanes per draw (launch_lu_warp)
 };
 constexpr int kWarpLuMaxM = 32;
 // core_n / nv / n_solve / prog_len come from the elimination plan (core_n = m and

@@ -39,6 +39,10 @@
 //     levels' backward program (staged in shared memory).  The residual
 //     nu - (I - Gamma) y0 from the sparse parent rows (FP64, or double-float
 //     FP32 for FP32 draws) drives one refinement solve with the same factors.
+// log|det| alone of FP32 draws: cores of at most 128 rows, and the last 128 rows of those up
+// to 224, by k_lu_small (blocks of 128 threads, four draws per SM); unplanned matrices of
+// which the scratch holds few by k_lu_cluster.  FP64 draws: logdet64.cu, where its plan
+// fits, else the FFMA form here.
 #include <algorithm>
 
 #include <cuda_bf16.h>

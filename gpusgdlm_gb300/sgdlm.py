@@ -496,7 +496,7 @@ class SGDLM:
         self._check(self._lib.sgdlm_set_forecast_solver(self._h, 1 if iterative else 0))
 
     def setWarpLu(self, enable: bool = True):
-        """m <= 32: one warp per draw with partial pivoting (default), or the
+        """m <= 32: 4 to 32 lanes per draw with partial pivoting (default), or the
         block LU kernels (include/sgdlm.h, sgdlm_set_warp_lu)."""
         self._check(self._lib.sgdlm_set_warp_lu(self._h, 1 if enable else 0))
 

@@ -266,7 +266,7 @@ int sgdlm_set_lu_options(sgdlm_handle h, int allow_tensor_cores, int max_ctas);
  * factored.  Results equal to the refinement tolerance. */
 int sgdlm_set_forecast_solver(sgdlm_handle h, int iterative);
 int sgdlm_get_lu_options(sgdlm_handle h, int *allow_tensor_cores, int *max_ctas);
-/* Small systems (m <= 32): 1 (default) one warp per draw, each lane one row, LU
+/* Small systems (m <= 32): 1 (default) 4, 8, 16 or 32 lanes per draw, each one row, LU
  * with partial pivoting (no redo pass, forecasts of FP32 draws refined three times);
  * 0 the block LU kernels as for larger m.  in_use: whether this engine's m takes
  * the warp path. */
