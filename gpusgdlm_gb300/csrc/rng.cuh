@@ -100,7 +100,7 @@ template <> struct Uniform<float> {
 //     are exact).  Error below 0.8 ulp (log(): 0.54 ulp).
 //   sin, cos of 2 pi u: the nearest of 1024 angles plus a rest of at most pi / 1024.
 //     Absolute error below 1.12e-16 (sincospi(): 1.29e-16).
-// 10 000 draws: the sampler 1084 -> 609 us at m = 100, 5.88 -> 3.4 ms at m = 400 (576 us at
+// 10 000 draws: the sampler 1084 -> 609 us at m = 100, 5.88 -> 3.3 ms at m = 400 (576 us at
 // m = 100 since pairs of normals beyond p_j are left out).
 // The table (trig_log_table, engine.cu) is 25 KB and read through L1.
 //   [0, 2048): cos, sin of 2 pi i / 1024; [2048, 3072): inv, upper and lower part of
