@@ -694,7 +694,7 @@ int alloc_sim(sgdlm_engine *h, size_t nsim) {
   CK(h->y_fc.reserve(nsim * m));
   CK(h->nu_fc.reserve(nsim * m));
   CK(h->draw_flags.reserve(nsim));
-  CK(h->pivot_list.reserve(nsim + 2));
+  CK(h->pivot_list.reserve(nsim + 3));
   CK(h->jac_list.reserve(nsim + 1));
   CK(h->part_a.reserve((size_t)h->chunks * m * (P + 2) + m * P));
   CK(h->part_b.reserve((size_t)h->chunks * m * P * P));
@@ -814,8 +814,9 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
     h->launches += 1;
   }
   // the fast pass appends the draws it flags to pivot_list; the redo visits those
-  CK(cudaMemsetAsync(h->pivot_list.ptr, 0, 2 * sizeof(int), h->stream));
-  int *next = h->pivot_list.ptr, *pivot_list = next + 1;
+  // (behind two work counters)
+  CK(cudaMemsetAsync(h->pivot_list.ptr, 0, 3 * sizeof(int), h->stream));
+  int *next = h->pivot_list.ptr, *pivot_list = next + 2;
   bool deep = false;
   if constexpr (std::is_same<T, double>::value) {
     // log|det| of FP64 draws: the deep elimination where there is one (2 to 30 times
@@ -831,7 +832,7 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
                                as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr,
                                h->draw_flags.ptr, x, as<T>(h->lambda), key, refine, y, rows,
                                x ? h->nu_fc.ptr : nullptr, pivot_list,
-                               iterative ? h->jac_list.ptr : nullptr);
+                               iterative ? h->jac_list.ptr : nullptr, next);
   launch_lu_fallback<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
                         as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x,
                         as<T>(h->lambda), key, y, rows, pivot_list);

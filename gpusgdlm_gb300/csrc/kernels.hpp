@@ -164,7 +164,9 @@ int launch_lu(cudaStream_t s, const LuPlan &plan, long n, const EliminationPlan 
                // are appended ([0] their count, [1..] their indices), or nullptr
                int *pivot_list = nullptr,
                // the same form: only the listed draws are factored, or nullptr: all
-               const int *draw_list = nullptr);
+               const int *draw_list = nullptr,
+               // two ints, zero on entry: the blocks' work counters, or nullptr
+               int *next = nullptr);
 // log|det| of unplanned FP32 draws (levels off, d_p above the tensor-core path's) by a
 // cluster of blocks per draw, where scratch holds only `slabs` matrices (d_p x d_p).
 // false: not launched (sizes for which launch_lu is the better choice, or no cluster fits).

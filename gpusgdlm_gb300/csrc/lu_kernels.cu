@@ -1844,7 +1844,10 @@ constexpr long kTailDraws = 16384;
 // draws, m = 220: 1189 us in the general kernel, 1113 us so; m = 130: 366, 350).
 // Mode kFront: log|det| of the draws first .. first + count - 1 only, and only the panels before
 // the core's last 128 rows, which k_lu_small<true> finishes: there a draw needs 128
-// threads, and four draws' chains of pivot blocks run on an SM instead of two.  10 000
+// threads, and four draws' chains of pivot blocks run on an SM instead of two.  Its blocks,
+// and k_lu_small's, take their draws from a counter: a block that waits for tensor memory
+// or an SM held by another engine's kernel has none to catch up on (three engines' steps
+// at m = 400 in turn: 4.60 ms a step with fixed shares, 4.26 ms).  10 000
 // draws at m = 400 (core of 215): 3.62 ms by one kernel, 2.52 + 0.52 ms so (2.84 with the
 // general kernel's code for solves and unplanned matrices in it); the 64 KB per
 // draw in between, 0.2 ms of memory traffic, go on beside the chains.
@@ -1859,7 +1862,8 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
          const double *__restrict__ x, const T *__restrict__ lambda, RngKey key, bool refine,
          double *__restrict__ y, GammaRows rows, const double *__restrict__ nu_in,
          int *__restrict__ pivot_list, const int *__restrict__ draw_list,
-         float *__restrict__ tail = nullptr, long first = 0, long count = 0) {
+         float *__restrict__ tail = nullptr, long first = 0, long count = 0,
+         int *__restrict__ next = nullptr) {
   static_assert(!TC || sizeof(T) == 4, "tensor-core path: FP32 draws");
   constexpr bool Front = Mode == kFront;
   static_assert(TC || !Front, "");
@@ -1912,7 +1916,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 2 : 1)
   const uint32_t tmem = TC ? s_tmem : 0u;
 
   const long n_todo = Front ? count : (draw_list ? min((long)draw_list[0], n) : n);
-  for (long it = blockIdx.x; it < n_todo; it += gridDim.x) {
+  __shared__ int s_next[2];
+  if constexpr (Front) {
+    if (tid == 0) s_next[1] = atomicAdd(next, 1);
+    __syncthreads();
+  }
+  int turn = 0;
+  for (long it = Front ? s_next[1] : blockIdx.x; it < n_todo;
+       it = Front ? (long)s_next[(turn ^= 1) ^ 1] : it + gridDim.x) {
+    if (Front && tid == 0) s_next[turn] = atomicAdd(next, 1);  // read after this draw's barriers
     const long i = Front ? first + it : (draw_list ? (long)draw_list[1 + it] : it);
     if (tid == 0) sflag = 0;
     bool bad = false;
@@ -2516,7 +2528,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
     k_lu_small(int m, int P, int dp, long n, EliminationPlan ep, const float *__restrict__ theta_g,
                double *__restrict__ logdet, int *__restrict__ draw_flags,
                int *__restrict__ pivot_list, int core_n, const float *__restrict__ tail, long first,
-               long count) {
+               long count, int *__restrict__ next) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   const SmallSmem S(Tail ? 0 : ep.nv, Tail ? 0 : m);
   float *Bs = reinterpret_cast<float *>(smem_raw + S.off_B);
@@ -2570,7 +2582,12 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
   };
-  for (long it = blockIdx.x; it < (Tail ? count : n); it += gridDim.x) {
+  __shared__ int s_next[2];
+  if (tid == 0) s_next[1] = atomicAdd(next, 1);
+  __syncthreads();
+  int turn = 0;
+  for (long it = s_next[1]; it < (Tail ? count : n); it = (long)s_next[(turn ^= 1) ^ 1]) {
+    if (tid == 0) s_next[turn] = atomicAdd(next, 1);  // read after this draw's barriers
     const long i = Tail ? first + it : it;
     const float *rest = tail + (size_t)it * kTailElems;
     if (tid == 0) sflag = Tail ? (int)rest[kSmallMaxDp * kSmallMaxDp] : 0;
@@ -2614,7 +2631,7 @@ __global__ void __launch_bounds__(kSmallThreads, 4)
       asm volatile("tcgen05.wait::st.sync.aligned;");
     }
     if constexpr (Tail) {
-      // this block's next 64 KB on their way to L2
+      // a draw's 64 KB on their way to L2, about as far ahead as the blocks will take it
       if (it + gridDim.x < count) {
         const float *ahead = tail + (size_t)(it + gridDim.x) * kTailElems + 32 * tid;
 #pragma unroll
@@ -3301,7 +3318,7 @@ int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &e
                const unsigned *sp, const T *theta, const T *theta_g, T *scratch,
                double *logdet, int *draw_flags,
                const double *x, const T *lambda, RngKey key, bool refine, double *y,
-               GammaRows rows, const double *nu_in, int *pivot_list, const int *draw_list) {
+               GammaRows rows, const double *nu_in, int *pivot_list, const int *draw_list, int *next) {
   // opt in to exactly the shared memory this plan needs (a failure here shows up
   // as a launch error that the engine reports)
   auto run = [&](auto kernel) {
@@ -3311,17 +3328,17 @@ int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &e
                                               pl.vals_smem, pl.prog_smem, n, ep, sp, theta,
                                               theta_g, scratch,
                                               logdet, draw_flags, x, lambda, key, refine, y, rows,
-                                              nu_in, pivot_list, draw_list, nullptr, 0, 0);
+                                              nu_in, pivot_list, draw_list, nullptr, 0, 0, nullptr);
   };
   if constexpr (sizeof(T) == 4) {
-    if (pl.small_grid > 0 && !x && !draw_list && theta_g && pivot_list) {
+    if (pl.small_grid > 0 && !x && !draw_list && theta_g && pivot_list && next) {
       auto *f = k_lu_small<false>;
       cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.small_smem);
       f<<<pl.small_grid, kSmallThreads, pl.small_smem, s>>>(pl.m, pl.P, pl.dp, n, ep, theta_g, logdet,
-                                                            draw_flags, pivot_list, ep.core_n, nullptr, 0, 0);
+                                                            draw_flags, pivot_list, ep.core_n, nullptr, 0, 0, next);
       return 1;
     }
-    if (pl.tail_draws > 0 && n > pl.grid && !x && !draw_list && theta_g && pivot_list) {
+    if (pl.tail_draws > 0 && n > pl.grid && !x && !draw_list && theta_g && pivot_list && next) {
       auto *front = k_lu<T, true, kFront>;
       auto *rest = k_lu_small<true>;
       cudaFuncSetAttribute(front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
@@ -3331,13 +3348,14 @@ int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &e
       const long parts = (n + pl.tail_draws - 1) / pl.tail_draws, per = (n + parts - 1) / parts;
       for (long first = 0; first < n; first += per) {
         const long count = std::min(per, n - first);
+        if (first > 0) cudaMemsetAsync(next, 0, 2 * sizeof(int), s);
         front<<<(unsigned)std::min<long>(pl.grid, count), pl.block, pl.smem, s>>>(
             pl.m, pl.P, pl.dp, pl.scratch_elems_per_cta, pl.vals_smem, pl.prog_smem, n, ep, sp, theta,
             theta_g, scratch, logdet, draw_flags, nullptr, nullptr, key, false, nullptr, rows, nullptr,
-            nullptr, nullptr, tail, first, count);
+            nullptr, nullptr, tail, first, count, next);
         rest<<<(unsigned)std::min<long>(pl.tail_grid, count), kSmallThreads, pl.small_smem, s>>>(
             pl.m, pl.P, kSmallMaxDp, n, ep, theta_g, logdet, draw_flags, pivot_list,
-            ep.core_n - (pl.dp - kSmallMaxDp), tail, first, count);
+            ep.core_n - (pl.dp - kSmallMaxDp), tail, first, count, next + 1);
       }
       return (int)(2 * parts);
     }
@@ -3425,12 +3443,12 @@ template int launch_lu<float>(cudaStream_t, const LuPlan &, long, const Eliminat
                                const unsigned *, const float *, const float *, float *,
                                double *, int *,
                                const double *, const float *, RngKey, bool, double *, GammaRows,
-                               const double *, int *, const int *);
+                               const double *, int *, const int *, int *);
 template int launch_lu<double>(cudaStream_t, const LuPlan &, long, const EliminationPlan &,
                                 const unsigned *, const double *, const double *, double *,
                                 double *, int *,
                                 const double *, const double *, RngKey, bool, double *,
-                                GammaRows, const double *, int *, const int *);
+                                GammaRows, const double *, int *, const int *, int *);
 template void launch_forecast_nu<float>(cudaStream_t, int, int, long, GammaRows, const float *,
                                         const double *, const float *, const float *, RngKey,
                                         double *);
