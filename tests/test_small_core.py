@@ -110,3 +110,24 @@ def test_last_rows_of_draws_that_need_pivoting(built_lib, m, spread):
     assert few_flags <= many_flags <= few_flags + 130
     assert spread < 3.0 or few_flags > 0
     s.close()
+
+
+def test_last_rows_in_two_parts(built_lib):
+    """More draws than one hand-over takes (16 384): the first draws against the same draws
+    alone, and the second part's log weights against the first's (independent draws of one
+    distribution: means within six standard errors, standard deviations within a tenth)."""
+    s, wl, par = _engine(275, 17, 278, 0.05)
+    logw = []
+    for n in (250, 16500):
+        s.setPosteriorParameters(*par)
+        s.setRngState(5, 0)
+        w = s.computeVBPosterior(n, n)["IS_weights"]
+        assert s.getStats()["draws_pivoted"] == 0
+        assert np.all(w > 0) and abs(w.sum() - 1.0) < 1e-12
+        logw.append(np.log(w))
+    few, many = logw
+    np.testing.assert_allclose(many[:250] - many[0], few - few[0], rtol=0, atol=1e-10)
+    a, b = many[:8250], many[8250:]
+    assert abs(a.mean() - b.mean()) <= 6 * many.std() * np.sqrt(2 / 8250)
+    assert abs(a.std() - b.std()) <= 0.1 * many.std()
+    s.close()
