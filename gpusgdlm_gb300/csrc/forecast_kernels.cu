@@ -35,6 +35,7 @@
 #include <algorithm>
 
 #include "kernels.hpp"
+#include "max_sets.hpp"
 
 namespace sgdlm {
 namespace {
@@ -65,7 +66,7 @@ struct JacSmem {
     yd = take((size_t)m * nb * sizeof(double));
     xa = take((size_t)m * nb * sizeof(float));
     xb = take((size_t)m * nb * sizeof(float));
-    red = take(4 * (size_t)nb * sizeof(unsigned));
+    red = take(kMaxSets * 2 * (size_t)nb * sizeof(unsigned));
     total = o;
   }
 };
@@ -116,13 +117,13 @@ __device__ __forceinline__ bool is_tiny(float f) {  // not zero, below the norma
 __device__ __forceinline__ unsigned key_of(float v) {
   return __float_as_uint(v == v ? fabsf(v) : INFINITY);
 }
-// Block-wide maxima of 2 NB keys (all zero-based): in place.  red: two sets of 2 NB
-// words used in turn (par); the set not in use is cleared for the next call.  Ends
-// on a barrier.
+// Block-wide maxima of 2 NB keys (all zero-based): in place.  red: kMaxSets sets of 2 NB
+// words, zero at first, used in turn (`set`); one barrier, and none is needed between
+// two calls (max_sets.hpp).
 template <int NB>
 __device__ __forceinline__ void block_max(unsigned (&a)[NB], unsigned (&b)[NB], unsigned *red,
-                                          int &par) {
-  unsigned *cur = red + par * 2 * NB;
+                                          int &set) {
+  unsigned *cur = red + set * 2 * NB;
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     const unsigned u = __reduce_max_sync(0xffffffffu, a[q]);
@@ -138,9 +139,8 @@ __device__ __forceinline__ void block_max(unsigned (&a)[NB], unsigned (&b)[NB], 
     a[q] = cur[2 * q];
     b[q] = cur[2 * q + 1];
   }
-  par ^= 1;
-  // every thread has passed the barrier, so has read the other set's last maxima
-  if (threadIdx.x < 2 * NB) red[par * 2 * NB + threadIdx.x] = 0u;
+  if (threadIdx.x < 2 * NB) red[set_to_clear(set) * 2 * NB + threadIdx.x] = 0u;
+  set = set_after(set);
 }
 
 // The thread's row in ELL form held in registers: K slots (entries beyond the row's
@@ -164,7 +164,7 @@ template <int K, int NB> struct Row {
 template <int K, int NB>
 __device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row<K, NB> &R,
                                            const float (&c)[NB], float *xa, float *xb,
-                                           unsigned *red, int &par, float tol, unsigned todo,
+                                           unsigned *red, int &set, float tol, unsigned todo,
                                            float (&x)[NB]) {
   unsigned conv = 0;
 #pragma unroll
@@ -206,7 +206,7 @@ __device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row
       if (live) x[b] = a0[b];
     }
     if (check) {
-      block_max<NB>(dk, xk, red, par);  // also the barrier between sweeps
+      block_max<NB>(dk, xk, red, set);  // also the barrier between sweeps
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const float xmax = __uint_as_float(xk[b]);
@@ -255,8 +255,8 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
     const uint32_t c1 = q + 1 < len ? (uint32_t)rows.ent[e0 + q + 1].y : (uint32_t)r;
     R.col[q >> 1] = c0 | (c1 << 16);
   }
-  if (tid < 4 * NB) red[tid] = 0u;
-  int par = 0;
+  if (tid < kMaxSets * 2 * NB) red[tid] = 0u;
+  int set = 0;
   __syncthreads();
   for (long i0 = (long)blockIdx.x * NB; i0 < n; i0 += (long)gridDim.x * NB) {
     const int nd = (int)min((long)NB, n - i0);
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
     if constexpr (sizeof(T) == 4) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) c[b] = (float)nud[b];
-      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kSweepTol, ok, yo);
+      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, ok, yo);
       if (ok) {
         // residual in FP64 and its correction by the same iteration.  The iterates are
         // widened once per row, the Gamma entries without the conversion instruction
@@ -312,14 +312,14 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) c[b] = (float)v[b];
-        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kCorrSweepTol, ok, x);
+        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kCorrSweepTol, ok, x);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           ka[b] = mine ? key_of(x[b]) : 0u;
           kb[b] = mine ? key_of(yo[b]) : 0u;
           out[b] = (double)yo[b] + (double)x[b];
         }
-        block_max<NB>(ka, kb, red, par);
+        block_max<NB>(ka, kb, red, set);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           const float dmax = __uint_as_float(ka[b]), ymax = __uint_as_float(kb[b]);
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
         ka[b] = (unsigned)__double2hiint(nud[b]) & 0x7FFFFFFFu;
         kb[b] = 0u;
       }
-      block_max<NB>(ka, kb, red, par);
+      block_max<NB>(ka, kb, red, set);
 #pragma unroll
       for (int b = 0; b < NB; ++b) {
         const int ex = (int)(ka[b] >> 20);  // biased exponent of the largest |nu|
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
         if (sc) nud[b] *= __hiloint2double((1023 - e) << 20, 0);
         c[b] = (float)nud[b];
       }
-      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kSweepTol, ok, yo);
+      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, ok, yo);
       unsigned todo = ok;
 #pragma unroll
       for (int b = 0; b < NB; ++b) out[b] = (double)yo[b];
@@ -373,7 +373,7 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) c[b] = (float)(v[b] * up);
-        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, par, kSweepTol, todo, x);
+        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, todo, x);
         ok &= ~(todo & ~conv);
         todo &= conv;
 #pragma unroll
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
           ka[b] = mine ? key_of(x[b]) : 0u;
           kb[b] = mine ? key_of((float)out[b]) : 0u;
         }
-        block_max<NB>(ka, kb, red, par);
+        block_max<NB>(ka, kb, red, set);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           const double dmax = (double)__uint_as_float(ka[b]) * down, ymax = (double)__uint_as_float(kb[b]);
