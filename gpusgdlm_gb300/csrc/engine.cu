@@ -214,9 +214,11 @@ struct sgdlm_engine {
   LuOptions lu_opt{};
   JacobiPlan jac32{}, jac64{};  // iterative forecast solves of FP32 and FP64 draws
   int forecast_iterative = 1;
-  // FP64: the current draws' log|det| were not needed by the forecast that drew them
-  // (sgdlm_get_draws computes them)
+  // FP64: the last forecast's draws' log|det| were not needed by it (complete_logdet
+  // computes them: for sgdlm_get_draws, or before the parental sets change).  pending_at:
+  // where in theta_g (elements) those draws' Gamma entries are once the draws have evolved
   bool logdet_pending = false;
+  size_t pending_at = 0;
   DevBuf<int> jac_list;    // nsim + 1: count, then the forecast draws left to factor
   ProposalState prop;
   int chunks = 0;          // VB draw chunks and draws per chunk (vb_chunking)
@@ -579,6 +581,8 @@ void release_sim(sgdlm_engine *h) {
   h->pivot_list.release();
   h->jac_list.release();
   h->sim_init = false;
+  h->logdet_pending = false;
+  h->pending_at = 0;
   h->nsim = 0;
   h->nsim_batch = 0;
 }
@@ -698,7 +702,10 @@ int alloc_sim(sgdlm_engine *h, size_t nsim) {
   CK(h->jac_list.reserve(nsim + 1));
   CK(h->part_a.reserve((size_t)h->chunks * m * (P + 2) + m * P));
   CK(h->part_b.reserve((size_t)h->chunks * m * P * P));
-  if (h->nsim != nsim) h->logdet_pending = false;
+  if (h->nsim != nsim) {  // no draws at this count yet
+    h->logdet_pending = false;
+    h->pending_at = 0;
+  }
   h->nsim = nsim;
   return SGDLM_OK;
 }
@@ -764,6 +771,7 @@ void sample_draws(sgdlm_engine *h, const double *m_t, const double *C_t, const d
                   const double *s_t, RngKey key) {
   const int m = (int)h->m, P = (int)h->P;
   const long n = (long)h->nsim;
+  h->logdet_pending = false;  // the draws are replaced
   launch_cholesky(h->stream, m, P, h->p.ptr, C_t, h->U64.ptr, h->U32.ptr);
   const T *U = std::is_same<T, float>::value ? reinterpret_cast<const T *>(h->U32.ptr)
                                               : reinterpret_cast<const T *>(h->U64.ptr);
@@ -783,12 +791,15 @@ template <typename T> bool iterative_forecast(const sgdlm_engine *h) {
   return h->forecast_iterative && jacobi_plan<T>(h).ok && !warp_lu(h);
 }
 
+// g_at: where in theta_g the draws' Gamma entries begin (pending_at).
 template <typename T>
-int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
+int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y, size_t g_at = 0) {
   const long n = (long)h->nsim;
   const bool refine = (h->precision != SGDLM_PRECISION_FP64);
-  // FP64: the log|det| of iteratively solved draws are left to sgdlm_get_draws
+  const T *theta_g = as<T>(h->theta_g) + g_at;
+  // FP64: the log|det| of iteratively solved draws are left to complete_logdet
   h->logdet_pending = std::is_same<T, double>::value && x && iterative_forecast<T>(h);
+  h->pending_at = 0;
   const GammaRows rows{h->g_rowptr.ptr, h->g_ent.ptr, h->g_extptr.ptr, h->g_extk.ptr};
   if (x) {
     const size_t nx = h->m * h->P;
@@ -798,7 +809,7 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
     h->launches += 2;
   }
   if (warp_lu(h)) {
-    launch_lu_warp<T>(h->stream, (int)h->m, n, h->num_sms, rows, as<T>(h->theta_g), h->g_nnz,
+    launch_lu_warp<T>(h->stream, (int)h->m, n, h->num_sms, rows, theta_g, h->g_nnz,
                       h->logdet.ptr, h->draw_flags.ptr, x ? h->nu_fc.ptr : nullptr, x ? y : nullptr,
                       h->tab64.ptr);
     h->launches += 1;
@@ -809,7 +820,7 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
   const bool iterative = iterative_forecast<T>(h) && x;
   if (iterative) {
     CK(cudaMemsetAsync(h->jac_list.ptr, 0, sizeof(int), h->stream));
-    launch_forecast_jacobi<T>(h->stream, jacobi_plan<T>(h), (int)h->m, n, rows, as<T>(h->theta_g),
+    launch_forecast_jacobi<T>(h->stream, jacobi_plan<T>(h), (int)h->m, n, rows, theta_g,
                               h->g_nnz, h->nu_fc.ptr, y, h->logdet.ptr, h->jac_list.ptr);
     h->launches += 1;
   }
@@ -823,20 +834,39 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y) {
     // fewer FP64 operations than the levels and dense core below)
     deep = !x && h->deep_launch.ok;
     if (deep)
-      launch_logdet64(h->stream, h->deep_launch, n, h->deep_dev, as<T>(h->theta_g),
+      launch_logdet64(h->stream, h->deep_launch, n, h->deep_dev, theta_g,
                       as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, pivot_list, next);
   }
   int lu_launches = 1;
   if (!deep)
     lu_launches = launch_lu<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
-                               as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr,
+                               theta_g, as<T>(h->lu_scratch), h->logdet.ptr,
                                h->draw_flags.ptr, x, as<T>(h->lambda), key, refine, y, rows,
                                x ? h->nu_fc.ptr : nullptr, pivot_list,
                                iterative ? h->jac_list.ptr : nullptr, next);
   launch_lu_fallback<T>(h->stream, h->plan, n, h->elim_dev, h->sp.ptr, as<T>(h->theta),
-                        as<T>(h->theta_g), as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x,
+                        theta_g, as<T>(h->lu_scratch), h->logdet.ptr, h->draw_flags.ptr, x,
                         as<T>(h->lambda), key, y, rows, pivot_list);
   h->launches += 1 + lu_launches;
+  return SGDLM_OK;
+}
+
+// The log|det| that the last forecast of FP64 draws left out, from those draws.
+int complete_logdet(sgdlm_engine *h) {
+  if (!h->logdet_pending) return SGDLM_OK;
+  return lu_draws<double>(h, nullptr, h->key((uint32_t)h->epoch), nullptr, h->pending_at);
+}
+// The draws evolve: the Gamma entries that pending log|det| are of go behind those in use
+// (theta_g has room for m max_p entries per draw); where they do not fit there, or the
+// redo would need the coefficients themselves (no levels), they are computed now.
+int keep_pending_draws(sgdlm_engine *h) {
+  if (!h->logdet_pending || h->pending_at) return SGDLM_OK;
+  const size_t used = (h->nsim * (size_t)h->g_nnz + 3) / 4 * 4;
+  if (used == 0 || h->eplan.nlev == 0 || 2 * used * sizeof(double) > h->theta_g.count)
+    return complete_logdet(h);
+  double *g = as<double>(h->theta_g);
+  CK(cudaMemcpyAsync(g + used, g, used * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+  h->pending_at = used;
   return SGDLM_OK;
 }
 
@@ -979,6 +1009,7 @@ int learned_draws(sgdlm_engine *h, RngKey key) {
   launch_proposal_features(s, m, P, h->p.ptr, h->sp.ptr, h->m_t.ptr, h->C_t.ptr, h->n_t.ptr,
                            h->s_t.ptr, q.X.ptr);
   launch_normalise(s, m, F, q.fsum.ptr, q.X.ptr);
+  h->logdet_pending = false;  // the draws are replaced
   mlp_forward(s, q.L, m, q.X.ptr, q.w.ptr, q.w16.ptr, q.acts());
   T *Uq = std::is_same<T, float>::value ? reinterpret_cast<T *>(q.Uq32.ptr)
                                         : reinterpret_cast<T *>(q.Uq64.ptr);
@@ -1212,6 +1243,8 @@ int upload_evolution_matrix(sgdlm_engine *h, const double *G) {
 template <typename T> int evolve(sgdlm_engine *h, bool with_G = false) {
   const int m = (int)h->m, P = (int)h->P;
   const long n = (long)h->nsim;
+  int st = keep_pending_draws(h);
+  if (st) return st;
   const RngKey key = h->key((uint32_t)h->epoch);
   h->epoch += 1;
   advance_device_epoch(h, 1);
@@ -1303,9 +1336,7 @@ int export_draws(sgdlm_engine *h, double *o_lambda, double *o_theta, double *o_l
     th.resize(m * n * P);
     if ((st = d2h(h, th.data(), h->theta.ptr, m * n * P * sizeof(T)))) return st;
   }
-  if (o_logdet && h->logdet_pending &&
-      (st = lu_draws<T>(h, nullptr, h->key((uint32_t)h->epoch), nullptr)))
-    return st;
+  if (o_logdet && (st = complete_logdet(h))) return st;
   if (o_logdet && (st = d2h(h, o_logdet, h->logdet.ptr, n * sizeof(double)))) return st;
   if ((st = sync(h))) return st;
   if (o_lambda)
@@ -1527,6 +1558,9 @@ int sgdlm_set_parental_sets(sgdlm_handle h, const unsigned *p, const unsigned *s
     if ((st = h2d(h, h->p.ptr, p, m * sizeof(unsigned)))) return st;
   }
   if (sp) {
+    // pending log|det| are of draws under the present sets
+    if (std::memcmp(h->h_sp.data(), sp, m * P * sizeof(unsigned)) != 0 && (st = complete_logdet(h)))
+      return st;
     std::memcpy(h->h_sp.data(), sp, m * P * sizeof(unsigned));
     if ((st = h2d(h, h->sp.ptr, sp, m * P * sizeof(unsigned)))) return st;
     if ((st = sync(h))) return st;
@@ -1706,9 +1740,10 @@ int sgdlm_set_precision(sgdlm_handle h, int precision) {
   if (precision != SGDLM_PRECISION_FP64 && precision != SGDLM_PRECISION_MIXED)
     return h->fail(SGDLM_ERR_BAD_ARG, "unknown precision");
   if (precision == h->precision) return SGDLM_OK;
+  int st0 = complete_logdet(h);  // while the draws' type is known
+  if (st0) return st0;
   const int old = h->precision;
   h->precision = precision;
-  h->logdet_pending = false;
   if (h->sim_init) {
     const size_t nsim = h->nsim, batch = h->nsim_batch;
     cudaStreamSynchronize(h->stream);
@@ -1728,10 +1763,12 @@ int sgdlm_set_precision(sgdlm_handle h, int precision) {
 int sgdlm_set_elimination_levels(sgdlm_handle h, int levels) {
   HCHECK(h);
   if (levels < 0 || levels > kMaxLevels) return h->fail(SGDLM_ERR_BAD_ARG, "levels must be in 0..16");
+  int st = h->pending_at ? complete_logdet(h) : SGDLM_OK;  // (keep_pending_draws: with levels)
+  if (st) return st;
   h->elim_levels = levels;
   if (!h->mem_init) return SGDLM_OK;
   cudaStreamSynchronize(h->stream);
-  int st = upload_elimination(h);
+  st = upload_elimination(h);
   if (st) return st;
   return replan_sim(h);
 }
@@ -2099,6 +2136,8 @@ int batch_capture(sgdlm_batch *b) {
     e = cudaStreamWaitEvent(h->stream, b->fork, 0);
     if (e != cudaSuccess) break;
     const uint64_t l0 = h->launches, ep0 = h->epoch;
+    const bool pending0 = h->logdet_pending;
+    const size_t pending_at0 = h->pending_at;
     status = h->precision == SGDLM_PRECISION_FP64
                  ? filter_step<double>(h, b->y[i], b->F[i], b->x[i], b->ess, b->fc[i], b->w[i],
                                        b->st[i])
@@ -2108,6 +2147,8 @@ int batch_capture(sgdlm_batch *b) {
     b->logdet_pending[i] = h->logdet_pending ? 1 : 0;
     h->launches = l0;   // counted when the graph runs
     h->epoch = ep0;     // advanced when the graph runs
+    h->logdet_pending = pending0;  // nothing has been drawn yet
+    h->pending_at = pending_at0;
     if (status == SGDLM_OK) e = cudaEventRecord(b->join[i], h->stream);
     if (e == cudaSuccess && status == SGDLM_OK) e = cudaStreamWaitEvent(b->origin, b->join[i], 0);
   }
@@ -2142,6 +2183,7 @@ int batch_launch(sgdlm_batch *b) {
     h->launches += b->launches_per_step[i];
     h->is_prior = true;
     h->logdet_pending = b->logdet_pending[i] != 0;
+    h->pending_at = 0;
   }
   return SGDLM_OK;
 }

@@ -317,10 +317,11 @@ __global__ void __launch_bounds__(128)
 }
 
 // Writes the identity plus the scattered -theta entries of draw i into the full
-// mp x mp matrix A (fillGammas, kernel_functions.cuh:822-842).
+// mp x mp matrix A (fillGammas, kernel_functions.cuh:822-842).  l0_e: the theta indices of
+// the Gamma copy's entries, which are then read there, or nullptr.
 template <typename T>
 __device__ void build_full(int m, int P, int mp, long n, long i, const unsigned *__restrict__ sp,
-                           Theta<T> theta, T *__restrict__ A) {
+                           Theta<T> theta, T *__restrict__ A, const int *__restrict__ l0_e = nullptr) {
   const int tid = threadIdx.x;
   const size_t n16 = (size_t)mp * mp * sizeof(T) / 16;
   uint4 *A16 = reinterpret_cast<uint4 *>(A);
@@ -328,11 +329,14 @@ __device__ void build_full(int m, int P, int mp, long n, long i, const unsigned 
   __syncthreads();
   for (int r = tid; r < mp; r += blockDim.x) A[(size_t)r * mp + r] = T(1);
   const size_t mm = (size_t)m * m;
-  for (int e = tid; e < m * P; e += blockDim.x) {
+  const bool copy = theta.g && l0_e;
+  const int cnt = copy ? theta.nnz : m * P;
+  for (int q = tid; q < cnt; q += blockDim.x) {
+    const int e = copy ? l0_e[q] : q;
     const unsigned pos = sp[e];
     if ((size_t)pos < mm) {
       const int row = (int)(pos % (unsigned)m), col = (int)(pos / (unsigned)m);
-      A[row + (size_t)mp * col] = -theta.at(i, e);
+      A[row + (size_t)mp * col] = -(copy ? theta.gamma(i, q, e) : theta.at(i, e));
     }
   }
   __syncthreads();
@@ -3138,7 +3142,7 @@ __global__ void __launch_bounds__(kThreads)
       // ---- the full matrix
       N = mp;
       ld_part = 0.0;
-      build_full<T>(m, P, mp, n, i, sp, theta, A);
+      build_full<T>(m, P, mp, n, i, sp, theta, A, planned ? ep.l0_e : nullptr);
       if (solve)
         for (int r = tid; r < mp; r += blockDim.x) b.z[r] = (r < m) ? (T)nu[r] : T(0);
       __syncthreads();
