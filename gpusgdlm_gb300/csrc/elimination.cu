@@ -12,20 +12,29 @@ namespace {
 constexpr double kMinLevelShare = 0.05;
 }  // namespace
 
+std::vector<int> gamma_order(int m, int P, const std::vector<unsigned> &sp) {
+  const size_t mm = (size_t)m * m;
+  std::vector<int> order;
+  for (int e = 0; e < m * P; ++e)
+    if ((size_t)sp[e] < mm) order.push_back(e);
+  std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
+    return sp[a] % (unsigned)m < sp[b] % (unsigned)m;
+  });
+  return order;
+}
+
 EliminationPlanHost plan_elimination(int m, int P, const std::vector<unsigned> &sp,
                                      int max_levels) {
   EliminationPlanHost pl;
   pl.m = m;
   pl.P = P;
-  const size_t mm = (size_t)m * m;
   // current pattern: row r -> (col -> slot), col c -> (row -> slot)
   std::vector<std::map<int, int>> rows(m), cols(m);
   std::vector<int> diag(m);
   for (int r = 0; r < m; ++r) diag[r] = (int)kSlotDiag0 + r;
   int nv = (int)kSlotDiag0 + m;
-  for (int e = 0; e < m * P; ++e) {
+  for (int e : gamma_order(m, P, sp)) {
     const unsigned pos = sp[e];
-    if ((size_t)pos >= mm) continue;
     const int r = (int)(pos % (unsigned)m), c = (int)(pos / (unsigned)m);
     rows[r][c] = nv;
     cols[c][r] = nv;
@@ -300,9 +309,8 @@ LogdetPlanHost plan_logdet(int m, int P, const std::vector<unsigned> &sp, int ma
   int nv = 1;  // slot 0: constant 0
   for (int r = 0; r < m; ++r) pl.diag_slot.push_back(slot[at(r, r)] = nv++);
   size_t nz = (size_t)m;
-  for (int e = 0; e < m * P; ++e) {
+  for (int e : gamma_order(m, P, sp)) {
     const unsigned pos = sp[e];
-    if ((size_t)pos >= mm) continue;
     const int r = (int)(pos % (unsigned)m), c = (int)(pos / (unsigned)m);
     pl.l0_slot.push_back(slot[at(r, c)] = nv++);
     rows[r].push_back(c);

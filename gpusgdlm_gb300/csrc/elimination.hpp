@@ -131,6 +131,11 @@ struct EliminationPlan {
   LevelStream stream;  // the levels for blocks of 256 threads (k_lu, FP32 draws, log|det|)
 };
 
+// The theta indices e = j*max_p + k of the Gamma entries (sp[e] < m*m), row of (I - Gamma)
+// by row, within a row in increasing e: the order of the draw-major Gamma copy and of
+// both plans' level-0 entries.
+std::vector<int> gamma_order(int m, int P, const std::vector<unsigned> &sp);
+
 // Builds the plan from the parental sets (sp: max_p x m, entries < m*m address
 // (I - Gamma) at row + m*col).  max_levels = 0, or parental sets with more than
 // kMaxSlots values, give no levels (the plain dense LU of the whole matrix).

@@ -202,6 +202,8 @@ struct sgdlm_engine {
   // the draws' Gamma entries draw-major (GammaDraws), room for m * P per draw
   DevBuf<unsigned char> theta_g;
   int g_nnz = 0;  // Gamma entries (rows' CSR length)
+  bool g_own_rows = true;  // every coefficient of series j addresses row j
+  bool g_stale = false;    // theta_g is not the present parental sets' copy of the draws
   DevBuf<double> logdet, w, y_fc, nu_fc, stats6, wpart, part_a, part_b;
   DevBuf<int> draw_flags, series_flags;
   // nsim + 2: the work counter of k_logdet64, then the count of the draws flagged for
@@ -343,9 +345,12 @@ int upload_gamma_rows(sgdlm_engine *h) {
   for (size_t r = 0; r < m; ++r) rowptr[r + 1] += rowptr[r];
   ent.resize(rowptr[m] > 0 ? rowptr[m] : 1);
   std::vector<int> fill(rowptr.begin(), rowptr.end() - 1);
+  h->g_own_rows = true;
   for (size_t e = 0; e < m * P; ++e) {
     const unsigned pos = h->h_sp[e];
-    if ((size_t)pos < mm) ent[fill[pos % m]++] = make_int2((int)e, (int)(pos / m));
+    if ((size_t)pos >= mm) continue;
+    ent[fill[pos % m]++] = make_int2((int)e, (int)(pos / m));
+    if (pos % m != e / P) h->g_own_rows = false;
   }
   CK(h->g_rowptr.alloc(m + 1));
   CK(h->g_ent.alloc(ent.size()));
@@ -759,9 +764,11 @@ void advance_device_epoch(sgdlm_engine *h, uint32_t delta) {
 }
 
 // The sampler's draw-major copy of the Gamma entries (read by the LU and
-// iterative-solve kernels).
+// iterative-solve kernels); not written by the sampler: lu_draws gathers it.
 template <typename T> GammaDraws<T> gamma_draws(sgdlm_engine *h) {
-  return GammaDraws<T>{as<T>(h->theta_g), h->g_rowptr.ptr, h->sp.ptr, h->g_nnz};
+  h->g_stale = !h->g_own_rows;
+  return GammaDraws<T>{h->g_own_rows ? as<T>(h->theta_g) : nullptr, h->g_rowptr.ptr, h->sp.ptr,
+                       h->g_nnz};
 }
 
 // sample -> LU -> fallback, from the given normal-gamma parameters (posterior
@@ -801,6 +808,12 @@ int lu_draws(sgdlm_engine *h, const double *x, RngKey key, double *y, size_t g_a
   h->logdet_pending = std::is_same<T, double>::value && x && iterative_forecast<T>(h);
   h->pending_at = 0;
   const GammaRows rows{h->g_rowptr.ptr, h->g_ent.ptr, h->g_extptr.ptr, h->g_extk.ptr};
+  if (h->g_stale && g_at == 0) {
+    launch_gather_gamma<T>(h->stream, (int)h->P, n, rows.ent, h->g_nnz, as<T>(h->theta),
+                           as<T>(h->theta_g));
+    h->g_stale = false;
+    h->launches += 1;
+  }
   if (x) {
     const size_t nx = h->m * h->P;
     launch_to_float(h->stream, nx, x, h->x32.ptr);
@@ -1564,6 +1577,7 @@ int sgdlm_set_parental_sets(sgdlm_handle h, const unsigned *p, const unsigned *s
     std::memcpy(h->h_sp.data(), sp, m * P * sizeof(unsigned));
     if ((st = h2d(h, h->sp.ptr, sp, m * P * sizeof(unsigned)))) return st;
     if ((st = sync(h))) return st;
+    h->g_stale = true;
     if ((st = upload_gamma_rows(h))) return st;
     if ((st = upload_elimination(h))) return st;
     if ((st = replan_sim(h))) return st;
@@ -2138,6 +2152,7 @@ int batch_capture(sgdlm_batch *b) {
     const uint64_t l0 = h->launches, ep0 = h->epoch;
     const bool pending0 = h->logdet_pending;
     const size_t pending_at0 = h->pending_at;
+    const bool stale0 = h->g_stale;
     status = h->precision == SGDLM_PRECISION_FP64
                  ? filter_step<double>(h, b->y[i], b->F[i], b->x[i], b->ess, b->fc[i], b->w[i],
                                        b->st[i])
@@ -2149,6 +2164,7 @@ int batch_capture(sgdlm_batch *b) {
     h->epoch = ep0;     // advanced when the graph runs
     h->logdet_pending = pending0;  // nothing has been drawn yet
     h->pending_at = pending_at0;
+    h->g_stale = stale0;
     if (status == SGDLM_OK) e = cudaEventRecord(b->join[i], h->stream);
     if (e == cudaSuccess && status == SGDLM_OK) e = cudaStreamWaitEvent(b->origin, b->join[i], 0);
   }
@@ -2184,6 +2200,7 @@ int batch_launch(sgdlm_batch *b) {
     h->is_prior = true;
     h->logdet_pending = b->logdet_pending[i] != 0;
     h->pending_at = 0;
+    h->g_stale = false;
   }
   return SGDLM_OK;
 }

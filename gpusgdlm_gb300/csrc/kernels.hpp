@@ -61,12 +61,13 @@ void launch_cholesky(cudaStream_t s, int m, int P, const unsigned *p, const doub
                      double *U64, float *U32);
 
 // The draws' Gamma entries (the simultaneous-parent coefficients), draw-major in
-// the CSR order of the rows of Gamma: row j holds series j's coefficients at the
-// positions sp[j*P + k] < m*m, in increasing k, from rowptr[j] on (GammaRows).
-// Draw i's entry q is v[i*nnz + q].  That order is also the order of increasing
-// theta index j*P + k, i.e. the elimination plan's level-0 order.  The sampler
-// writes this copy beside the series-major theta; the LU and iterative-solve
-// kernels read a draw's nnz values as one run.
+// the CSR order of the rows of Gamma (GammaRows), which is also the elimination
+// plans' level-0 order (gamma_order).  Draw i's entry q is v[i*nnz + q].  Where every
+// coefficient of series j addresses row j (as parents do), its entries are the run from
+// rowptr[j] on, in increasing k, and the sampler writes this copy beside the series-major
+// theta; for other parental sets, and for draws made under other ones, it is gathered
+// (launch_gather_gamma).  The LU and iterative-solve kernels read a draw's nnz values as
+// one run.
 template <typename T> struct GammaDraws {
   T *v;                 // nsim * nnz, or nullptr: not written
   const int *rowptr;    // m + 1
@@ -146,6 +147,10 @@ template <typename T>
 void launch_lu_warp(cudaStream_t s, int m, long n, int num_sms, GammaRows rows, const T *theta_g,
                     int nnz, double *logdet, int *draw_flags, const double *nu, double *y,
                     const double *tab);
+// The draw-major copy of the Gamma entries (ent: GammaRows) from the series-major theta.
+template <typename T>
+void launch_gather_gamma(cudaStream_t s, int P, long n, const int2 *ent, int nnz, const T *theta,
+                         T *theta_g);
 struct EliminationPlan;
 template <typename T>
 // theta: the draws series-major; theta_g: their Gamma entries (GammaDraws layout,

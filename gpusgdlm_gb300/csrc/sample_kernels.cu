@@ -354,6 +354,19 @@ __global__ void __launch_bounds__(kSampleThreads)
   }
 }
 
+// The draws' Gamma entries from theta, one per thread; scattered reads, as only draws whose
+// parental sets changed, or address other rows than their series', come here.
+template <typename T>
+__global__ void __launch_bounds__(128)
+    k_gather_gamma(int P, long n, const int2 *__restrict__ ent, int nnz, const T *__restrict__ theta,
+                   T *__restrict__ theta_g) {
+  const int q = blockIdx.x * 128 + threadIdx.x;
+  if (q >= nnz) return;
+  const int e = ent[q].x, j = e / P, k = e - j * P;
+  for (long i = blockIdx.y; i < n; i += gridDim.y)
+    theta_g[(size_t)i * nnz + q] = theta[((size_t)j * n + i) * P + k];
+}
+
 template <typename T> size_t sample_smem(int P) {
   return ((size_t)P * P + P + (size_t)kSampleThreads * P) * sizeof(T);
 }
@@ -411,6 +424,18 @@ void launch_evolve(cudaStream_t s, int m, int P, long n, const unsigned *p,
                                          compat_beta_no_boost, lambda, theta, gd, draw_flags, G);
   });
 }
+
+template <typename T>
+void launch_gather_gamma(cudaStream_t s, int P, long n, const int2 *ent, int nnz, const T *theta,
+                         T *theta_g) {
+  if (nnz == 0) return;
+  const dim3 grid((unsigned)((nnz + 127) / 128), (unsigned)(n < 4096 ? n : 4096));
+  k_gather_gamma<T><<<grid, 128, 0, s>>>(P, n, ent, nnz, theta, theta_g);
+}
+template void launch_gather_gamma<float>(cudaStream_t, int, long, const int2 *, int, const float *,
+                                         float *);
+template void launch_gather_gamma<double>(cudaStream_t, int, long, const int2 *, int, const double *,
+                                          double *);
 
 template void launch_sample<float>(cudaStream_t, int, int, long, const double *,
                                    const double *, const double *, const float *, RngKey,
