@@ -17,6 +17,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -114,7 +115,9 @@ struct ProposalState {
 // Page-locked staging of an engine's small host copies.  A copy from or to pageable
 // memory makes the host wait for it (about 10 us each; a VB call has eight); staged,
 // a call's copies are queued and the call waits once.  Copies of more than kStagedMost
-// bytes, or that no longer fit, go the direct way.
+// bytes, or that no longer fit, from or to memory that the host may not read (device
+// pointers: the copy's direction is then the addresses'), and those of calls that other
+// threads make meanwhile (StageLease) go the direct way.
 struct HostStage {
   static constexpr size_t kBytes = 1u << 20, kStagedMost = 1u << 17;
   struct Out {
@@ -123,7 +126,7 @@ struct HostStage {
   };
   unsigned char *buf = nullptr;
   size_t used = 0;
-  bool failed = false;
+  std::atomic<const void *> holder{nullptr};  // the thread whose call stages its copies
   std::vector<Out> outs;  // device-to-host copies to hand on once the stream is idle
   HostStage() = default;
   HostStage(const HostStage &) = delete;
@@ -131,14 +134,28 @@ struct HostStage {
   ~HostStage() {
     if (buf) cudaFreeHost(buf);
   }
-  unsigned char *take(size_t bytes) {
-    if (bytes > kStagedMost || failed) return nullptr;
+  // with the state's memory, not by the first copy (which may be made while another
+  // stream is captured); without it every copy goes the direct way
+  void make() {
     if (!buf && cudaHostAlloc(&buf, kBytes, cudaHostAllocDefault) != cudaSuccess) {
       (void)cudaGetLastError();
       buf = nullptr;
-      failed = true;
+    }
+  }
+  static const void *this_thread() {
+    static thread_local char mark;
+    return &mark;
+  }
+  bool mine() const { return holder.load(std::memory_order_relaxed) == this_thread(); }
+  // a place for a copy from or to `host`, or nullptr
+  unsigned char *take(const void *host, size_t bytes) {
+    if (!buf || bytes > kStagedMost || !mine()) return nullptr;
+    cudaPointerAttributes pa{};  // 0.1 us
+    if (cudaPointerGetAttributes(&pa, host) != cudaSuccess) {
+      (void)cudaGetLastError();
       return nullptr;
     }
+    if (pa.type != cudaMemoryTypeUnregistered && pa.type != cudaMemoryTypeHost) return nullptr;
     const size_t at = (used + 63) / 64 * 64;
     if (at + bytes > kBytes) return nullptr;
     used = at + bytes;
@@ -146,9 +163,34 @@ struct HostStage {
   }
   // the stream is idle: the copies out reach their destinations
   void finish() {
+    if (!mine()) return;
     for (const Out &o : outs) std::memcpy(o.dst, buf + o.at, o.bytes);
     outs.clear();
     used = 0;
+  }
+};
+
+// The staging buffer for the length of an API call: the calling thread's, unless another
+// thread's call has it.  What a call that failed between its copies and its wait has left
+// is dropped (its destinations are the caller's again).
+struct StageLease {
+  HostStage &stage;
+  cudaStream_t stream;
+  bool held;
+  StageLease(HostStage &st, cudaStream_t s) : stage(st), stream(s) {
+    const void *none = nullptr;
+    held = stage.holder.compare_exchange_strong(none, HostStage::this_thread(), std::memory_order_acquire);
+  }
+  StageLease(const StageLease &) = delete;
+  StageLease &operator=(const StageLease &) = delete;
+  ~StageLease() {
+    if (!held) return;
+    if (stage.used) {
+      cudaStreamSynchronize(stream);
+      stage.outs.clear();
+      stage.used = 0;
+    }
+    stage.holder.store(nullptr, std::memory_order_release);
   }
 };
 
@@ -228,15 +270,6 @@ struct sgdlm_engine {
   cudaEvent_t ev[8] = {};
   HostStage stage;
 
-  // A call that failed between its copies and its wait leaves them behind; their
-  // destinations are the caller's again.
-  void drop_staged() {
-    if (stage.used == 0) return;
-    cudaStreamSynchronize(stream);
-    stage.outs.clear();
-    stage.used = 0;
-  }
-
   void log(int level, const char *fmt, ...) {
     char buf[512];
     va_list ap;
@@ -309,7 +342,7 @@ namespace {
   } while (0)
 
 int h2d(sgdlm_engine *h, void *dst, const void *src, size_t bytes) {
-  if (unsigned char *b = h->stage.take(bytes)) {
+  if (unsigned char *b = h->stage.take(src, bytes)) {
     std::memcpy(b, src, bytes);
     src = b;
   }
@@ -318,7 +351,7 @@ int h2d(sgdlm_engine *h, void *dst, const void *src, size_t bytes) {
 }
 // dst holds the values once sync() has returned.
 int d2h(sgdlm_engine *h, void *dst, const void *src, size_t bytes) {
-  unsigned char *b = h->stage.take(bytes);
+  unsigned char *b = h->stage.take(dst, bytes);
   CK(cudaMemcpyAsync(b ? b : dst, src, bytes, cudaMemcpyDeviceToHost, h->stream));
   if (b) h->stage.outs.push_back(HostStage::Out{dst, (size_t)(b - h->stage.buf), bytes});
   return SGDLM_OK;
@@ -562,6 +595,7 @@ int alloc_state(sgdlm_engine *h) {
   CK(h->wpart.alloc(4 * (size_t)kWeightBlocks));
   CK(h->x32.alloc(P * m));
   CK(h->dev_epoch.alloc(1));
+  h->stage.make();
   h->h_p.assign(m, 0);
   h->h_sp.assign(P * m, 0xFFFFFFFFu);
   // Parental sets default to "no simultaneous parents" (all external).
@@ -1183,13 +1217,14 @@ int forecast(sgdlm_engine *h, double *o_y, const double *x, double *o_lambda, do
   // a page-locked, device-mapped destination receives the draws straight from the
   // LU kernels (over the host link while they run); any other goes through y_fc
   double *ydst = h->y_fc.ptr;
+  bool pageable = false;
   if (o_y) {
     cudaPointerAttributes pa{};
-    if (cudaPointerGetAttributes(&pa, o_y) == cudaSuccess && pa.type == cudaMemoryTypeHost &&
-        pa.devicePointer != nullptr)
+    const bool known = cudaPointerGetAttributes(&pa, o_y) == cudaSuccess;
+    if (!known) (void)cudaGetLastError();
+    pageable = known && pa.type == cudaMemoryTypeUnregistered;
+    if (known && pa.type == cudaMemoryTypeHost && pa.devicePointer != nullptr)
       ydst = static_cast<double *>(pa.devicePointer);
-    else
-      (void)cudaGetLastError();  // pageable memory is not an error here
   }
   if ((st = lu_draws<T>(h, h->x_t.ptr, key, ydst))) return st;
   CK(cudaEventRecord(h->ev[2], s));
@@ -1197,7 +1232,7 @@ int forecast(sgdlm_engine *h, double *o_y, const double *x, double *o_lambda, do
   if (iterative_forecast<T>(h) && (st = d2h(h, &factored, h->jac_list.ptr, sizeof(int))))
     return st;
   if (o_y && ydst == h->y_fc.ptr) {
-    touch_pages(o_y, n * m * sizeof(double));
+    if (pageable) touch_pages(o_y, n * m * sizeof(double));
     if ((st = d2h(h, o_y, h->y_fc.ptr, n * m * sizeof(double)))) return st;
   }
   std::vector<T> lam, th;
@@ -1364,12 +1399,10 @@ int export_draws(sgdlm_engine *h, double *o_lambda, double *o_theta, double *o_l
 
 }  // namespace
 
-#define HCHECK(h)                                  \
-  do {                                             \
-    if (!(h)) return SGDLM_ERR_BAD_ARG;            \
-    cudaSetDevice((h)->device);                    \
-    (h)->drop_staged();                            \
-  } while (0)
+#define HCHECK(h)                     \
+  if (!(h)) return SGDLM_ERR_BAD_ARG; \
+  cudaSetDevice((h)->device);         \
+  const StageLease stage_lease((h)->stage, (h)->stream)
 
 extern "C" {
 
