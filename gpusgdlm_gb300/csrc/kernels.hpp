@@ -106,14 +106,19 @@ struct LuPlan {
   int tc;              // trailing updates on the tensor cores (tcgen05)
   int small_grid;      // > 0: log|det| by k_lu_small on so many blocks ...
   size_t small_smem;   // ... with this much shared memory each
-  int tail_draws;      // > 0: log|det| by k_lu up to the core's last 128 rows, these by
-  int tail_grid;       // k_lu_small on so many blocks, tail_draws draws at a time through
-  size_t tail_offset;  // slabs from this element of the scratch on
+  int tail_grid;       // > 0: where the caller has room for the hand-over, log|det| by
+                       // k_lu up to the core's last 128 rows, these by k_lu_small on so
+                       // many blocks; kTailBytes per draw, kTailDraws draws at most
   size_t scratch_elems_per_cta;  // dense core + per-draw values of the sparse levels
   size_t fb_elems_per_cta;       // the redo's: the above, or a full m_p x m_p slab
   int fb_core_smem;              // the redo factors the dense core in shared memory
   size_t scratch_elems_total;    // covers both passes
 };
+// What k_lu hands to k_lu_small of a draw: the core's last 128 x 128 after the panels
+// before (column-major, FP32), then whether a check failed; 128-byte aligned.
+constexpr size_t kTailElems = (size_t)128 * 128 + 32, kTailBytes = kTailElems * sizeof(float);
+// ... of so many draws at a time: 1 GiB, one part up to 16 384 draws
+constexpr long kTailDraws = 16384;
 // Tuning knobs of the fast pass: allow_tc = 0 keeps the FFMA instantiation where
 // the tensor-core one would apply; max_grid > 0 caps the persistent grid (fewer
 // CTAs, more draws each: room for other work on the GPU at the same time).
@@ -171,7 +176,9 @@ int launch_lu(cudaStream_t s, const LuPlan &plan, long n, const EliminationPlan 
                // the same form: only the listed draws are factored, or nullptr: all
                const int *draw_list = nullptr,
                // two ints, zero on entry: the blocks' work counters, or nullptr
-               int *next = nullptr);
+               int *next = nullptr,
+               // room for the hand-over of tail_draws draws (plan.tail_grid > 0)
+               float *tail = nullptr, long tail_draws = 0);
 // log|det| of unplanned FP32 draws (levels off, d_p above the tensor-core path's) by a
 // cluster of blocks per draw, where scratch holds only `slabs` matrices (d_p x d_p).
 // false: not launched (sizes for which launch_lu is the better choice, or no cluster fits).

@@ -1834,12 +1834,8 @@ __device__ __forceinline__ void block_multipliers_rest(T *Lp, const T *D, int Rg
   __syncthreads();
 }
 
-// What k_lu<float, true, kFront> leaves of a draw to k_lu_small<true>: the last 128 x 128 of
-// the core after the panels before (column-major), then whether a check failed.
 constexpr int kSmallMaxDp = 128;
-constexpr size_t kTailElems = (size_t)kSmallMaxDp * kSmallMaxDp + 32;
-// ... for so many draws at a time: 1 GiB, one part up to 16 384 draws
-constexpr long kTailDraws = 16384;
+static_assert(kTailElems == (size_t)kSmallMaxDp * kSmallMaxDp + 32, "");
 
 // TC: trailing updates on the tensor cores (FP32 draws, d_p <= 224); a separate
 // instantiation, so that the FFMA path's register tiles do not weigh on it.
@@ -3279,31 +3275,20 @@ LuPlan plan_lu(int m, int P, long n, int num_sms, int core_n, int nv, int n_solv
     if (opt.max_grid > 0) pl.small_grid = std::min(pl.small_grid, opt.max_grid);
     pl.small_grid = (int)std::min<long>(pl.small_grid, n);
   }
-  // larger ones on the tensor cores: the last 128 rows by k_lu_small<true>, from slabs
-  // behind k_lu's (16 systems of m = 20 .. 400, 10 000 draws each, whole steps: 37.9 ms
-  // without, 30.6 ms with the split)
-  pl.tail_draws = 0;
-  if (pl.tc && pl.vals_smem && pl.dp > kSmallMaxDp) {
-    pl.small_smem = SmallSmem(0, 0).total;
-    pl.tail_grid = num_sms * 4;
-    if (opt.max_grid > 0) pl.tail_grid = std::min(pl.tail_grid, opt.max_grid);
-    pl.tail_draws = (int)std::min<long>(n, kTailDraws);
-  }
   long grid = (long)num_sms * ctas_per_sm;
   if (opt.max_grid > 0 && grid > opt.max_grid) grid = opt.max_grid;
   if (grid > n) grid = n;
   if (grid < 1) grid = 1;
   pl.grid = (int)grid;
   pl.scratch_elems_per_cta = (size_t)pl.dp * pl.dp + (((size_t)nv + 3) / 4) * 4;
-  size_t total = pl.scratch_elems_per_cta * pl.grid;
-  if (pl.tail_draws > 0) {
-    // (no fewer draws than one per resident block: with those the split gains nothing)
-    if (n > pl.grid) {
-      pl.tail_offset = (total + 31) / 32 * 32;
-      total = pl.tail_offset + (size_t)pl.tail_draws * kTailElems;
-    } else {
-      pl.tail_draws = 0;
-    }
+  const size_t total = pl.scratch_elems_per_cta * pl.grid;
+  // larger ones on the tensor cores: the last 128 rows by k_lu_small<true> (16 systems of
+  // m = 20 .. 400, 10 000 draws each, whole steps: 37.9 ms without, 30.6 ms with the split);
+  // no fewer draws than one per resident block: with those the split gains nothing
+  if (pl.tc && pl.vals_smem && pl.dp > kSmallMaxDp && n > pl.grid) {
+    pl.small_smem = SmallSmem(0, 0).total;
+    pl.tail_grid = num_sms * 4;
+    if (opt.max_grid > 0) pl.tail_grid = std::min(pl.tail_grid, opt.max_grid);
   }
   // the redo needs the dense core and the value slots, or a full m_p x m_p slab,
   // per CTA; it shares the slab array, which grows to one slab per SM for it
@@ -3322,7 +3307,8 @@ int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &e
                const unsigned *sp, const T *theta, const T *theta_g, T *scratch,
                double *logdet, int *draw_flags,
                const double *x, const T *lambda, RngKey key, bool refine, double *y,
-               GammaRows rows, const double *nu_in, int *pivot_list, const int *draw_list, int *next) {
+               GammaRows rows, const double *nu_in, int *pivot_list, const int *draw_list, int *next,
+               float *tail, long tail_draws) {
   // opt in to exactly the shared memory this plan needs (a failure here shows up
   // as a launch error that the engine reports)
   auto run = [&](auto kernel) {
@@ -3342,14 +3328,20 @@ int launch_lu(cudaStream_t s, const LuPlan &pl, long n, const EliminationPlan &e
                                                             draw_flags, pivot_list, ep.core_n, nullptr, 0, 0, next);
       return 1;
     }
-    if (pl.tail_draws > 0 && n > pl.grid && !x && !draw_list && theta_g && pivot_list && next) {
+    // Fewer than four draws per resident block at a time cost more in starting and draining
+    // blocks than the split gains: 10 000 draws at m = 400 (304 blocks) in parts of 10 000,
+    // 5 000, 2 500, 1 667, 1 250, 1 000 and 715 2.91, 3.02, 3.18, 3.36, 3.61, 3.69 and
+    // 4.03 ms, 3.75 ms by one kernel; at m = 290 1.38, 1.45, 1.61, 1.68, 1.86, 1.81 and 2.05,
+    // 1.86 ms.
+    tail_draws = std::min<long>(tail_draws, kTailDraws);
+    if (pl.tail_grid > 0 && tail && (tail_draws >= n || tail_draws >= 4L * pl.grid) && !x && !draw_list &&
+        theta_g && pivot_list && next) {
       auto *front = k_lu<T, true, kFront>;
       auto *rest = k_lu_small<true>;
       cudaFuncSetAttribute(front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
       cudaFuncSetAttribute(rest, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.small_smem);
-      float *tail = scratch + pl.tail_offset;
       // equal parts of at most tail_draws
-      const long parts = (n + pl.tail_draws - 1) / pl.tail_draws, per = (n + parts - 1) / parts;
+      const long parts = (n + tail_draws - 1) / tail_draws, per = (n + parts - 1) / parts;
       for (long first = 0; first < n; first += per) {
         const long count = std::min(per, n - first);
         if (first > 0) cudaMemsetAsync(next, 0, 2 * sizeof(int), s);
@@ -3447,12 +3439,12 @@ template int launch_lu<float>(cudaStream_t, const LuPlan &, long, const Eliminat
                                const unsigned *, const float *, const float *, float *,
                                double *, int *,
                                const double *, const float *, RngKey, bool, double *, GammaRows,
-                               const double *, int *, const int *, int *);
+                               const double *, int *, const int *, int *, float *, long);
 template int launch_lu<double>(cudaStream_t, const LuPlan &, long, const EliminationPlan &,
                                 const unsigned *, const double *, const double *, double *,
                                 double *, int *,
                                 const double *, const double *, RngKey, bool, double *,
-                                GammaRows, const double *, int *, const int *, int *);
+                                GammaRows, const double *, int *, const int *, int *, float *, long);
 template void launch_forecast_nu<float>(cudaStream_t, int, int, long, GammaRows, const float *,
                                         const double *, const float *, const float *, RngKey,
                                         double *);
