@@ -800,7 +800,13 @@ int replan_sim(sgdlm_engine *h) {
   int st = plan_sim(h, (long)h->nsim, &pl);
   if (st) return st;
   if (pl.scratch_elems_total * h->tsize() > h->lu_scratch.count) {
-    CK(h->lu_scratch.alloc(pl.scratch_elems_total * h->tsize()));
+    h->lu_tail.release();  // taken again below where there is room
+    const cudaError_t e = h->lu_scratch.alloc(pl.scratch_elems_total * h->tsize());
+    if (e != cudaSuccess) {
+      (void)cudaGetLastError();
+      release_sim(h);  // (no kernel may run without its scratch)
+      return h->cuda_fail(e, "the LU's scratch for a new plan");
+    }
   }
   h->plan = pl;
   place_tail(h);

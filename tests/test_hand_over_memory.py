@@ -14,6 +14,7 @@ from gpusgdlm_gb300.sgdlm import _pd
 
 pytestmark = pytest.mark.gpu
 
+SIM_NOT_INIT, OUT_OF_MEMORY = 4, 8  # status codes of include/sgdlm.h
 M, KMAX, SLAB = 275, 17, 4 * (128 * 128 + 32)
 
 
@@ -120,3 +121,18 @@ def test_the_buffer_goes_first(built_lib):
         got, _ = _log_dets(s, wl, large)
         s.close()
     np.testing.assert_array_equal(got, want)
+
+
+def test_plan_without_memory(built_lib):
+    """A plan whose scratch cannot be had gives the simulation memory back; with memory it
+    is set up anew."""
+    n = 310
+    s, wl = _engine()
+    want, _ = _log_dets(s, wl, n)
+    with _hold(8 << 20):  # (no levels: 288 x 288 values per block, 100 MB)
+        assert s._lib.sgdlm_set_elimination_levels(s._h, 0) == OUT_OF_MEMORY
+        assert s.nsim == 0
+        assert s._lib.sgdlm_compute_vb_posterior(s._h, None, None, None, None, None, None) == SIM_NOT_INIT
+    got, _ = _log_dets(s, wl, n)
+    np.testing.assert_allclose(got, want, rtol=0, atol=1e-4)  # another elimination order
+    s.close()
