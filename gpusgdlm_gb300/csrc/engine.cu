@@ -35,7 +35,7 @@
 #include "elimination.hpp"
 #include "kernels.hpp"
 #include "proposal.hpp"
-#include "rng.cuh"
+#include "trig_log.hpp"
 
 using namespace sgdlm;
 
@@ -684,34 +684,6 @@ int plan_sim(sgdlm_engine *h, long n, LuPlan *out) {
   }
   *out = pl;
   return SGDLM_OK;
-}
-
-// The table of rng.cuh's FP64 logarithm, sine and cosine.
-std::vector<double> trig_log_table() {
-  std::vector<double> t(kTabSize, 0.0);
-  const long double pi = acosl(-1.0L), grid = ldexpl(1.0L, 42);
-  const long double ln2 = logl(2.0L), ln2_hi = kLn2Hi;
-  for (int i = 0; i < 1024; ++i) {
-    const long double a = 2.0L * pi * i / 1024.0L;
-    t[2 * i] = i % 512 == 256 ? 0.0 : (double)cosl(a);
-    t[2 * i + 1] = i % 512 == 0 ? 0.0 : (double)sinl(a);
-  }
-  for (int j = 0; j < kLogIntervals; ++j) {
-    long double c = 1.0L + (j + 0.5L) / kLogIntervals;
-    if (j >= kLogIntervals / 2) c *= 0.5L;
-    if (j == 0 || j == kLogIntervals - 1) c = 1.0L;
-    const double inv = (double)(1.0L / c);
-    const long double l = -logl((long double)inv), hi = roundl(l * grid) / grid;
-    double *e = &t[kTabLog + 4 * j];
-    e[0] = inv;
-    e[1] = (double)hi;
-    e[2] = (double)(l - hi);
-  }
-  for (int k = 0; k < 34; ++k) {
-    t[kTabLn2 + 2 * k] = (double)(-k * ln2_hi);
-    t[kTabLn2 + 2 * k + 1] = (double)(-k * (ln2 - ln2_hi));
-  }
-  return t;
 }
 
 // Where launch_lu hands the last rows of a core over (plan.tail_grid > 0): a buffer of its

@@ -35,7 +35,7 @@ enum : int {
 struct RngKey {
   uint32_t k0, k1, epoch;
   const uint32_t *dev_epoch;
-  const double *tab;  // table of the FP64 logarithm, sine and cosine (rng.cuh); FP64 draws
+  const double *tab;  // table of the FP64 logarithm, sine and cosine (trig_log.hpp); FP64 draws
 };
 
 // Advances the device-side epoch counter by `delta` (fused step).

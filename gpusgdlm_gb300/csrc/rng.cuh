@@ -14,6 +14,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "trig_log.hpp"
+
 namespace sgdlm {
 
 enum : uint32_t {
@@ -86,86 +88,8 @@ template <> struct Uniform<float> {
   }
 };
 
-// ---- FP64 logarithm, sine and cosine by table -----------------------------------
-// FP64 is the narrow pipe of this GPU: a warp's log() costs about 30 FMA slots,
-// sincospi() about 26, and a FP64 draw takes one of each per two normals and three
-// logarithms per gamma.  Table-driven reductions (P. T. P. Tang, "Table-driven
-// implementation of the logarithm function in IEEE floating-point arithmetic", ACM
-// TOMS 16, 1990, and the same idea with the angle-addition formulas) leave short
-// polynomials: 12 and 14 FMA slots, the uniforms' bits taken by integer operations.
-//   log: x = 2^k m, m in [3/4, 3/2), m = (1 + f) / inv with inv from 256 intervals
-//     (|f| <= 2^-8; inv = 1 for the two intervals beside 1, so that log is accurate
-//     relative to its size there), log x = k log 2 + log(1 / inv) + log1p(f), the
-//     constants in two parts, the upper one a multiple of 2^-42 (sums of upper parts
-//     are exact).  Error below 0.8 ulp (log(): 0.54 ulp).
-//   sin, cos of 2 pi u: the nearest of 1024 angles plus a rest of at most pi / 1024.
-//     Absolute error below 1.12e-16 (sincospi(): 1.29e-16).
-// 10 000 draws: the sampler 1084 -> 609 us at m = 100, 5.88 -> 3.3 ms at m = 400 (576 us at
-// m = 100 since pairs of normals beyond p_j are left out).
-// The table (trig_log_table, engine.cu) is 25 KB and read through L1.
-//   [0, 2048): cos, sin of 2 pi i / 1024; [2048, 3072): inv, upper and lower part of
-//   log(1 / inv), 0; [3072, 3140): upper and lower part of -k log 2, k = 0 .. 33.
-constexpr int kLogIntervals = 256;
-constexpr int kTabLog = 2048, kTabLn2 = kTabLog + 4 * kLogIntervals, kTabSize = kTabLn2 + 2 * 34;
-constexpr double kLn2Hi = 0x1.62e42fefa38p-1;  // log 2 rounded to a multiple of 2^-42
-
-// log1p(f) + log(1 / inv_j) + (khi + klo) for mantissa bits `frac` (52 bits) of a
-// value in [1, 2); the value is halved in the upper half of the intervals.
-__device__ __forceinline__ double log_reduced(uint64_t frac, const double *tab, double khi,
-                                              double klo) {
-  const int j = (int)(frac >> 44);
-  const uint64_t ex = j >= kLogIntervals / 2 ? 0x3FEull : 0x3FFull;
-  const double m = __longlong_as_double((long long)((ex << 52) | frac));
-  const double2 t0 = __ldg(reinterpret_cast<const double2 *>(tab + kTabLog + 4 * j));
-  const double lo = __ldg(tab + kTabLog + 4 * j + 2);
-  const double f = fma(m, t0.x, -1.0);
-  double q = 1.0 / 7.0;
-  q = fma(q, f, -1.0 / 6.0);
-  q = fma(q, f, 1.0 / 5.0);
-  q = fma(q, f, -1.0 / 4.0);
-  q = fma(q, f, 1.0 / 3.0);
-  q = fma(q, f, -1.0 / 2.0);
-  const double p = fma(f * f, q, f);
-  return (khi + t0.y) + (p + (klo + lo));
-}
-// log((a + 1/2) 2^-32)
-__device__ __forceinline__ double log_uniform(uint32_t a, const double *tab) {
-  const uint64_t v = 2ull * a + 1ull;  // u = v 2^-33
-  const int lz = __clzll((long long)v);
-  const uint64_t frac = (v << lz >> 11) & 0x000FFFFFFFFFFFFFull;
-  // u = 2^(30 - lz) (1 + frac), the exponent one higher where the mantissa is halved
-  const int k = lz - 30 - (int)(frac >> 51);
-  const double2 kk = __ldg(reinterpret_cast<const double2 *>(tab + kTabLn2 + 2 * k));
-  return log_reduced(frac, tab, kk.x, kk.y);
-}
-// log(x) for any x (the library's for zero, subnormal, negative and non-finite ones)
-__device__ __forceinline__ double log_table(double x, const double *tab) {
-  const uint64_t b = (uint64_t)__double_as_longlong(x);
-  const int ex = (int)(b >> 52);
-  if (ex < 1 || ex > 2046) return log(x);
-  const uint64_t frac = b & 0x000FFFFFFFFFFFFFull;
-  const double k = (double)(ex - 1023 + (int)(frac >> 51));
-  const double lo = __ldg(tab + kTabLn2 + 3);  // of -log 2
-  return log_reduced(frac, tab, k * kLn2Hi, -k * lo);
-}
-// sin and cos of 2 pi (b + 1/2) 2^-32
-__device__ __forceinline__ void sincos_uniform(uint32_t b, const double *tab, double &s, double &c) {
-  const uint64_t v = 2ull * b + 1ull;  // the angle in units of 2 pi 2^-33
-  const uint32_t i = (uint32_t)((v + (1u << 22)) >> 23);
-  const int64_t d = (int64_t)v - ((int64_t)i << 23);  // |d| <= 2^22
-  const double2 t0 = __ldg(reinterpret_cast<const double2 *>(tab) + (i & 1023u));
-  // d as a double: added into the low bits of 1.5 2^52
-  const double x = (__longlong_as_double(0x4338000000000000ll + d) - 0x1.8p52) *
-                   7.3145903963357981e-10;  // 2 pi 2^-33
-  const double t = x * x;
-  const double sx = fma(t * x, fma(t, 1.0 / 120.0, -1.0 / 6.0), x);
-  const double cm = t * fma(t, 1.0 / 24.0, -0.5);
-  c = t0.x + fma(-t0.y, sx, t0.x * cm);
-  s = t0.y + fma(t0.x, sx, t0.y * cm);
-}
-
 // Box-Muller (1958): two uniforms -> two independent standard normals.  tab: the
-// FP64 table (not read for FP32).
+// table of trig_log.hpp (FP64; not read for FP32).
 template <typename T>
 __device__ __forceinline__ void box_muller(uint32_t a, uint32_t b, T &z0, T &z1, const double *tab);
 
