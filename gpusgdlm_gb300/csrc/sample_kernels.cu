@@ -320,6 +320,10 @@ __global__ void __launch_bounds__(kSampleThreads)
       for (int k = 0; k < PMAX; ++k)
         if (k < P) row[k] = g[k];
     }
+    // an inactive coefficient's sum: U_W's zeros times omega, NaN where omega is not finite
+    T zeros = T(0);
+#pragma unroll
+    for (int l = 0; l < PMAX; ++l) zeros += T(0) * w[l];
     constexpr int W = VEC ? V16<T>::W : 1;
 #pragma unroll
     for (int k = 0; k < PMAX; k += W) {
@@ -331,7 +335,7 @@ __global__ void __launch_bounds__(kSampleThreads)
           o[0] = row[k];
 #pragma unroll
         for (int b = 0; b < W; ++b) {
-          T acc = T(0);
+          T acc = zeros;
           if (k + b < na) acc = column_dot<T, VEC>(Us, P, k + b, w);
           o[b] = acc + o[b];
         }
