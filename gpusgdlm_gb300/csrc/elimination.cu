@@ -387,9 +387,10 @@ LogdetPlanHost plan_logdet(int m, int P, const std::vector<unsigned> &sp, int ma
     if (nv > max_slots || nv > kMaxSlots || pl.terms.size() > kMaxTermWords) return LogdetPlanHost{};
     pl.n_terms += list.size();
     // entries by decreasing term count (stable), 32 to a chunk
-    std::vector<int> ord(cell.size()), place(cell.size());
-    for (size_t k = 0; k < ord.size(); ++k) ord[k] = (int)k;
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return count[a] > count[b]; });
+    std::vector<int> ord(cell.size()), place(cell.size()), at_count(S.size() + 2, 0);
+    for (int c : count) ++at_count[S.size() - (size_t)c + 1];  // (a term per pivot at most)
+    for (size_t c = 1; c < at_count.size(); ++c) at_count[c] += at_count[c - 1];
+    for (size_t k = 0; k < ord.size(); ++k) ord[at_count[S.size() - (size_t)count[k]]++] = (int)k;
     for (size_t c0 = 0; c0 < ord.size(); c0 += 32) {
       const size_t tofs = pl.terms.size();
       pl.terms.resize(tofs + 32 * (size_t)count[ord[c0]], pack16(kSlotZero, kSlotZero));
