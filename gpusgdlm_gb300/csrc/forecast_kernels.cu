@@ -14,9 +14,13 @@
 //     kMaxSweeps, then one correction d; max|d| <= 1e-3 max|y| (the rule the
 //     factorising path applies to its refinement step); y + d is written.
 //   FP64 draws: y, nu and the residual's Gamma entries are FP64, and corrections
-//     are added until one is at most 2^-36 max|y| (usually the second).  A
-//     correction is right to about 2^-19 of its size, so what is left is below the
-//     rounding of y itself: the result is as good as a solve with FP64 factors.
+//     are added until one is, in every row, at most 2^-36 of the row's size
+//     |nu_r| + sum |gamma_rq y_q| (usually the second).  The sweeps settle every row to
+//     2^-20 of its size too, so a correction is right to about 2^-19 of its own and what is
+//     left is below the rounding of y itself, also in series far smaller than the largest
+//     (measured against max|y| alone, as FP32 draws are, a block of series 10^-8 as large
+//     and slower to converge was left with errors of 10^-10 of its size, for 5 to 12 % less
+//     time): the result is as good as a solve with FP64 factors.
 // Any other draw (slow or no convergence: spectral radius near or above one,
 // non-finite values) is appended to `list` and solved by the LU kernels
 // (partial pivoting where needed).
@@ -51,7 +55,8 @@ constexpr float kSweepTol = 9.5367431640625e-07f;   // 2^-20
 constexpr float kCorrSweepTol = 9.765625e-04f;      // 2^-10
 constexpr double kCorrTol = 1e-3;
 constexpr int kCorrBits = 20;                         // bits a correction adds
-constexpr double kDoneTol = 1.4551915228366852e-11;  // 2^-36: FP64 draws' last correction
+constexpr double kDoneTol = 1.4551915228366852e-11;  // 2^-36: FP64 draws' last correction, per row
+constexpr double kUnevenTol = 2.220446049250313e-16;  // 2^-52: the same where not all rows settled
 constexpr int kMaxCorrections = 4;                    // FP64 draws
 
 struct JacSmem {
@@ -143,6 +148,8 @@ __device__ __forceinline__ void block_max(unsigned (&a)[NB], unsigned (&b)[NB], 
   set = set_after(set);
 }
 
+constexpr unsigned kTopBit = 0x80000000u;
+
 // The thread's row in ELL form held in registers: K slots (entries beyond the row's
 // length have value 0 and point at the row itself), the column indices packed two
 // to a register, NB draws' values.
@@ -155,27 +162,32 @@ template <int K, int NB> struct Row {
 };
 
 // Sweeps x <- c + Gamma x from x = c over this thread's row r, for the draws in
-// `todo` (a mask).  Returns the mask of the draws that converged (max|dx| <= tol
-// max|x|, everything finite); x receives the row's last iterate of each draw, which
-// stops there while the others go on.  wlen: the longest row of this warp, rounded
+// `todo` (a mask).  Returns the mask of the draws that converged (everything finite, and
+// max|dx| <= tol max|x|); x receives the row's last iterate of each draw, which
+// stops there while the others go on.  ROWS: a draw goes on until |dx_r| <= tol size_r in
+// every row, size_r = |c_r| + sum |gamma_rq x_q| (`size`), or to the last sweep: a row whose
+// terms nearly cancel in a neighbour may stay above that by the neighbour's rounding (one
+// draw in 10^4); `even`: the draws whose rows have all come there.  wlen: the longest row of this warp, rounded
 // up to even (warp-uniform): slots beyond it are padding in every row of the warp
 // (value 0, so skipping them leaves every sum unchanged).  Ends on a barrier; xa and
 // xb are free on entry and after it.
-template <int K, int NB>
+template <int K, int NB, bool ROWS>
 __device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row<K, NB> &R,
                                            const float (&c)[NB], float *xa, float *xb,
                                            unsigned *red, int &set, float tol, unsigned todo,
-                                           float (&x)[NB]) {
+                                           float (&x)[NB], float (&size)[NB], unsigned &even) {
   unsigned conv = 0;
+  even = 0;
 #pragma unroll
   for (int b = 0; b < NB; ++b) x[b] = c[b];
   if (mine) st_row<NB>(xa, r, x);
   __syncthreads();
   float *cur = xa, *nxt = xb;
   for (int it = 1; it <= kMaxSweeps && todo; ++it) {
-    float a0[NB], a1[NB];
+    const bool check = (it & 3) == 0;
+    float a0[NB], a1[NB], sz[NB];
 #pragma unroll
-    for (int b = 0; b < NB; ++b) a0[b] = c[b], a1[b] = 0.f;
+    for (int b = 0; b < NB; ++b) a0[b] = c[b], a1[b] = 0.f, sz[b] = fabsf(c[b]);
 #pragma unroll
     for (int q = 0; q < K; q += 2) {
       if (q >= wlen) break;
@@ -186,6 +198,10 @@ __device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row
       for (int b = 0; b < NB; ++b) {
         a0[b] = fmaf(R.val[b][q], u[b], a0[b]);
         a1[b] = fmaf(R.val[b][q + 1], v[b], a1[b]);
+        if (ROWS && check) {
+          sz[b] = fmaf(fabsf(R.val[b][q]), fabsf(u[b]), sz[b]);
+          sz[b] = fmaf(fabsf(R.val[b][q + 1]), fabsf(v[b]), sz[b]);
+        }
       }
     }
 #pragma unroll
@@ -194,13 +210,19 @@ __device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row
     float *t = cur;
     cur = nxt;
     nxt = t;
-    const bool check = (it & 3) == 0;
     unsigned dk[NB], xk[NB];
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       const bool live = mine && (todo >> b & 1);
       if (check) {
-        dk[b] = live ? key_of(a0[b] - x[b]) : 0u;
+        if (ROWS) {
+          // a row above its bound: the top bit (magnitudes lie below it)
+          const float d = a0[b] - x[b];
+          dk[b] = live ? key_of(d) | (fabsf(d) <= tol * sz[b] ? 0u : kTopBit) : 0u;
+          if (live) size[b] = sz[b];
+        } else {
+          dk[b] = live ? key_of(a0[b] - x[b]) : 0u;
+        }
         xk[b] = live ? key_of(a0[b]) : 0u;
       }
       if (live) x[b] = a0[b];
@@ -213,7 +235,11 @@ __device__ __forceinline__ unsigned jacobi(bool mine, int r, int wlen, const Row
         if (!(todo >> b & 1)) continue;
         if (!(xmax < INFINITY)) {
           todo &= ~(1u << b);
-        } else if (__uint_as_float(dk[b]) <= tol * xmax) {
+        } else if (ROWS && dk[b] < kTopBit) {
+          todo &= ~(1u << b);
+          conv |= 1u << b;
+          even |= 1u << b;
+        } else if ((!ROWS || it == kMaxSweeps) && __uint_as_float(dk[b] & ~kTopBit) <= tol * xmax) {
           todo &= ~(1u << b);
           conv |= 1u << b;
         }
@@ -270,12 +296,13 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
       for (int q = 0; q < K; ++q) R.val[b][q] = (b < nd && q < len) ? (float)th[q] : 0.f;
       nud[b] = (mine && b < nd) ? nu[(size_t)r * n + i0 + b] : 0.0;
     }
-    float c[NB], x[NB], yo[NB];
+    float c[NB], x[NB], yo[NB], size[NB] = {};
+    unsigned even;
     unsigned ka[NB], kb[NB];
     if constexpr (sizeof(T) == 4) {
 #pragma unroll
       for (int b = 0; b < NB; ++b) c[b] = (float)nud[b];
-      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, ok, yo);
+      ok = jacobi<K, NB, false>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, ok, yo, size, even);
       if (ok) {
         // residual in FP64 and its correction by the same iteration.  The iterates are
         // widened once per row, the Gamma entries without the conversion instruction
@@ -312,7 +339,8 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) c[b] = (float)v[b];
-        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kCorrSweepTol, ok, x);
+        const unsigned conv =
+            jacobi<K, NB, false>(mine, r, wlen, R, c, xa, xb, red, set, kCorrSweepTol, ok, x, size, even);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           ka[b] = mine ? key_of(x[b]) : 0u;
@@ -349,8 +377,9 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
         if (sc) nud[b] *= __hiloint2double((1023 - e) << 20, 0);
         c[b] = (float)nud[b];
       }
-      ok = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, ok, yo);
+      ok = jacobi<K, NB, true>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, ok, yo, size, even);
       unsigned todo = ok;
+      float csize[NB] = {};  // (a correction's)
 #pragma unroll
       for (int b = 0; b < NB; ++b) out[b] = (double)yo[b];
       double up = 1.0, down = 1.0;
@@ -373,24 +402,29 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
         }
 #pragma unroll
         for (int b = 0; b < NB; ++b) c[b] = (float)(v[b] * up);
-        const unsigned conv = jacobi<K, NB>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, todo, x);
+        const unsigned conv =
+            jacobi<K, NB, true>(mine, r, wlen, R, c, xa, xb, red, set, kSweepTol, todo, x, csize, even);
         ok &= ~(todo & ~conv);
         todo &= conv;
+        // the top bit of ka: a row whose correction is not yet small against its own size;
+        // ka is then the largest such row's
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
           if (todo >> b & 1) out[b] += (double)x[b] * down;
-          ka[b] = mine ? key_of(x[b]) : 0u;
+          const float done = (float)((even >> b & 1 ? kDoneTol : kUnevenTol) * up);
+          ka[b] = mine ? key_of(x[b]) | (fabsf(x[b]) <= done * size[b] ? 0u : kTopBit) : 0u;
           kb[b] = mine ? key_of((float)out[b]) : 0u;
         }
         block_max<NB>(ka, kb, red, set);
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
-          const double dmax = (double)__uint_as_float(ka[b]) * down, ymax = (double)__uint_as_float(kb[b]);
+          const double dmax = (double)__uint_as_float(ka[b] & ~kTopBit) * down,
+                       ymax = (double)__uint_as_float(kb[b]);
           if (!(todo >> b & 1)) continue;
           if (!(ymax < INFINITY && dmax <= kCorrTol * ymax)) {
             ok &= ~(1u << b);
             todo &= ~(1u << b);
-          } else if (dmax <= kDoneTol * ymax) {
+          } else if (ka[b] < kTopBit) {
             todo &= ~(1u << b);
           }
         }

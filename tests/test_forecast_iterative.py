@@ -98,3 +98,58 @@ def test_fp32_two_blocks_per_sm(built_lib, m, kmax, mean):
     err = np.abs(y - ref).max(axis=0) / np.abs(ref).max(axis=0)
     assert err.max() <= 1e-8
     s.close()
+
+
+@pytest.mark.parametrize("m,kmax,n,scale,own", [
+    (40, 4, 300, 1e-6, 0.1), (100, 6, 2000, 1e-8, 0.12), (400, 8, 320, 1e-5, 0.1), (540, 5, 100, 1e-7, 0.1)])
+def test_fp64_series_of_different_scales(built_lib, m, kmax, n, scale, own):
+    """Half of the series are `scale` as large as the others, depend on each other only and
+    converge more slowly: their forecasts are as exact as the large ones'.  Error of each
+    value against the size of the terms it is the sum of, |nu_r| + sum |gamma_rq y_q|; the
+    bound is the file's 1e-12."""
+    half = m // 2
+    rng = np.random.default_rng(m)
+    P = kmax + 1
+    sp = np.full((P, m), 2147483648, dtype=np.uint32, order="F")
+    a = np.zeros((P, m))
+    for j in range(m):
+        block = np.arange(half) if j < half else np.arange(half, m)
+        sp[1:, j] = j + m * rng.choice(block[block != j], size=kmax, replace=False)
+        a[1:, j] = rng.uniform(-0.01, 0.01, kmax) if j < half else own * rng.choice([0.7, 1.0], kmax)
+    s = SGDLM(1, strict=True, precision="fp64")
+    s.setSimultaneousParents(np.full(m, P), np.where(sp >= m * m, np.nan, sp).astype(float))
+    s.setDiscountFactors(np.full(m, 0.97), np.full((P, P, m), 0.98))
+    s.setPriorParameters(a, np.repeat((1e-8 * np.eye(P))[:, :, None], m, axis=2), np.full(m, 20.0),
+                         np.where(np.arange(m) < half, 1.0, scale**2))
+    x = np.zeros((P, m))
+    wl = dict(P=P)
+    y = _forecast(s, wl, n, x, True)
+    assert s.getStats()["forecast_draws_factored"] == 0
+    th = s.getDraws()["thetas"]
+    ref = _forecast(s, wl, n, x, False)
+    G = np.zeros((n, m, m))
+    for j in range(m):
+        G[:, j, sp[1:, j] // m] = th[1:, j, :].T
+    nu = np.abs(ref.T - np.einsum("irq,qi->ir", G, ref))
+    size = nu + np.einsum("irq,qi->ir", np.abs(G), np.abs(ref))
+    assert (np.abs(y - ref).T / size).max() <= 1e-12
+    s.close()
+
+
+def test_fp64_rows_that_cancel(built_lib):
+    """Rows whose terms nearly cancel in a neighbour do not send a draw to the LU: the
+    bench's kind of system, 40 000 draws (one in 10 000 has such a row), against the
+    factored solves."""
+    m, n = 60, 40000
+    s, wl = _engine(m, 17, "fp64")
+    P = wl["P"]
+    rng = np.random.default_rng(8)
+    s.setPriorParameters(rng.normal(0, 0.06, size=(P, m)), np.repeat((1e-4 * np.eye(P))[:, :, None], m, axis=2),
+                         np.full(m, 20.0), np.full(m, 1.0))
+    x = wl["F_of"](2, False)
+    y = _forecast(s, wl, n, x, True)
+    assert s.getStats()["forecast_draws_factored"] == 0
+    ref = _forecast(s, wl, n, x, False)
+    err = np.abs(y - ref).max(axis=0) / np.abs(ref).max(axis=0)
+    assert err.max() <= 1e-12
+    s.close()
