@@ -25,17 +25,15 @@
 // non-finite values) is appended to `list` and solved by the LU kernels
 // (partial pivoting where needed).
 //
-// A block solves NB = 2 draws at a time, their iterates side by side in shared
-// memory: one gather of two floats, one column index and one barrier per sweep serve
-// both.  The sweeps are bound by the gathers' shared-memory wavefronts (bank
-// conflicts: 32 scattered 4-byte loads take about 3.5, two 16-lane phases of 8-byte
-// loads about 6 for two draws) and by issue slots.  10 000 FP32 draws at m = 400: one
-// draw per block 908 us, two 833 us, four 949 us (one block per SM each); two with the
-// registers cut to 72 a thread, so that two blocks share an SM and one sweeps while the
-// other waits at its barrier (K <= 20, a few spilled words outside the sweeps), 758 us;
-// and with the residual's conversions to FP64, three FP64-rate instructions per entry
-// before, down to one, 628 us.  FP64 draws: two 1.52 ms, four 1.87 ms, and 94.5 ms with
-// FP64 factors.
+// The sweeps are bound by the gathers' shared-memory wavefronts (bank conflicts: 32
+// scattered 4-byte loads take about 3.5), by the barrier of each sweep and by issue slots;
+// so several blocks share an SM, and some sweep while others wait.  Where it is faster
+// (two_draws) a block solves NB = 2 FP32 draws at a time, their iterates side by side in
+// shared memory: one gather of two floats (two 16-lane phases: about 6 wavefronts for two
+// draws), one column index and one barrier per sweep serve both, with 72 registers a thread
+// for two blocks on an SM.  10 000 FP32 draws at m = 400 (K = 18): 628 us (908 us one by one
+// with the residual's conversions to FP64 at three FP64-rate instructions per entry; they
+// are down to one).  FP64 draws, one per block: 1.5 ms, and 94.5 ms with FP64 factors.
 #include <algorithm>
 
 #include "kernels.hpp"
@@ -459,21 +457,33 @@ __global__ void __launch_bounds__(NB > 1 ? (FULL ? kJacGroupThreads : kJacPairTh
 
 // ELL widths: the smallest of these that holds the longest row
 constexpr int kJacWidths[] = {8, 12, 16, 18, 20, 24, 32};
-// and the widest rows of that form: FP32 kernels fit 72 registers with few spills up to 20;
-// FP64 ones gain up to 12 (m = 100: 231 us, 209 so) and lose beyond (m = 400, 18: 1505, 1525)
-constexpr int kJacPairWidth = 20, kJacPairWidth64 = 12;
+// Two draws per block: FP32 draws, K entries per row,
+//   K <= 8 (m to 448), K <= 18 (m from 385 to 448): the form for two blocks on an SM;
+//   K >= 24 (m to 512): one block with 128 registers per thread;
+// elsewhere one draw per block, of which the 64 registers per thread leave room for more
+// blocks.  Time of two draws per block to that of one, 10 000 draws (3 000, 40 000 alike):
+//   K = 8: m = 33 0.97, 64 1.09, 100 0.98, 133 0.98, 200 0.98, 300 0.91, 448 0.93, 500 1.16;
+//   12: m = 64 1.16, 100 1.05, 180 1.12, 256 1.04, 300 1.09, 400 0.98, 448 0.97;
+//   16: 100 1.05, 200 0.99, 300 1.06, 400 0.99, 448 1.00; 18: 250 1.08, 300 1.13, 350 1.04,
+//   400 1.00, 448 1.01, 500 1.10; 20: 200 1.13, 300 1.16, 400 1.05, 448 1.09;
+//   24: 200 0.97, 300 1.11, 400 0.97, 448 0.95, 500 0.98; 32: 200 0.83, 300 1.02, 400 0.87,
+//   500 0.75.  FP64 draws: 1.00 to 1.27 (m = 33 .. 500, K = 8 .. 24), so one.
+template <typename T> bool two_draws(int K, int threads) {
+  if (sizeof(T) == 8 || threads > kJacGroupThreads) return false;
+  return K >= 24 || (threads <= kJacPairThreads && (K <= 8 || (K <= 18 && threads > 384)));
+}
 
 // Calls f with the kernel of type T, width K and draws per block (group: two).
-template <typename T, typename F> void with_jacobi_kernel(int K, bool group, int threads, F f) {
-  constexpr int pair_width = sizeof(T) == 4 ? kJacPairWidth : kJacPairWidth64;
-#define SGDLM_JACOBI(KK)                                                           \
-  case KK:                                                                         \
-    if (group && threads <= kJacPairThreads && KK <= pair_width)                    \
-      f(k_forecast_jacobi<T, KK, 2, (KK > pair_width)>, 2);                        \
-    else if (group)                                                                \
-      f(k_forecast_jacobi<T, KK, 2, true>, 2);                                     \
-    else                                                                           \
-      f(k_forecast_jacobi<T, KK, 1, true>, 1);                                     \
+template <typename T, typename F> void with_jacobi_kernel(int K, bool group, F f) {
+#define SGDLM_JACOBI(KK)                                          \
+  case KK:                                                        \
+    if constexpr (sizeof(T) == 4 && (KK <= 18 || KK >= 24)) {      \
+      if (group) {                                                \
+        f(k_forecast_jacobi<T, KK, 2, (KK >= 24)>, 2);            \
+        break;                                                    \
+      }                                                           \
+    }                                                             \
+    f(k_forecast_jacobi<T, KK, 1, true>, 1);                      \
     break
   switch (K) {
     SGDLM_JACOBI(8);
@@ -501,10 +511,10 @@ template <typename T> JacobiPlan plan_jacobi(int m, int max_row, int num_sms) {
   jp.threads = (m + 31) / 32 * 32;
   // [0] one draw per block, [1] two
   for (int g = 0; g < 2; ++g) {
-    if (g == 1 && jp.threads > kJacGroupThreads) break;
+    if (g == 1 && !two_draws<T>(jp.nnz, jp.threads)) break;
     int per_sm = 0;
     cudaError_t e = cudaSuccess;
-    with_jacobi_kernel<T>(jp.nnz, g == 1, jp.threads, [&](auto kernel, int nb) {
+    with_jacobi_kernel<T>(jp.nnz, g == 1, [&](auto kernel, int nb) {
       jp.draws[g] = nb;
       jp.smem[g] = JacSmem(m, nb).total;
       if (jp.smem[g] > 48 * 1024)
@@ -529,12 +539,13 @@ template <typename T>
 void launch_forecast_jacobi(cudaStream_t s, const JacobiPlan &jp, int m, long n, GammaRows rows,
                             const T *theta_g, int nnz, const double *nu, double *y,
                             double *logdet, int *list) {
-  // two draws per block once they fill half of the SMs' resident blocks; below that
-  // one draw per block spreads them over more SMs
-  const int g = jp.draws[1] > 0 && n >= (long)jp.grid[1] * jp.draws[1] / 2 ? 1 : 0;
+  // two draws per block (where the plan has them) from two rounds of the resident blocks
+  // on; fewer draws spread over more SMs one by one (m = 400, K = 18, 304 blocks: 304 draws
+  // 51 us one by one, 61 us in twos; 608 74, 76; 912 96, 113; 1 216 116, 117; 2 432 205, 203)
+  const int g = jp.draws[1] > 0 && n >= 2L * jp.grid[1] * jp.draws[1] ? 1 : 0;
   const long blocks = (n + jp.draws[g] - 1) / jp.draws[g];
   const unsigned grid = (unsigned)std::max<long>(std::min<long>(jp.grid[g], blocks), 1);
-  with_jacobi_kernel<T>(jp.nnz, g == 1, jp.threads, [&](auto kernel, int) {
+  with_jacobi_kernel<T>(jp.nnz, g == 1, [&](auto kernel, int) {
     if (jp.smem[g] > 48 * 1024)
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)jp.smem[g]);
     kernel<<<grid, (unsigned)jp.threads, jp.smem[g], s>>>(m, n, rows, theta_g, nnz, nu, y, logdet, list,

@@ -203,7 +203,7 @@ void launch_logdet64(cudaStream_t s, const Logdet64Launch &L, long n, const Logd
 // (forecast_kernels.cu).  ok = 0: every draw keeps the factorising path.
 struct JacobiPlan {
   int ok, threads, nnz;  // threads: m rounded up to 32; nnz: ELL slots per row (8..32)
-  // [0]: one draw per block, [1]: two (draws[1] = 0: not available at this m)
+  // [0]: one draw per block, [1]: two (draws[1] = 0: not where one is faster)
   int draws[2], grid[2];
   size_t smem[2];
   // thread t takes row order[t] (the rows by decreasing length, so that a warp's

@@ -153,3 +153,21 @@ def test_fp64_rows_that_cancel(built_lib):
     err = np.abs(y - ref).max(axis=0) / np.abs(ref).max(axis=0)
     assert err.max() <= 1e-12
     s.close()
+
+
+@pytest.mark.parametrize("m,rows", [(447, 8), (448, 8), (449, 8), (384, 12), (385, 12), (385, 18), (385, 20),
+                                    (510, 24), (512, 30), (513, 30)])
+def test_two_draws_per_block(built_lib, m, rows):
+    """FP32 draws at and beside the sizes where a block takes two: the same bits as a few
+    draws one by one, up to an odd last one."""
+    s, wl = _engine(m, rows, "mixed", seed=m)
+    x = wl["F_of"](2, False)
+    many = _forecast(s, wl, 2501, x, True)
+    assert s.getStats()["forecast_draws_factored"] == 0
+    few = _forecast(s, wl, 5, x, True)
+    np.testing.assert_array_equal(few, many[:, :5])
+    s.setForecastSolver(True)
+    s.setRngState(11, 0)
+    odd = s.computeForecast(2500, 2500, x)
+    np.testing.assert_array_equal(odd, many[:, :2500])
+    s.close()
