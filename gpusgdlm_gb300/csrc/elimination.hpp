@@ -147,9 +147,9 @@ EliminationPlanHost plan_elimination(int m, int P, const std::vector<unsigned> &
 // sub-partition, 19 per SM), so for FP64 draws the plan spends indices to save
 // operations: many more levels, each a set of independent nodes of low Markowitz
 // cost (row count times column count), until the remaining nodes' matrix is nearly
-// dense.  At m = 400 with ~8.5 parents per series that is 1.6e6 multiply-adds per
-// draw (19 levels, 165 dense nodes) instead of the 3.9e6 of four greedy levels and a
-// 224 x 224 core; at m = 100, 8e3 instead of 1e5.  A node's slots are handed on once
+// dense.  At m = 400 with ~8.5 parents per series that is 1.4e6 multiply-adds per
+// draw (18 levels, 154 dense nodes) instead of the 3.8e6 of four greedy levels and a
+// 224 x 224 core; at m = 100, 1.1e4 instead of 9e4.  A node's slots are handed on once
 // it is eliminated (only log|det| is wanted, nothing is solved), so that the live
 // values stay in shared memory.
 //

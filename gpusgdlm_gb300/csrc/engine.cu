@@ -249,8 +249,8 @@ struct sgdlm_engine {
   bool g_stale = false;    // theta_g is not the present parental sets' copy of the draws
   DevBuf<double> logdet, w, y_fc, nu_fc, stats6, wpart, part_a, part_b;
   DevBuf<int> draw_flags, series_flags;
-  // nsim + 2: the work counter of k_logdet64, then the count of the draws flagged for
-  // the redo and their list
+  // nsim + 3: two work counters (k_logdet64's, or the two kernels' of FP32 log|det|), then
+  // the count of the draws flagged for the redo and their list
   DevBuf<int> pivot_list;
   DevBuf<double> mean_m, mean_C, mean_n, mean_s, mean_lambda, mean_log_lambda;
   DevBuf<uint32_t> dev_epoch;

@@ -15,7 +15,7 @@
 // its next draw from a counter: where several engines share the GPU, a block whose SM
 // was held by another engine's kernel starts late and takes fewer (three engines' steps
 // at m = 400 in turn: 62.3 ms a step with a fixed share per block, 56.0 ms).  10 000 draws:
-// m = 400 40.7 ms (76 % of the FP64 pipe; one block per SM, so the panels' columns are
+// m = 400 40.6 ms (68 % of the FP64 pipe; one block per SM, so the panels' columns are
 // not covered), 94.5 ms with four levels and the 224 x 224 core; m = 100 0.46 ms
 // (13.0 ms); m = 200 3.3 ms.  Panels of 16 columns: 45.2 ms at m = 400.
 #include <algorithm>
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 1 : kWarpsPerSm * 32 / NT)
                int *__restrict__ draw_flags, int *__restrict__ pivot_list, int *__restrict__ next) {
   constexpr int NW = NT / 32;
   extern __shared__ __align__(16) double vals[];  // the slots, and the dense part M at m_at
-  __shared__ double prow[2][kW + 1];               // a panel's pivot row (16: its reciprocal)
+  __shared__ double prow[2][kW + 1];               // a panel's pivot row (kW: its reciprocal)
   __shared__ double red_m[NW];
   __shared__ int red_e[NW], red_b[NW];
   __shared__ unsigned s_next;                      // the block's next draw

@@ -145,8 +145,10 @@ int sgdlm_compute_forecast(sgdlm_handle h, double *y_tp1, const double *x_tp1,
 
 /* Copies the current draw buffers to host in the reference's draw-major layouts,
  * lambdas (m x nsim) and thetas (max_p x m x nsim) as in computeForecastDebug
- * (RcppWrapper.cpp:557-569), and the last per-draw log|det(I - Gamma)| (nsim).
- * Any pointer may be NULL. */
+ * (RcppWrapper.cpp:557-569), and the last per-draw log|det(I - Gamma)| (nsim): of
+ * the last VB call's or forecast's draws under the parental sets of that call, NaN
+ * for FP32 forecast draws that the iterative solve did not factor (FP64 ones are
+ * computed here).  Any pointer may be NULL. */
 int sgdlm_get_draws(sgdlm_handle h, double *lambdas, double *thetas, double *log_dets);
 
 /* ---- engine options (no counterpart in the reference's interface) ---- */
