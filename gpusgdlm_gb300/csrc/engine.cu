@@ -691,12 +691,11 @@ int plan_sim(sgdlm_engine *h, long n, LuPlan *out) {
 // the device's memory stay free, so that such buffers of any number of engines hold less
 // than an eighth of it and cost none its memory; else the room behind the Gamma copy
 // (theta_g has m max_p entries per draw: 2 870 draws at a time at m = 400, max_p = 20,
-// 10 000 draws; 3.18 instead of 2.91 ms).
+// 10 000 draws; 3.18 instead of 2.91 ms).  Once taken it stays where it is while the other
+// buffers do: a batch's recorded step holds its address.
 void place_tail(sgdlm_engine *h) {
-  if (h->plan.tail_grid == 0) return;
+  if (h->plan.tail_grid == 0 || h->lu_tail.ptr) return;
   const size_t want = (size_t)std::min<long>((long)h->nsim, kTailDraws) * kTailBytes;
-  if (h->lu_tail.count >= want) return;
-  h->lu_tail.release();
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || free_b < want ||
       free_b - want < total_b / 8 * 7 || h->lu_tail.alloc(want) != cudaSuccess) {
@@ -705,13 +704,10 @@ void place_tail(sgdlm_engine *h) {
   }
 }
 float *tail_room(sgdlm_engine *h, long *draws) {
-  if (h->lu_tail.ptr) {
-    *draws = (long)(h->lu_tail.count / kTailBytes);
-    return reinterpret_cast<float *>(h->lu_tail.ptr);
-  }
   const size_t used = (h->nsim * (size_t)h->g_nnz * sizeof(float) + 127) / 128 * 128;
-  *draws = h->theta_g.count > used ? (long)((h->theta_g.count - used) / kTailBytes) : 0;
-  return reinterpret_cast<float *>(h->theta_g.ptr + used);
+  const size_t behind = h->theta_g.count > used ? h->theta_g.count - used : 0;
+  *draws = (long)(std::max(behind, h->lu_tail.count) / kTailBytes);
+  return reinterpret_cast<float *>(h->lu_tail.count >= behind ? h->lu_tail.ptr : h->theta_g.ptr + used);
 }
 
 int alloc_sim_buffers(sgdlm_engine *h, size_t nsim, const LuPlan &pl) {
@@ -747,6 +743,7 @@ int alloc_sim(sgdlm_engine *h, size_t nsim) {
   // free and allocate gigabytes every call; every buffer is written before it
   // is read within a call
   h->plan = pl;
+  if (nsim > h->logdet.count) h->lu_tail.release();  // more draws than ever: every buffer is replaced
   vb_chunking((long)nsim, (int)m, h->num_sms, &h->chunks, &h->chunk_draws);
   st = alloc_sim_buffers(h, nsim, pl);
   if (st == SGDLM_ERR_OUT_OF_MEMORY && h->lu_tail.ptr) {  // what is not needed goes first

@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpusgdlm_gb300 import SGDLM
+from gpusgdlm_gb300 import SGDLM, Batch
 from gpusgdlm_gb300.sgdlm import _pd
 
 pytestmark = pytest.mark.gpu
@@ -121,6 +121,39 @@ def test_the_buffer_goes_first(built_lib):
         got, _ = _log_dets(s, wl, large)
         s.close()
     np.testing.assert_array_equal(got, want)
+
+
+def test_recorded_steps_keep_their_buffers(built_lib):
+    """A batch's recorded step stays valid while the draw count goes up and down within what
+    the engine has held before (here in FP64, which has no hand-over)."""
+    P = _engine()[1]["P"]
+    n, out = 1000, []
+    for detour in (False, True):
+        s, wl = _engine()
+        s.setPrecision("fp64")
+        assert s._lib.sgdlm_init_sim_memory(s._h, 3000, 3000) == 0
+        s.setPrecision("mixed")
+        assert s._lib.sgdlm_init_sim_memory(s._h, n, n) == 0
+        s.setPriorParameters(np.zeros((P, M)), np.repeat((1e-3 * np.eye(P))[:, :, None], M, axis=2),
+                             np.full(M, 50.0), np.ones(M))
+        s.setRngState(5, 0)
+        y, F, x = (torch.from_numpy(np.ravel(v, order="F").copy()).cuda()
+                   for v in (wl["y"][1], wl["F_of"](1), wl["F_of"](2, False)))
+        w, fc = (torch.zeros(k, dtype=torch.float64, device="cuda") for k in (n, n * M))
+        torch.cuda.synchronize()
+        b = Batch([s])
+        b.record([y.data_ptr()], [F.data_ptr()], [x.data_ptr()], 0.0, [fc.data_ptr()], [w.data_ptr()])
+        if detour:
+            for k in (2500, n):
+                assert s._lib.sgdlm_init_sim_memory(s._h, k, k) == 0
+        b.step()
+        s.synchronize()
+        out.append((w.cpu().numpy(), fc.cpu().numpy()))
+        b.close()
+        s.close()
+    assert np.all(out[0][0] > 0) and np.isfinite(out[0][1]).all()
+    for a, c in zip(*out):
+        np.testing.assert_array_equal(a, c)
 
 
 def test_plan_without_memory(built_lib):
