@@ -48,6 +48,13 @@ def _log_dets(s, wl, n):
     return ld, launches
 
 
+@pytest.fixture(autouse=True)
+def _free_device():
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < _most() + (4 << 30):
+        pytest.skip("another process holds the device's memory")
+
+
 @contextlib.contextmanager
 def _hold(keep_free):
     """The device's free memory but keep_free bytes, for a while."""
